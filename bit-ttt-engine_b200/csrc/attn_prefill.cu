@@ -1,7 +1,8 @@
 // Causal attention of many new tokens per sequence over the Q8 KV cache (layers/attention.rs:198-217 on a prompt) on the
 // tcgen05 integer tensor cores, with the arithmetic of the decode kernel: a rotated query value is S * Q / 2^27 with four
-// signed 7-bit digits, a weight p * v_scale is B * U / 2^29 with four unsigned bytes, all digit sums are exact int32
-// accumulators, and the softmax runs in f32.
+// signed 7-bit digits, a weight p * v_scale is B * U / 2^32 with four unsigned bytes and B = the power of two above the largest
+// value scale of 512 positions, all digit sums are exact int32 accumulators, and the softmax runs in f32.  The scores are
+// the decode kernel's bit by bit; the sums are taken in another order.
 //
 // Two kernels.  prefill_rows_kernel turns the q | k | v rows of the new tokens into what the attention reads: keys (rotated)
 // and values into the cache as the append of a single token does, queries (rotated) into their digits, in place - a head's
@@ -15,17 +16,20 @@
 // of the MN-major B operand.  Cache bytes only lose their offset of 128 on the way to shared memory (xor 0x80).
 // The 64 query vectors are two groups of 32 with eight softmax warps and an MMA warp each, so that one group's softmax runs
 // under the other's MMAs; four loader warps fill a ring of three K | V tiles.
-// Softmax reference: a weight may exceed the running maximum by up to e^kHead before the maximum is moved (U has three bits
-// of headroom), so after the first tiles the integer accumulators run on from tile to tile; only where a score or a value
-// scale breaks its bound does the group read them out, join them into f32 sums in shared memory and rescale.
+// Softmax reference of a vector: the largest score so far, or one that a score exceeds by less than what the power of two B
+// leaves free (a weight is below B then, and U below 2^32).  While it holds, the integer accumulators run on from tile to
+// tile; where a score breaks it, that vector's four columns are read out, joined into f32 sums in shared memory and
+// rescaled, and of all vectors where B changes.
 //
-
-
-// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 869 -> 171 us, 16 x 128 tokens 302 -> 57; 1B shape (heads of
-// 64), 4 x 511 tokens 297 -> 60 us, 16 x 128 tokens 231 -> 41; 2 tokens 10.7 -> 9.2.  About 3 600 clocks per 64 x 128 scores,
-// where the products take 1 100: bound by the latency of a group's chain scores - vote - weights - products, and by what an
-// item begins and ends with.  With four softmax warps to a group (32 vectors a thread) the short items of heads of 64 took
-// 1.5 times as long; scores and weights through integer conversion instructions 1.1 times.
+// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 223 us, 16 x 128 tokens 300 -> 61; 1B shape (heads of
+// 64), 4 x 511 tokens 298 -> 71 us, 16 x 128 tokens 231 -> 47; 2 tokens 10.7 -> 9.2; 16 tokens after 2000 51.9 -> 52.8.  The products
+// of 64 x 128 scores take 1 100 clocks: bound by the instructions of the softmax warps and the latency of a group's chain
+// scores - vote - weights - products, and by what an item begins and ends with.  Of the 223 us 39 are moves of references,
+// which random scores ask for in most tiles (185 with references that never move); a weight word with two bits left free
+// for scores above the reference needed hardly any (184), but a weight then had 30 bits.  With four softmax warps to a group (32
+// vectors a thread) the short items of heads of 64 took 1.5 times as long; scores and weights through integer conversion
+// instructions 1.1 times; columns read out by fours of vectors 235 us, by two vectors 228, unrolled 276.
+#include <cfloat>
 #include <type_traits>
 
 #include "bt_common.cuh"
@@ -46,15 +50,12 @@ constexpr int kOpBytes = 8 * kChunk;         // an operand tile of up to 128 col
 constexpr int kPChunk = kTilePos * 16;       // the same of the weight words, whose writers are neighbouring positions
 constexpr int kPBytes = 8 * kPChunk;
 constexpr int kSoftWarps = 16, kLoadWarps = 4;
-constexpr int kGroupThreads = kSoftWarps / 2 * 32, kHalfVec = kGroupVec / 2;
+constexpr int kHalfVec = kGroupVec / 2, kHalfThreads = 128;
 constexpr int kThreads = (kSoftWarps + kLoadWarps + 4) * 32;  // + an MMA warp per group, two idle: the roles are whole warpgroups
 constexpr int kRegsSoft = 96, kRegsLoad = 56, kRegsMma = 40;
 constexpr int kMaxDim = 128;
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kHead = 2.07f;           // < 3 ln 2
-constexpr int kHeadBits = 3;
-constexpr float kLow = -1e30f;           // the running maximum before the first tile
-constexpr int kMaxRun = 256;             // tiles between two read-outs: 256 * 128 positions * 255 * 128 < 2^31
+constexpr int kBoundTiles = 4;           // tiles of a weight bound
+constexpr int kMaxRun = 256;             // tiles between two read-outs at most: 256 * 128 positions * 255 * 128 < 2^31
 // Integers become floats without a conversion (16 a clock and SM, as the exponential): an integer below 2^22 added to the bit
 // pattern of kMagic is the pattern of kMagic plus that integer.  The score accumulators start at the pattern, so that the
 // MMAs leave floats; kMagicHi takes it out of a digit and, 128 times smaller, out of the digit below in the same addition.
@@ -70,15 +71,14 @@ struct Smem {
     alignas(128) uint8_t u[2][kPBytes];                // weight words of a group's tile
     alignas(16) float osum[2][kGroupVec][kMaxDim];     // what has been read out of the accumulators
     alignas(16) float cq[2][kGroupVec];                // S / 2^27 times the score scaling
-    alignas(16) float thr[2][kGroupVec];               // scores above this move the reference
-    alignas(16) float mlog[2][kGroupVec];              // reference * log2(e)
-    alignas(16) float fac[2][kGroupVec];               // e^(old - new reference) of a read-out; at the end the denominators
+    alignas(16) float mref[2][kGroupVec];              // reference of the weights
+    alignas(16) float fac[2][kGroupVec];               // e^(old - new reference) of a move; at the end the denominators
     alignas(16) float inv[2][kGroupVec];               // and their reciprocals
     alignas(16) int seen[2][kGroupVec];                // last position a vector sees
     alignas(16) int at[2][2][kGroupVec];               // [item & 1]: where its output goes (-1: nowhere)
-    float mref[2][kGroupVec];
     float wred[2][4][kGroupVec];                       // per warp: maxima of a tile, sums at the end
-    float wv[2][4];
+    uint32_t moved[2][2];                              // per half: the vectors whose reference moves
+    alignas(16) float wv[2][2][4];                                 // per half and warp: largest value scale of a bound's tiles
     uint64_t full[kStages], empty[kStages];
     uint64_t q_full[2], q_empty[2], s_full[2], s_empty[2], p_full[2], pv_done[2];
     uint32_t tmem;
@@ -102,17 +102,20 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
     return r != 0;
 }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 // the loads into v are complete (v is named, so that no use of it is moved before the wait)
 __device__ __forceinline__ void ld_wait16(uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
                    "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
                  :: "memory");
+}
+// four consecutive columns of this thread's tensor-memory lane, which are zero afterwards
+__device__ __forceinline__ void tmem_take4(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n\t"
+        "tcgen05.wait::ld.sync.aligned;\n\t"
+        "tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%5, %5, %5, %5};"
+        : "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]) : "r"(taddr), "r"(0) : "memory");
 }
 // An item of the persistent loop: the heaviest query blocks first, dealt to the CTAs forwards and backwards in turn.
 struct Item {
@@ -175,7 +178,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
     if (warp < kSoftWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoft));
         // ---------------- softmax of group g: thread = position (scores, weights) or dim (outputs) r, half of the vectors ----------------
-        const int g = warp >> 3, w4 = warp & 3, r = 32 * w4 + lane, h0 = (warp >> 2 & 1) * kHalfVec, tg = tid & (kGroupThreads - 1), bar_id = 1 + g;
+        const int g = warp >> 3, w4 = warp & 3, r = 32 * w4 + lane, half = warp >> 2 & 1, h0 = half * kHalfVec, th = tid & (kHalfThreads - 1), bar_id = 1 + (warp >> 2);
+        const int own = h0 + th;  // th < kHalfVec: the vector this thread looks after
         const uint32_t s_addr = tmem + ((uint32_t)(32 * w4) << 16) + g * kCols + 4 * h0, o_addr = s_addr + 2 * kCols;
         const int per_group = kGroupVec >> a.rep_log;
         uint32_t magic[16];
@@ -193,14 +197,16 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
         int n = 0;  // tiles of all items so far
         Item it = {};
         // what the first tile of an item needs from global memory, requested before the item in front is finished
+        // (a value scale that is no number or negative counts as zero, as it does in the decode kernel)
         float ks_next = 0.0f, vs_next = 0.0f, q_scale = 0.0f;
+        auto value_scale = [&](const float* vs, int at, int t_len) { return at < t_len ? fmaxf(vs[at], 0.0f) : 0.0f; };
         auto prefetch = [&]() {
-            const int64_t row = ((int64_t)it.b * a.n_kv + it.kvh) * a.cache.max_seq + r;
-            ks_next = r < it.t_len ? a.cache.k_s[row] : 0.0f;
-            vs_next = r < it.t_len ? a.cache.v_s[row] : 0.0f;
-            if (tg < kGroupVec) {
-                const int tok = min(it.q0 + g * per_group + (tg >> a.rep_log), a.q_rows - 1);  // (beyond the last token: the last again, not stored)
-                q_scale = a.qscale[((int64_t)it.b * a.q_rows + tok) * a.n_heads + (it.kvh << a.rep_log) + (tg & ((1 << a.rep_log) - 1))];
+            const int64_t row = ((int64_t)it.b * a.n_kv + it.kvh) * a.cache.max_seq;
+            ks_next = r < it.t_len ? a.cache.k_s[row + r] : 0.0f;
+            vs_next = value_scale(a.cache.v_s + row, r, it.t_len);
+            if (th < kHalfVec) {
+                const int tok = min(it.q0 + g * per_group + (own >> a.rep_log), a.q_rows - 1);  // (beyond the last token: the last again, not stored)
+                q_scale = a.qscale[((int64_t)it.b * a.q_rows + tok) * a.n_heads + (it.kvh << a.rep_log) + (own & ((1 << a.rep_log) - 1))];
             }
         };
         bool more = items.get(0, &it);
@@ -210,40 +216,25 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             const float *ks = a.cache.k_s + row_base, *vs = a.cache.v_s + row_base;
             const int first = it.q0 + g * per_group;  // the group's first new token
             const int first_seen = it.p + min(first, a.q_rows - 1), tiles = it.tiles, t_len = it.t_len;
-            if (tg < kGroupVec) {
-                const int tok = first + (tg >> a.rep_log);
-                sm.cq[g][tg] = __fmul_rn(q_scale, a.scaling);
-                sm.seen[g][tg] = it.p + min(tok, a.q_rows - 1);
-                sm.at[round & 1][g][tg] = tok < a.q_rows ? (tok * a.n_heads + (it.kvh << a.rep_log) + (tg & ((1 << a.rep_log) - 1))) * HD : -1;
-                sm.mref[g][tg] = sm.thr[g][tg] = kLow;
-                sm.mlog[g][tg] = kLow * kLog2e;
+            if (th < kHalfVec) {
+                const int tok = first + (own >> a.rep_log);
+                sm.cq[g][own] = __fmul_rn(q_scale, a.scaling);
+                sm.seen[g][own] = it.p + min(tok, a.q_rows - 1);
+                sm.mref[g][own] = -FLT_MAX;
+                sm.at[round & 1][g][own] = tok < a.q_rows ? (tok * a.n_heads + (it.kvh << a.rep_log) + (own & ((1 << a.rep_log) - 1))) * HD : -1;
             }
             float l[kHalfVec], s[kHalfVec];
 #pragma unroll
             for (int v = 0; v < kHalfVec; ++v) l[v] = 0.0f;
-            bool kept = false;  // osum holds something
-            float bound = 0.0f, up = 0.0f, down = 0.0f;
-            int run = 0;  // tiles in the accumulators
-            ptx::named_bar_sync(bar_id, kGroupThreads);
-            // the accumulators of the tiles so far, as f32, joined with what was read out before; use(v, value) for each
-            // vector.  They are zero afterwards.
-            auto read_out = [&](auto use) {
-                uint32_t d[2][16];
-                ptx::tmem_ld16(o_addr, d[0]);
-#pragma unroll
-                for (int c = 0; c < kHalfVec / 4; ++c) {
-                    ld_wait16(d[c & 1]);
-                    if (c + 1 < kHalfVec / 4) ptx::tmem_ld16(o_addr + 16 * (c + 1), d[(c + 1) & 1]);
-                    ptx::tmem_st16(o_addr + 16 * c, {});
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t* b = &d[c & 1][4 * i];
-                        const long long sum = (long long)(int)b[3] * (1 << 24) + ((long long)(int)b[2] * (1 << 16) + ((long long)(int)b[1] * (1 << 8) + (int)b[0]));
-                        const float f = fmaf((float)(int)(sum >> 32), 4294967296.0f, (float)(uint32_t)sum);
-                        use(4 * c + i, fmaf(f, down, kept ? sm.osum[g][h0 + 4 * c + i][r] : 0.0f));
-                    }
-                }
-                ptx::tmem_st_wait();
+            uint32_t kept = 0;            // vectors of which osum holds something
+            uint32_t ex = 0, ex_new = 0;  // exponent of the weight bound, of these tiles and of the next kBoundTiles
+            float up = 0.0f, down = 0.0f, room = 0.0f;  // room: how far a score may exceed its reference
+            ptx::named_bar_sync(bar_id, kHalfThreads);
+            // of vector v, whose four digit columns are b: the accumulator as f32, joined with what was read out before
+            auto joined = [&](const uint32_t* b, int v) {
+                const long long sum = (long long)(int)b[3] * (1 << 24) + ((long long)(int)b[2] * (1 << 16) + ((long long)(int)b[1] * (1 << 8) + (int)b[0]));
+                const float f = fmaf((float)(int)(sum >> 32), 4294967296.0f, (float)(uint32_t)sum);
+                return fmaf(f, down, kept >> v & 1 ? sm.osum[g][h0 + v][r] : 0.0f);
             };
             // lane v % 16 ends with the warp's join of vector h0 + v (x is consumed)
             auto across = [&](float (&x)[kHalfVec], auto join) {
@@ -260,14 +251,23 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             for (int t = 0; t < tiles; ++t, ++n) {
                 const float k_scale = ks_next, v_scale = vs_next;
                 const int at = t * kTilePos + r;
+                // The value scales of the next bound's tiles are looked at in the tile before its first one (of the first bound: in
+                // the first), so that the bound is known when that tile's scores are compared with their reference.
+                const bool look = t == 0 || (t % kBoundTiles == kBoundTiles - 1 && t + 1 < tiles);
+                float v_look[kBoundTiles] = {};
+                if (look) {
+                    const int from = at + (t > 0 ? kTilePos : 0);
+#pragma unroll
+                    for (int i = 0; i < kBoundTiles; ++i) v_look[i] = value_scale(vs, from + i * kTilePos, t_len);
+                }
                 if (t + 1 < tiles) {
-                    const bool live = at + kTilePos < t_len;
-                    ks_next = live ? ks[at + kTilePos] : 0.0f;
-                    vs_next = live ? vs[at + kTilePos] : 0.0f;
+                    ks_next = at + kTilePos < t_len ? ks[at + kTilePos] : 0.0f;
+                    vs_next = value_scale(vs, at + kTilePos, t_len);
                 }
                 wait(&sm.s_full[g], n);
                 ptx::tc_fence_after();
-                bool over = v_scale > bound;
+                const float v_most = fmaxf(fmaxf(v_look[0], v_look[1]), fmaxf(v_look[2], v_look[3]));
+                bool over = false;  // some score is too far above its reference
                 auto scores = [&](auto masked_tag) {
                     constexpr bool kMasked = decltype(masked_tag)::value;
                     uint32_t d[2][16];
@@ -277,8 +277,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                         ld_wait16(d[c & 1]);
                         if (c + 1 < kHalfVec / 4) ptx::tmem_ld16(s_addr + 16 * (c + 1), d[(c + 1) & 1]);
                         ptx::tmem_st16(s_addr + 16 * c, magic);  // (the loads of these columns are complete)
-                        const float4 cq = *reinterpret_cast<const float4*>(&sm.cq[g][h0 + 4 * c]), th = *reinterpret_cast<const float4*>(&sm.thr[g][h0 + 4 * c]);
-                        const float cqv[4] = {cq.x, cq.y, cq.z, cq.w}, thv[4] = {th.x, th.y, th.z, th.w};
+                        const float4 cq = *reinterpret_cast<const float4*>(&sm.cq[g][h0 + 4 * c]), mr = *reinterpret_cast<const float4*>(&sm.mref[g][h0 + 4 * c]);
+                        const float cqv[4] = {cq.x, cq.y, cq.z, cq.w}, mrv[4] = {mr.x, mr.y, mr.z, mr.w};
                         int4 last = make_int4(0, 0, 0, 0);
                         if (kMasked) last = *reinterpret_cast<const int4*>(&sm.seen[g][h0 + 4 * c]);
                         const int lastv[4] = {last.x, last.y, last.z, last.w};
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                             float x = __fmul_rn(__fmul_rn(fmaf(hi, 16384.0f, lo), k_scale), cqv[i]);
                             if (kMasked && at > lastv[i]) x = -INFINITY;
                             s[4 * c + i] = x;
-                            over |= x > thv[i];
+                            over |= __fsub_rn(x, mrv[i]) > room;
                         }
                     }
                 };
@@ -301,53 +301,80 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&sm.s_empty[g]);
-                const bool move = bar_or(bar_id, kGroupThreads, over || t == 0 || run >= kMaxRun);
-                if (n > 0) {
-                    wait(&sm.pv_done[g], n - 1);  // the weight words are free, the accumulators hold the tiles before
-                    ptx::tc_fence_after();
-                }
-                if (move) {
+                if (__any_sync(0xffffffffu, over)) {
                     float m[kHalfVec];
 #pragma unroll
                     for (int v = 0; v < kHalfVec; ++v) m[v] = s[v];
                     across(m, [](float x, float y) { return fmaxf(x, y); });
-                    const unsigned vm = __reduce_max_sync(0xffffffffu, __float_as_uint(v_scale));
-                    if (lane == 0) sm.wv[g][w4] = __uint_as_float(vm);  // (the same from both halves)
-                    ptx::named_bar_sync(bar_id, kGroupThreads);
-                    if (tg < kGroupVec) {
-                        const float old = sm.mref[g][tg];
-                        const float mx = fmaxf(old, fmaxf(fmaxf(sm.wred[g][0][tg], sm.wred[g][1][tg]), fmaxf(sm.wred[g][2][tg], sm.wred[g][3][tg])));
-                        sm.fac[g][tg] = exp2f((old - mx) * kLog2e);
-                        sm.mref[g][tg] = mx;
-                        sm.thr[g][tg] = mx + kHead;
-                        sm.mlog[g][tg] = mx * kLog2e;
-                    }
-                    // the power of two above the largest value scale so far (kept inside the range its inverse needs)
-                    const float big = fmaxf(fmaxf(sm.wv[g][0], sm.wv[g][1]), fmaxf(sm.wv[g][2], sm.wv[g][3]));
-                    const uint32_t ex = max(__float_as_uint(bound) >> 23, (uint32_t)min(max((int)(__float_as_uint(big) >> 23), 40), 250) + 1);
-                    ptx::named_bar_sync(bar_id, kGroupThreads);
-                    if (t > 0) {
-                        read_out([&](int v, float o) { sm.osum[g][h0 + v][r] = o * sm.fac[g][h0 + v]; });
-                        kept = true;
-#pragma unroll
-                        for (int v = 0; v < kHalfVec; ++v) l[v] *= sm.fac[g][h0 + v];
-                    }
-                    bound = __uint_as_float(ex << 23);
-                    up = __uint_as_float((254 - ex + 32 - kHeadBits) << 23);  // 2^29 / bound
-                    down = __uint_as_float((ex - 32 + kHeadBits) << 23);      // bound / 2^29
-                    run = 0;
+                } else if (lane < kHalfVec) {
+                    sm.wred[g][w4][h0 + lane] = -FLT_MAX;
                 }
-                ++run;
-                const float w_scale = __fmul_rn(v_scale, up) * (1.0f / 65536.0f);
+                if (look) {
+                    const unsigned vm = __reduce_max_sync(0xffffffffu, __float_as_uint(v_most));
+                    if (lane == 0) sm.wv[g][half][w4] = __uint_as_float(vm);
+                }
+                const bool move = bar_or(bar_id, kHalfThreads, over);
+                if (n > 0) {
+                    wait(&sm.pv_done[g], n - 1);  // the weight words are free, the accumulators hold the tiles before
+                    ptx::tc_fence_after();
+                }
+                const bool new_bound = t % kBoundTiles == 0, all = (new_bound && ex_new != ex) || t % kMaxRun == 0;
+                const float room_now = room;
+                if (look) {
+                    // The power of two above the largest value scale of these tiles, and 2^-19 more, so that a weight is below 2^32
+                    // whatever the last bits of its exponential (kept where the bound and 2^-32 of it are floats).  What that
+                    // power leaves free is room for scores above the reference.
+                    const float4 v4 = *reinterpret_cast<const float4*>(sm.wv[g][half]);
+                    const float big = fmaxf(fmaxf(v4.x, v4.y), fmaxf(v4.z, v4.w));
+                    const uint32_t bits = __float_as_uint(fmaf(big, 1.0f / 524288.0f, big));
+                    ex_new = min(max((bits >> 23) + 1, 33u), 254u);
+                    room = (bits >> 23) < 254u ? fmaxf(-logf(__uint_as_float((bits & 0x7fffffu) | 126u << 23)) - 1.0f / 262144.0f, 0.0f) : 0.0f;
+                }
+                if (move || (all && t > 0)) {
+                    if (move) {
+                        if (th < kHalfVec) {
+                            const float old = sm.mref[g][own], most = fmaxf(fmaxf(sm.wred[g][0][own], sm.wred[g][1][own]), fmaxf(sm.wred[g][2][own], sm.wred[g][3][own]));
+                            const bool moves = __fsub_rn(most, old) > room_now;
+                            const uint32_t moved = __ballot_sync(0xffffu, moves);
+                            if (th == 0) sm.moved[g][half] = t > 0 ? moved : 0u;
+                            sm.fac[g][own] = moves ? expf(__fsub_rn(old, most)) : 1.0f;
+                            if (moves) sm.mref[g][own] = most;
+                        }
+                        ptx::named_bar_sync(bar_id, kHalfThreads);
+#pragma unroll
+                        for (int c = 0; c < kHalfVec / 4; ++c) {
+                            const float4 f = *reinterpret_cast<const float4*>(&sm.fac[g][h0 + 4 * c]);
+                            l[4 * c] *= f.x; l[4 * c + 1] *= f.y; l[4 * c + 2] *= f.z; l[4 * c + 3] *= f.w;
+                        }
+                    }
+                    // read out the vectors whose reference has moved (of a new bound all); their columns are zero afterwards.  (Not
+                    // unrolled: this code is run rarely and together, and the rest of the loop has to stay in the instruction cache.)
+                    const uint32_t which = all && t > 0 ? (1u << kHalfVec) - 1 : sm.moved[g][half];
+#pragma unroll 1
+                    for (uint32_t rest = which; rest; rest &= rest - 1) {
+                        const int v = __ffs(rest) - 1;
+                        uint32_t d[4];
+                        tmem_take4(o_addr + 4 * v, d);
+                        sm.osum[g][h0 + v][r] = joined(d, v) * (move ? sm.fac[g][h0 + v] : 1.0f);
+                    }
+                    ptx::tmem_st_wait();
+                    kept |= which;
+                }
+                if (new_bound) {
+                    ex = ex_new;
+                    up = __uint_as_float((270 - ex) << 23);   // 2^16 / bound
+                    down = __uint_as_float((ex - 32) << 23);  // bound / 2^32
+                }
+                const float w_scale = fminf(__fmul_rn(v_scale, up), 65535.9375f);  // (smaller already, but for scales beyond the last bound)
                 uint8_t* words = sm.u[g] + h0 / 4 * kPChunk + r * 16;
 #pragma unroll
                 for (int c = 0; c < kHalfVec / 4; ++c) {
-                    const float4 ml = *reinterpret_cast<const float4*>(&sm.mlog[g][h0 + 4 * c]);
-                    const float mlv[4] = {ml.x, ml.y, ml.z, ml.w};
+                    const float4 mr = *reinterpret_cast<const float4*>(&sm.mref[g][h0 + 4 * c]);
+                    const float mrv[4] = {mr.x, mr.y, mr.z, mr.w};
                     uint32_t w[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float e = ex2(fmaf(s[4 * c + i], kLog2e, -mlv[i]));
+                        const float e = expf(__fsub_rn(s[4 * c + i], mrv[i]));
                         l[4 * c + i] += e;
                         const float upper = fmaf(e, w_scale, kMagicWord);  // the word's upper half, rounded; what is left of it (signed) in 2^-16
                         const float rest = fmaf(e, w_scale, -__fsub_rn(upper, kMagicWord));
@@ -364,21 +391,32 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             more = items.get(round + 1, &it);
             if (more) prefetch();
             across(l, [](float x, float y) { return x + y; });
-            ptx::named_bar_sync(bar_id, kGroupThreads);
-            if (tg < kGroupVec) {
-                const float sum = (sm.wred[g][0][tg] + sm.wred[g][1][tg]) + (sm.wred[g][2][tg] + sm.wred[g][3][tg]);
-                sm.fac[g][tg] = sum;
-                sm.inv[g][tg] = __frcp_rn(sum);
+            ptx::named_bar_sync(bar_id, kHalfThreads);
+            if (th < kHalfVec) {
+                const float sum = (sm.wred[g][0][own] + sm.wred[g][1][own]) + (sm.wred[g][2][own] + sm.wred[g][3][own]);
+                sm.fac[g][own] = sum;
+                sm.inv[g][own] = __frcp_rn(sum);
             }
             wait(&sm.pv_done[g], n - 1);
             ptx::tc_fence_after();
-            ptx::named_bar_sync(bar_id, kGroupThreads);
-            read_out([&](int v, float o) {
-                // o / sum, correctly rounded: the quotient by the reciprocal and one correction by its remainder (Markstein 1990)
-                const int to = sm.at[round & 1][g][h0 + v];
-                const float sum = sm.fac[g][h0 + v], inv = sm.inv[g][h0 + v], q = o * inv;
-                if (to >= 0 && r < HD) out[to] = fmaf(fmaf(-sum, q, o), inv, q);
-            });
+            ptx::named_bar_sync(bar_id, kHalfThreads);
+            uint32_t d[2][16];
+            ptx::tmem_ld16(o_addr, d[0]);
+#pragma unroll
+            for (int c = 0; c < kHalfVec / 4; ++c) {
+                ld_wait16(d[c & 1]);
+                if (c + 1 < kHalfVec / 4) ptx::tmem_ld16(o_addr + 16 * (c + 1), d[(c + 1) & 1]);
+                ptx::tmem_st16(o_addr + 16 * c, {});
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int v = 4 * c + i, to = sm.at[round & 1][g][h0 + v];
+                    const float o = joined(&d[c & 1][4 * i], v), sum = sm.fac[g][h0 + v], inv = sm.inv[g][h0 + v];
+                    // o / sum, correctly rounded: the quotient by the reciprocal and one correction by its remainder (Markstein 1990)
+                    const float q = o * inv;
+                    if (to >= 0 && r < HD) out[to] = fmaf(fmaf(-sum, q, o), inv, q);
+                }
+            }
+            ptx::tmem_st_wait();
             ptx::tc_fence_before();
         }
     } else if (warp < kSoftWarps + kLoadWarps) {

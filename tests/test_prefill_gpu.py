@@ -159,10 +159,10 @@ def attention_64(qkv, rows, heads, kv_heads, hd, past, theta):
 
 
 @pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 32), (4, 2, 64), (4, 4, 96), (8, 2, 128), (8, 1, 64)])
-@pytest.mark.parametrize("batch,past,n", [(1, 0, 2), (3, 0, 65), (2, 0, 128), (1, 127, 2), (1, 100, 29), (1, 257, 400)])
+@pytest.mark.parametrize("batch,past,n", [(1, 0, 2), (3, 0, 65), (2, 0, 128), (1, 127, 2), (1, 100, 29), (1, 257, 400), (31, 200, 65)])
 def test_prefill_attention_against_64_bits(bt, syn, heads, kv_heads, hd, batch, past, n):
-    # partial query blocks and key tiles, tiles that end on and beside the last key, several items per CTA, every number of
-    # heads per KV head.  In f32 a score has a relative error of a few 2^-24 (rotation, joining of the digits, three
+    # partial query blocks and key tiles, tiles that end on and beside the last key, every number of heads per KV head; 31
+    # sequences make 186 items and more, so that CTAs (148 at most) take several in turn.  In f32 a score has a relative error of a few 2^-24 (rotation, joining of the digits, three
     # factors), which the exponential turns into |score| (< 4 here) times that, an output one of a few 2^-24 more: 5e-7
     # bounds the relative error of the whole (2-norm), about 7e-8 is what is measured.
     cfg = syn.BitLlamaConfig("llama", 300, heads * hd, 2, heads, kv_heads, 256, max_position_embeddings=past + n + 8)
@@ -179,4 +179,72 @@ def test_prefill_attention_against_64_bits(bt, syn, heads, kv_heads, hd, batch, 
         for b in range(batch):
             want = attention_64(qkv[b], gpu.kv_cache(li).export(b, past + n), heads, kv_heads, hd, past, cfg.rope_theta)
             assert np.linalg.norm(att[b] - want) <= 5e-7 * np.linalg.norm(want)
+    assert bt.lib().bt_device_check(0) == 0
+
+
+def rows_for_scores(rng, q, scores):
+    """Key rows whose scores with the query vectors q [kv_heads, hd] (rotated) are `scores` [past], up to f32 roundings; random values."""
+    kv_heads, hd = q.shape
+    b = np.round(q / np.abs(q).max(-1, keepdims=True) * 127)
+    scale = np.abs(scores) * np.sqrt(hd) / (q * b).sum(-1, keepdims=True)
+    kq = np.where(scores[None, :, None] < 0, -b[:, None], b[:, None]) + 128
+    vq = rng.integers(0, 256, kq.shape)
+    return [kq.astype(np.uint8), scale.astype(np.float32), vq.astype(np.uint8), rng.uniform(0.005, 0.03, scale.shape).astype(np.float32)]
+
+
+def steered_rows(rng, kind, q, past):
+    at = np.arange(past)
+    if kind == "growing":    # the maximum moves in every tile, as far as the last cached key
+        return rows_for_scores(rng, q, at / 40)
+    if kind == "falling":
+        return rows_for_scores(rng, q, -at / 40)
+    if kind in ("1e6", "1e7", "1e8"):  # scores of which an f32 holds the difference to the maximum in a few bits, or hardly at all
+        return rows_for_scores(rng, q, float(kind) + rng.integers(0, 4, past) + at // 128)
+    rows = rows_for_scores(rng, q, rng.normal(0, 2, past))
+    if kind == "value scales":  # powers of two up and down from tile to tile, and rows of zeros
+        rows[3] = (rows[3] * 2.0 ** ((at // 128 * 7) % 24 - 12)).astype(np.float32)
+        rows[2][:, at % 5 == 0], rows[3][:, at % 5 == 0] = 128, 0
+    if kind == "odd scales":  # no number, negative: nothing, as for the decode kernel; the smallest, the largest that count
+        rows[3][:, at % 7 == 0], rows[3][:, at % 7 == 3] = np.nan, -1.0
+        rows[3][:, :128], rows[3][:, 128:] = rows[3][:, :128] * np.float32(1e-25), rows[3][:, 128:] * np.float32(1e28)
+    return rows
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 32), (4, 2, 64), (8, 2, 128), (8, 1, 64)])
+@pytest.mark.parametrize("kind,past", [("growing", 600), ("falling", 600), ("1e6", 600), ("1e7", 600), ("1e8", 600), ("value scales", 1400),
+                                       ("odd scales", 700), ("random", 513), ("random", 33000)])
+def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, past):
+    # Peaked, huge and unequal rows, where the reference of the weights and their bound move, and more tiles than the
+    # accumulators hold (33 000 positions).  The two kernels compute the same scores and weights of the same bits and differ in the
+    # order of the sums and in the maximum that a weight is relative to at first: up to 16 moves, each with three roundings
+    # and an exponential good to 2^-22 at most, hence 16 * 2^-22 of the 2-norm.
+    n, theta = 3, 10000.0
+    cfg = syn.BitLlamaConfig("llama", 300, heads * hd, 1, heads, kv_heads, 256, max_position_embeddings=past + n, rope_theta=theta)
+    gpu = syn.build_model(syn.make_weights(cfg, seed=past + hd), max_batch=1)
+    rng = np.random.default_rng(past + hd)
+    tokens = rng.integers(0, 300, (1, n))
+    gpu.set_trace(True, rows=n)
+
+    def prefill():
+        gpu.seek(past)
+        gpu.prefill(tokens)
+        return gpu.read_trace(n)[0]
+
+    qkv = prefill()["qkv"]  # of the first layer: the same whatever the cache holds
+    half = hd // 2
+    ang = (np.float32(past) * (1 / theta ** (np.arange(0, hd, 2) / hd)).astype(np.float32)).astype(np.float64)
+    q = qkv[0, :heads * hd].astype(np.float64).reshape(kv_heads, -1, hd)[:, 0]
+    q = np.concatenate([q[:, :half] * np.cos(ang) - q[:, half:] * np.sin(ang), q[:, :half] * np.sin(ang) + q[:, half:] * np.cos(ang)], -1)
+    rows = steered_rows(rng, kind, q, past)
+    gpu.kv_cache(0).load(0, *rows)
+    trace = prefill()
+    assert np.array_equal(trace["qkv"], qkv)
+    cache = bt.QuantizedKVCache(past + n, 1, kv_heads, hd)
+    cache.load(0, *rows)
+    for i in range(n):
+        pos = torch.full((1,), past + i, dtype=torch.int32, device="cuda")
+        want = bt.attn_decode(cache, torch.from_numpy(qkv[i:i + 1]).cuda(), pos, heads, theta).cpu().numpy().reshape(heads, hd).astype(np.float64)
+        got = trace["att"][i].reshape(heads, hd)
+        assert np.isfinite(want).all()
+        assert (np.linalg.norm(got - want, axis=-1) <= 16 * 2.0 ** -22 * np.linalg.norm(want, axis=-1)).all(), (kind, i)
     assert bt.lib().bt_device_check(0) == 0
