@@ -21,12 +21,12 @@
 // tile; where a score breaks it, that vector's four columns are read out, joined into f32 sums in shared memory and
 // rescaled, and of all vectors where B changes.
 //
-// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 223 us, 16 x 128 tokens 300 -> 61; 1B shape (heads of
-// 64), 4 x 511 tokens 298 -> 71 us, 16 x 128 tokens 231 -> 47; 2 tokens 10.7 -> 9.2; 16 tokens after 2000 51.9 -> 52.8.  The products
+// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 227 us, 16 x 128 tokens 300 -> 57; 1B shape (heads of
+// 64), 4 x 511 tokens 298 -> 75 us, 16 x 128 tokens 231 -> 51; 2 tokens 10.7 -> 10.2; 16 tokens after 2000 51.9 -> 53.6.  The products
 // of 64 x 128 scores take 1 100 clocks: bound by the instructions of the softmax warps and the latency of a group's chain
-// scores - vote - weights - products, and by what an item begins and ends with.  Of the 223 us 39 are moves of references,
-// which random scores ask for in most tiles (185 with references that never move); a weight word with two bits left free
-// for scores above the reference needed hardly any (184), but a weight then had 30 bits.  With four softmax warps to a group (32
+// scores - vote - weights - products, and by what an item begins and ends with.  Of the 227 us 39 are moves of references,
+// which random scores ask for in most tiles; a weight word with two bits left free for scores above the
+// reference needed hardly any, but a weight then had 30 bits.  With four softmax warps to a group (32
 // vectors a thread) the short items of heads of 64 took 1.5 times as long; scores and weights through integer conversion
 // instructions 1.1 times; columns read out by fours of vectors 235 us, by two vectors 228, unrolled 276.
 #include <cfloat>
@@ -73,7 +73,6 @@ struct Smem {
     alignas(16) float cq[2][kGroupVec];                // S / 2^27 times the score scaling
     alignas(16) float mref[2][kGroupVec];              // reference of the weights
     alignas(16) float fac[2][kGroupVec];               // e^(old - new reference) of a move; at the end the denominators
-    alignas(16) float inv[2][kGroupVec];               // and their reciprocals
     alignas(16) int seen[2][kGroupVec];                // last position a vector sees
     alignas(16) int at[2][2][kGroupVec];               // [item & 1]: where its output goes (-1: nowhere)
     float wred[2][4][kGroupVec];                       // per warp: maxima of a tile, sums at the end
@@ -233,8 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             // of vector v, whose four digit columns are b: the accumulator as f32, joined with what was read out before
             auto joined = [&](const uint32_t* b, int v) {
                 const long long sum = (long long)(int)b[3] * (1 << 24) + ((long long)(int)b[2] * (1 << 16) + ((long long)(int)b[1] * (1 << 8) + (int)b[0]));
-                const float f = fmaf((float)(int)(sum >> 32), 4294967296.0f, (float)(uint32_t)sum);
-                return fmaf(f, down, kept >> v & 1 ? sm.osum[g][h0 + v][r] : 0.0f);
+                return fmaf(__ll2float_rn(sum), down, kept >> v & 1 ? sm.osum[g][h0 + v][r] : 0.0f);
             };
             // lane v % 16 ends with the warp's join of vector h0 + v (x is consumed)
             auto across = [&](float (&x)[kHalfVec], auto join) {
@@ -392,11 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             if (more) prefetch();
             across(l, [](float x, float y) { return x + y; });
             ptx::named_bar_sync(bar_id, kHalfThreads);
-            if (th < kHalfVec) {
-                const float sum = (sm.wred[g][0][own] + sm.wred[g][1][own]) + (sm.wred[g][2][own] + sm.wred[g][3][own]);
-                sm.fac[g][own] = sum;
-                sm.inv[g][own] = __frcp_rn(sum);
-            }
+            if (th < kHalfVec) sm.fac[g][own] = (sm.wred[g][0][own] + sm.wred[g][1][own]) + (sm.wred[g][2][own] + sm.wred[g][3][own]);
             wait(&sm.pv_done[g], n - 1);
             ptx::tc_fence_after();
             ptx::named_bar_sync(bar_id, kHalfThreads);
@@ -410,10 +404,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int v = 4 * c + i, to = sm.at[round & 1][g][h0 + v];
-                    const float o = joined(&d[c & 1][4 * i], v), sum = sm.fac[g][h0 + v], inv = sm.inv[g][h0 + v];
-                    // o / sum, correctly rounded: the quotient by the reciprocal and one correction by its remainder (Markstein 1990)
-                    const float q = o * inv;
-                    if (to >= 0 && r < HD) out[to] = fmaf(fmaf(-sum, q, o), inv, q);
+                    const float o = joined(&d[c & 1][4 * i], v);
+                    if (to >= 0 && r < HD) out[to] = __fdiv_rn(o, sm.fac[g][h0 + v]);
                 }
             }
             ptx::tmem_st_wait();

@@ -200,6 +200,11 @@ def steered_rows(rng, kind, q, past):
         return rows_for_scores(rng, q, -at / 40)
     if kind in ("1e6", "1e7", "1e8"):  # scores of which an f32 holds the difference to the maximum in a few bits, or hardly at all
         return rows_for_scores(rng, q, float(kind) + rng.integers(0, 4, past) + at // 128)
+    if kind == "small sums":  # the largest weight belongs to a row of zeros; what is left are small negative sums
+        rows = rows_for_scores(rng, q, np.where(at == 7, 40.0, np.where(at == 9, 30.3, 10.0)))
+        rows[2][:], rows[3][:] = rng.integers(124, 128, rows[2].shape), 0.01
+        rows[2][:, 7] = 128
+        return rows
     rows = rows_for_scores(rng, q, rng.normal(0, 2, past))
     if kind == "value scales":  # powers of two up and down from tile to tile, and rows of zeros
         rows[3] = (rows[3] * 2.0 ** ((at // 128 * 7) % 24 - 12)).astype(np.float32)
@@ -212,7 +217,7 @@ def steered_rows(rng, kind, q, past):
 
 @pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 32), (4, 2, 64), (8, 2, 128), (8, 1, 64)])
 @pytest.mark.parametrize("kind,past", [("growing", 600), ("falling", 600), ("1e6", 600), ("1e7", 600), ("1e8", 600), ("value scales", 1400),
-                                       ("odd scales", 700), ("random", 513), ("random", 33000)])
+                                       ("odd scales", 700), ("small sums", 140), ("random", 513), ("random", 33000)])
 def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, past):
     # Peaked, huge and unequal rows, where the reference of the weights and their bound move, and more tiles than the
     # accumulators hold (33 000 positions).  The two kernels compute the same scores and weights of the same bits and differ in the
