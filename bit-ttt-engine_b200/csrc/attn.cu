@@ -356,10 +356,12 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
     // P.V ownership: warp = (group of 32 dims dg, position group pq); the warp handles the 32-position steps
     // pq, pq + n_pq, ... of every tile for dims 32 dg .. 32 dg + 31.  Four 32-bit loads of V rows (dims
     // 32 dg + 4 g .. + 3 of four positions) are transposed into the B fragments of four MMAs, MMA e holding
-    // dim 32 dg + 4 n + e in column n.
+    // dim 32 dg + 4 n + e in column n.  Heads of 96 make three groups of dims: six warps work, the other two have neither
+    // steps nor a place in `part` (n_pq * hd <= 2 * kMaxHd for the groups that do).
     const int n_dg = hd >> 5;
     const int n_pq = kAttnWarps / n_dg;
     const int dg = warp % n_dg, pq = warp / n_dg;
+    const bool pv_warp = HD > 0 || pq < n_pq;
     int acc[MB][4][4], ones[MB][4];
     float psum[kRounds], mx[NB];
     int dc[NB][2];  // the "- 128" terms of this lane's two columns of every block
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                 if (HD == 128 && n_here == kTilePos) {  // two fixed steps per warp
                     pv_step(pq);
                     pv_step(pq + 2);
-                } else {
+                } else if (pv_warp) {
                     for (int ks = pq; 32 * ks < n_here; ks += n_pq) pv_step(ks);
                 }
             }
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                                 x += shfl_xor_ll(x, 4);
                                 x += shfl_xor_ll(x, 8);
                                 // MMA e, column n = dim 32 dg + 4 n + e; this lane holds n = 2t and 2t + 1
-                                if ((g & 3) == 0 && v < G)
+                                if ((g & 3) == 0 && v < G && pv_warp)
                                     sm.part[(pq * G + v) * hd + 32 * dg + 4 * (2 * t + cc) + e] = __fmul_rn(__ll2float_rn(x), wdown);
                             }
                         }

@@ -167,10 +167,13 @@ def test_kv_append_standalone_and_import_export(bt, oracle):
 
 
 @pytest.mark.parametrize("n_heads,n_kv,hd,t0,batch", [(32, 8, 128, 2040, 1), (32, 4, 64, 700, 1), (8, 8, 96, 300, 2),
-                                                         (32, 8, 128, 1500, 24)])
+                                                         (8, 4, 96, 27, 1), (8, 4, 96, 60, 3), (8, 2, 96, 123, 1), (8, 2, 96, 700, 80),
+                                                         (16, 2, 96, 300, 2), (32, 8, 128, 1500, 24)])
 def test_attention_long_context_many_spans(bt, oracle, n_heads, n_kv, hd, t0, batch):
     # a long seeded context: with one sequence the positions are cut over a whole cluster of spans
-    # (16 x 128 at 2048), with 24 sequences x 8 KV heads every CTA walks many tiles of its own
+    # (16 x 128 at 2048), with 24 sequences x 8 KV heads every CTA walks many tiles of its own; heads of 96 with one to
+    # eight query heads per KV head, whose eight warps do not divide into groups of 32 dims, in one span and in several,
+    # across lengths of 32, 64 and 128
     rng = np.random.default_rng(t0 + hd)
     max_seq = t0 + 16
     cache = bt.QuantizedKVCache(max_seq, batch, n_kv, hd)
