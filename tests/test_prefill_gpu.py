@@ -137,6 +137,38 @@ def test_prefill_errors(bt, syn):
     assert gpu.current_pos == 8
 
 
+@pytest.mark.parametrize("hidden,heads,kv_heads,ff,batch,n", [
+    (2048, 32, 4, 5632, 2, 592), (2048, 32, 4, 5632, 3, 400), (2048, 32, 4, 5632, 1, 300), (4096, 32, 8, 14336, 1, 260), (4096, 32, 8, 14336, 2, 300),
+    (1024, 8, 2, 3600, 3, 670)])
+def test_prefill_row_quantisers(bt, oracle, syn, hidden, heads, kv_heads, ff, batch, n):
+    # RMSNorm and SiLU * up of many rows, on both sides of the row counts and lengths at which another row kernel is taken; 3600
+    # inputs leave the last threads without values.  A trace wants silu(gate) * up in memory and takes it from the kernel that
+    # holds rows in shared memory: logits, and the second layer's cache rows (of every token), have to be the same
+    # bits; of some rows every stage is the oracle's.
+    cfg = syn.BitLlamaConfig("llama", 300, hidden, 2, heads, kv_heads, ff, max_position_embeddings=n)
+    w = syn.make_weights(cfg, seed=hidden + ff, from_latent=False)
+    gpu, ref = syn.build_model(w, max_batch=batch), oracle.model_from_weights(w)
+    tokens = np.random.default_rng(ff).integers(0, 300, (batch, n))
+
+    def prefill():
+        gpu.reset_kv_cache()
+        return [gpu.prefill(tokens)[0]] + [x for li in range(2) for b in range(batch) for x in gpu.kv_cache(li).export(b, n)]
+
+    plain = prefill()
+    gpu.set_trace(True, rows=batch * n)
+    for a, b in zip(plain, prefill()):
+        assert np.array_equal(a, b)
+    trace, rows = gpu.read_trace(batch * n), [0, 1, 131, batch * n - 1]
+    for L, t in zip(ref.layers, trace):
+        t = {name: x[rows] for name, x in t.items()}
+        xn = oracle.rmsnorm(t["h_in"], L.norm1, ref.cfg.rms_eps)
+        assert np.array_equal(t["qkv"], np.concatenate([L.q(xn), L.k(xn), L.v(xn)], axis=1))
+        xn = oracle.rmsnorm(t["h_mid"], L.norm2, ref.cfg.rms_eps)
+        assert rel_err(t["act"], oracle.silu_mul(L.gate(xn), L.up(xn))) <= 1e-6
+        assert np.array_equal(t["h_out"], t["h_mid"] + L.down(t["act"]))
+    assert bt.lib().bt_device_check(0) == 0
+
+
 def attention_64(qkv, rows, heads, kv_heads, hd, past, theta):
     """softmax(q k / sqrt(hd)) v in 64 bits for one sequence: qkv [n, (heads + 2 kv_heads) hd] before the rotation (its keys
     and values unused), rows = the cache's (k bytes, k scales, v bytes, v scales) up to the last new token."""
