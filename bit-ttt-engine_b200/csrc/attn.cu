@@ -115,7 +115,7 @@ struct AttnSmemT {
     float ml[2][G];                                         // this span's running maximum / denominator (read by the cluster)
     float corr[G];
     float wmax[kAttnWarps][G];
-    float wsum[kAttnWarps][(G + 7) / 8];
+    float wsum[kAttnWarps];
     float wvmax[kAttnWarps];
     float wup, wdown;                                       // weight scale of the chunk: 2^32 / B and B / 2^32
     float knew[kMaxHd], vnew[kMaxHd];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
     constexpr int kChunk = Smem::kChunk;
     constexpr int NB = Smem::kCols8 / 8;           // 8-column blocks of the score MMAs (two query vectors each)
     constexpr int MB = Smem::kRows16 / 16;         // 16-row blocks of the P.V MMAs (four query vectors each)
-    constexpr int kRounds = (G + kAttnWarps - 1) / kAttnWarps;  // weight rounds per tile: a warp turns one query vector's 128 scores into digits
+    static_assert(G <= kAttnWarps, "a warp turns one query vector's 128 scores of a tile into digits");
     constexpr bool kSplitDigits = 2 * G <= kAttnWarps;          // few vectors: two warps share one
     const int hd = HD > 0 ? HD : a.head_dim, half = hd >> 1;
     const int b = blockIdx.x / a.n_kv, kvh = blockIdx.x % a.n_kv;
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
     const int dg = warp % n_dg, pq = warp / n_dg;
     const bool pv_warp = HD > 0 || pq < n_pq;
     int acc[MB][4][4], ones[MB][4];
-    float psum[kRounds], mx[NB];
+    float psum, mx[NB];
     int dc[NB][2];  // the "- 128" terms of this lane's two columns of every block
     float qs[NB];   // and the scale of the query vector they belong to
 
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                 fetch(fc, cur >= 1 ? cur - 1 : kStages - 1);  // two tiles ahead = the buffer of the tile before (three buffers)
                 advance(fc);
                 const int n_here = min(kTilePos, clen - ti * kTilePos);
-                // FULL: a whole tile that every query may see (decode; all but the last tile of a span)
+                // FULL: a whole tile (all but the last one of a span)
                 auto score_tile = [&](auto full_tag) {
                     constexpr bool FULL = decltype(full_tag)::value;
                     if (!FULL && 16 * warp >= n_here) return;
@@ -494,13 +494,12 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[mb][e][0] = acc[mb][e][1] = acc[mb][e][2] = acc[mb][e][3] = 0;
             }
-#pragma unroll
-            for (int e = 0; e < kRounds; ++e) psum[e] = 0.0f;
+            psum = 0.0f;
             const float wup = sm.wup;
             for (int ti = 0; ti < ctiles; ++ti, cur = cur + 1 == kStages ? 0 : cur + 1) {
                 const int n_here = min(kTilePos, clen - ti * kTilePos);
                 uint8_t (*wd)[kWStride] = sm.wdig[ti & 1];
-                // weight digits of the tile: a warp takes one query vector per round, lane L the slots 4 L .. 4 L + 3 =
+                // weight digits of the tile: a warp takes one query vector, lane L the slots 4 L .. 4 L + 3 =
                 // positions 16 (L / 4) + 4 i + L % 4, i = 0..3: the four positions that one lane feeds into an MMA
                 // lie in one word, and so do the rows it reads from V.
                 const bool full_tile = n_here == kTilePos;
@@ -519,9 +518,9 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                         uint32_t u[2];
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
-                            const bool live = full_tile || (r0 + 4 * i < n_here && sv[i] != -INFINITY);
+                            const bool live = full_tile || r0 + 4 * i < n_here;  // (beyond the tile the buffer holds anything)
                             const float pe = live ? expf(__fsub_rn(sv[i], m_new)) : 0.0f;
-                            psum[0] += pe;
+                            psum += pe;
                             u[i] = live ? __float2uint_rn(__fmul_rn(__fmul_rn(pe, vv[i]), wup)) : 0u;
                         }
                         const uint32_t o0 = __shfl_xor_sync(0xffffffffu, u[0], 16), o1 = __shfl_xor_sync(0xffffffffu, u[1], 16);
@@ -532,9 +531,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                         *reinterpret_cast<uint32_t*>(&wd[4 * v + 2 * sub + 1][4 * wi]) = sub == 0 ? dig[2] : dig[0];
                     }
                 } else {
-#pragma unroll
-                for (int e = 0; e < kRounds; ++e) {
-                    const int v = warp + e * kAttnWarps;
+                    const int v = warp;
                     if (v < G) {  // warp-uniform
                         const float4 s4 = *reinterpret_cast<const float4*>(&sm.sbuf[v][ti * kTilePos + 4 * lane]);
                         const float4 v4 = *reinterpret_cast<const float4*>(&sm.vsc[ti * kTilePos + 4 * lane]);
@@ -544,10 +541,9 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                         uint32_t u[4], dig[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            // (beyond the tile the buffer holds anything; a masked score is -inf and gives exp = 0)
-                            const bool live = full_tile || (r0 + 4 * i < n_here && sv[i] != -INFINITY);
+                            const bool live = full_tile || r0 + 4 * i < n_here;
                             const float pe = live ? expf(__fsub_rn(sv[i], m_new)) : 0.0f;
-                            psum[e] += pe;
+                            psum += pe;
                             // weight of the value row: p * v_scale (the value bytes enter the MMA as integers)
                             u[i] = live ? __float2uint_rn(__fmul_rn(__fmul_rn(pe, vv[i]), wup)) : 0u;
                         }
@@ -555,7 +551,6 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
 #pragma unroll
                         for (int j = 0; j < 4; ++j) *reinterpret_cast<uint32_t*>(&wd[4 * v + j][4 * lane]) = dig[3 - j];
                     }
-                }
                 }
                 cp_async_wait<1>();
                 __syncthreads();  // the tile landed, its weight digits are complete; everybody is done with the tile before
@@ -617,11 +612,8 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                         }
                     }
                 }
-#pragma unroll
-                for (int e = 0; e < kRounds; ++e) {
-                    const float ws = warp_sum(psum[e]);
-                    if (lane == 0) sm.wsum[warp][e] = ws;  // query vector warp + 8 e (two warps per vector: warp / 2)
-                }
+                const float ws = warp_sum(psum);
+                if (lane == 0) sm.wsum[warp] = ws;  // query vector `warp` (two warps per vector: warp / 2)
             }
             __syncthreads();
             for (int it = tid; it < G * hd; it += kAttnThreads) {
@@ -631,7 +623,7 @@ __global__ void __launch_bounds__(kAttnThreads, NREP <= 4 ? 2 : 1) attn_kernel(A
                 sm.opart[it] = fmaf(sm.opart[it], sm.corr[v], add);
             }
             if (tid < G) {
-                const float ps = kSplitDigits ? __fadd_rn(sm.wsum[2 * tid][0], sm.wsum[2 * tid + 1][0]) : sm.wsum[tid % kAttnWarps][tid / kAttnWarps];
+                const float ps = kSplitDigits ? __fadd_rn(sm.wsum[2 * tid], sm.wsum[2 * tid + 1]) : sm.wsum[tid];
                 sm.ml[1][tid] = fmaf(sm.ml[1][tid], sm.corr[tid], ps);
             }
             __syncthreads();

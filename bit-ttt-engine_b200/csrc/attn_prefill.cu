@@ -521,12 +521,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
 template <int HD>
 __global__ void __launch_bounds__(256) prefill_rows_kernel(KvCacheView cache, float* __restrict__ qkv, const int32_t* __restrict__ pos,
                                                            const float* __restrict__ rope_cos, const float* __restrict__ rope_sin,
-                                                           int q_rows, int n_heads, int n_kv, float* __restrict__ qscale, int first_slot) {
+                                                           int q_rows, int n_heads, int n_kv, float* __restrict__ qscale) {
     constexpr int W = HD <= 32 ? 8 : (HD <= 64 ? 16 : 32), half = HD / 2;
     const int slots = n_heads + 2 * n_kv, lane = threadIdx.x % W;
     const int64_t row = blockIdx.x;
     const int b = (int)blockIdx.x / q_rows, p = pos[b] + (int)blockIdx.x % q_rows;
-    const int slot = first_slot + ((int)blockIdx.y * (int)blockDim.x + (int)threadIdx.x) / W;
+    const int slot = ((int)blockIdx.y * (int)blockDim.x + (int)threadIdx.x) / W;
     const bool active = slot < slots && 4 * lane < HD;
     float* src = qkv + row * (int64_t)slots * HD + (int64_t)slot * HD;
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -608,9 +608,8 @@ cudaError_t launch_rows_hd(const KvCacheView& cache, float* qkv, const int32_t* 
                            int q_rows, int n_heads, int n_kv, float* qscale, cudaStream_t stream) {
     if ((int64_t)batch * q_rows > (1 << 30)) return cudaErrorInvalidValue;
     constexpr int W = HD <= 32 ? 8 : (HD <= 64 ? 16 : 32);
-    const int first = qscale ? 0 : n_heads;
-    const dim3 grid((unsigned)(batch * q_rows), (unsigned)(((n_heads + 2 * n_kv - first) * W + 255) / 256));
-    prefill_rows_kernel<HD><<<grid, 256, 0, stream>>>(cache, qkv, pos, rope_cos, rope_sin, q_rows, n_heads, n_kv, qscale, first);
+    const dim3 grid((unsigned)(batch * q_rows), (unsigned)(((n_heads + 2 * n_kv) * W + 255) / 256));
+    prefill_rows_kernel<HD><<<grid, 256, 0, stream>>>(cache, qkv, pos, rope_cos, rope_sin, q_rows, n_heads, n_kv, qscale);
     return cudaGetLastError();
 }
 

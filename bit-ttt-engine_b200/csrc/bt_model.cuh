@@ -84,9 +84,9 @@ cudaError_t launch_row_quant_bf16(const __nv_bfloat16* x, int64_t x_stride, int 
 // Spans per (sequence, KV head) and positions per span for a cache of max_seq positions; rep = query
 // heads per KV head (selects the kernel instance whose cluster limit applies).
 void attn_plan(int64_t batch, int64_t n_kv, int64_t max_seq, int sm_count, int rep, int* splits, int* span);
-// Prefill.  The rows of q_rows new tokens per sequence (qkv rows [b][i], positions pos[b] + i) are made ready for the
-// attention: RoPE + Q8 append of the keys and values into the cache; with `qscale` ([rows][n_heads], else null) RoPE on the
-// queries too and their digits in place of their floats, for launch_prefill_attn.
+// Prefill.  The rows of q_rows new tokens per sequence (qkv rows [b][i], positions pos[b] + i) are made ready for
+// launch_prefill_attn: RoPE + Q8 append of the keys and values into the cache, RoPE on the queries and their digits in place
+// of their floats, qscale [rows][n_heads].
 cudaError_t launch_prefill_rows(const KvCacheView& cache, float* qkv, const int32_t* pos, const float* rope_cos, const float* rope_sin,
                                 int batch, int q_rows, int n_heads, int n_kv, int hd, float* qscale, cudaStream_t stream);
 struct PrefillAttnArgs {

@@ -869,9 +869,8 @@ bt_status enqueue_prefill_chunk(bt_model* m, int batch, int n, int past, int ttt
             BT_CUDA_TRY(launch_gemm_tc(L.qkv->dev(), nullptr, H, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_qkv, m->qkv_dim, EPI_F32, err, sm, s, true));
             BT_CUDA_TRY(trace_copy(m, li, TR_QKV, m->pf_qkv, M, s));
             const int rep = m->nh_l / m->nkv_l;
-            const bool blocks = n > 1;
-            BT_CUDA_TRY(launch_prefill_rows(L.kv->view, m->pf_qkv, m->pos, m->rope_cos, m->rope_sin, batch, n, m->nh_l, m->nkv_l, m->head_dim, blocks ? m->pf_qs : nullptr, s));
-            if (blocks) {
+            if (n > 1) {
+                BT_CUDA_TRY(launch_prefill_rows(L.kv->view, m->pf_qkv, m->pos, m->rope_cos, m->rope_sin, batch, n, m->nh_l, m->nkv_l, m->head_dim, m->pf_qs, s));
                 PrefillAttnArgs a = {};
                 a.qdig = reinterpret_cast<const uint8_t*>(m->pf_qkv);
                 a.qscale = m->pf_qs;
@@ -884,7 +883,7 @@ bt_status enqueue_prefill_chunk(bt_model* m, int batch, int n, int past, int ttt
                 a.scaling = (float)(1.0 / sqrt((double)m->head_dim));
                 a.err = err;
                 BT_CUDA_TRY(launch_prefill_attn(a, s));
-            } else {
+            } else {  // a single token: the decode kernel, which appends its rows itself
                 AttnArgs a;
                 a.qkv = m->pf_qkv;
                 a.cache = L.kv->view;
