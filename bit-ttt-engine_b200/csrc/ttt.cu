@@ -267,8 +267,8 @@ cudaError_t launch_pl(float* w, const float* feats, int batch, int t_len, int d,
 }  // namespace
 
 // States from which a lane takes two rows: there are several CTAs for every SM then (512 states of 128 x 128, chunks of four
-// tokens: 55.0 us with one row, 41.9 with two; 600 of 64 x 64, 33 tokens: 26.7 and 23.5).  With fewer a state's own latency
-// counts, and one row a lane has twice the warps for it.
+// tokens: 55.0 us with one row, 41.9 with two; 600 of 64 x 64, 33 tokens: 26.7 and 23.5; of 32 x 32, 16 tokens, 512: 10.3 and
+// 9.0, 8192: 94.5 and 82.4).  With fewer a state's own latency counts, and one row a lane has twice the warps for it.
 static constexpr int kManyStates = 512;
 
 cudaError_t launch_ttt_chunk(float* w, const float* feats, int batch, int t_len, int d, float lr, int chunk,
@@ -278,6 +278,7 @@ cudaError_t launch_ttt_chunk(float* w, const float* feats, int batch, int t_len,
     if (batch <= 0 || t_len <= 0) return cudaSuccess;
     const int pl = (d + 31) / 32;
     const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0;  // the row kernels load 16 bytes at a time
+    if (aligned && d == 32 && batch >= kManyStates) return launch_rows<2, 2>(w, feats, batch, t_len, d, lr, chunk, z_out, stream, absmax_out, pdl);
     if (aligned && d == 32) return launch_rows<2, 1>(w, feats, batch, t_len, d, lr, chunk, z_out, stream, absmax_out, pdl);
     if (aligned && d == 64 && batch >= kManyStates) return launch_rows<4, 2>(w, feats, batch, t_len, d, lr, chunk, z_out, stream, absmax_out, pdl);
     if (aligned && d == 64) return launch_rows<4, 1>(w, feats, batch, t_len, d, lr, chunk, z_out, stream, absmax_out, pdl);

@@ -53,7 +53,7 @@ def test_ttt_chunkwise(bt, oracle, t_len, chunk):
 
 
 @pytest.mark.parametrize("states", [511, 512, 700])
-@pytest.mark.parametrize("d,t_len,chunk", [(64, 16, 16), (64, 7, 1), (128, 5, 4), (128, 16, 16)])
+@pytest.mark.parametrize("d,t_len,chunk", [(32, 16, 16), (32, 7, 1), (64, 16, 16), (64, 7, 1), (128, 5, 4), (128, 16, 16)])
 def test_ttt_many_states_equal_few(bt, states, d, t_len, chunk):
     # from 512 states on a lane takes two rows: the same operations in the same order, so the same bits as the states in
     # small groups
