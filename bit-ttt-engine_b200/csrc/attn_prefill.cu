@@ -22,13 +22,13 @@
 // rescaled, and of all vectors where B changes.
 //
 // mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 227 us, 16 x 128 tokens 300 -> 57; 1B shape (heads of
-// 64), 4 x 511 tokens 298 -> 75 us, 16 x 128 tokens 231 -> 51; 2 tokens 10.7 -> 10.2; 16 tokens after 2000 51.9 -> 53.6.  The products
-// of 64 x 128 scores take 1 100 clocks: bound by the instructions of the softmax warps and the latency of a group's chain
-// scores - vote - weights - products, and by what an item begins and ends with.  Of the 227 us 39 are moves of references,
-// which random scores ask for in most tiles; a weight word with two bits left free for scores above the
-// reference needed hardly any, but a weight then had 30 bits.  With four softmax warps to a group (32
-// vectors a thread) the short items of heads of 64 took 1.5 times as long; scores and weights through integer conversion
-// instructions 1.1 times; columns read out by fours of vectors 235 us, by two vectors 228, unrolled 276.
+// 64), 4 x 511 tokens 298 -> 75 us, 16 x 128 tokens 231 -> 51; 2 tokens 10.7 -> 10.2; 16 tokens after 2000 51.9 -> 53.6.  Bound by the
+// instructions of the softmax warps (8B shape, 2048 tokens: issue slots 62 % busy, tensor pipe 15 %) and the latency of a
+// group's chain scores - vote - weights - products.  Of the 227 us about 40 are moves of references, which random
+// scores ask for in most tiles; a weight word with two bits left free for scores above the reference needed hardly any,
+// but a weight then had 30 bits.  With four softmax warps to a group (32 vectors a thread) the short items of heads of 64
+// took 1.5 times as long; scores and weights through integer conversion instructions 1.1 times; columns read out by fours of
+// vectors 235 us, by two vectors 228, unrolled 276.
 #include <cfloat>
 #include <type_traits>
 

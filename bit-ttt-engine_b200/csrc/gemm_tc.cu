@@ -9,9 +9,9 @@
 //   warp 0     producer: 1-D bulk copies of the packed weight tiles (8 x 1 KB per 256-input
 //              chunk) and of the chunk's int8 activation block into a shared-memory ring;
 //   warp 1     MMA issuer (one thread): tcgen05.mma.kind::i8 with the A operand (weights, u8) in
-//              TENSOR MEMORY and the B operand (activations, s8) in shared memory, K-major without
-//              swizzle; accumulators in tensor memory, two sets, so that the MMAs of the next unit
-//              run while the previous one is drained;
+//              TENSOR MEMORY and the B operand (activations, s8) in shared memory, K-major in the 64-byte
+//              swizzle; accumulators in tensor memory, two sets where there is room, so that the MMAs of the
+//              next unit run while the previous one is drained;
 //   8 unpack warps: a thread owns one weight row (= one TMEM lane) of one row set (with one row set, two warps per
 //              lane quarter take the chunks in turn).  It loads the row's 64
 //              packed bytes of the chunk, isolates field r of every byte with a shift and an AND (values 0, 1, 2 =
@@ -75,7 +75,7 @@ __device__ __forceinline__ uint32_t instr_desc_i8(int m, int n) {
 struct TcArgs {
     const uint8_t* tiles;      // one basis, tiled layout [row_tile][k_tile][1024]
     int64_t row_tiles, k_tiles, n_out;
-    const int8_t* qtc;         // activations: [token_block][k_tile][4 residues][NT/8][4][8][16]
+    const int8_t* qtc;         // activations: [token_block][k_tile][4 residues][NT tokens][64], swizzled (gemm_tc_act_offset)
     const int32_t* qsum;       // [m]
     const float* sx;           // [m]
     const float* sw_tiles;     // [row_tiles][2]

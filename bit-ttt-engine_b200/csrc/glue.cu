@@ -649,12 +649,14 @@ cudaError_t launch_embed(const int32_t* tokens, const __nv_bfloat16* table, int 
 // Rows that the kernel takes: the values and, for the tensor-core product, their bytes in shared memory.
 bool row_quant_fits(int64_t k, int64_t k_tiles) { return 4 * k + k_tiles * kTileK <= 200 * 1024; }
 
-// The kernel that keeps its values in registers: 2 groups of four values a thread where all such threads fit the GPU at once
-// (2048 a SM) and a row's own latency counts, 8 groups beyond that, where several rows share an SM in turn (2044 x 2048
-// RMSNorm: 12.2 us with 2 groups, 10.6 with 8; 64 x 4096: 4.3 and 7.7).  Few rows too wide for 512 threads of 2 groups stay
-// with the kernel above (64 rows x 14336, SiLU: 6.8 us there, 7.3 us with 8 groups a thread).
+// The kernel that keeps its values in registers: 2 groups of four values a thread while a row's own latency counts, 8 groups
+// beyond that, where several rows share an SM in turn (2044 x 2048 RMSNorm: 12.2 us with 2 groups, 10.6 with 8; 64 x 4096:
+// 4.3 and 7.7).  The line between them is a measured one, for the 148 SMs of a B200: 2048 threads of 2 groups a SM (of which
+// 1536 can be resident: 32 to 35 registers, 512 threads a CTA).  Few rows too wide for 512 threads of 2 groups stay with
+// the kernel above (64 rows x 14336, SiLU: 6.8 us there, 7.3 us with 8 groups a thread).
+static constexpr int64_t kFewRowGroups = 2ll * 148 * 2048;
 static int row_quant_groups(int batch, int groups) {  // groups per thread; 0: the kernel above
-    if ((int64_t)batch * groups <= 2ll * 148 * 2048) return groups <= 2 * 512 ? 2 : (batch >= 256 && groups <= 8 * 512 ? 8 : 0);
+    if ((int64_t)batch * groups <= kFewRowGroups) return groups <= 2 * 512 ? 2 : (batch >= 256 && groups <= 8 * 512 ? 8 : 0);
     return groups <= 8 * 512 ? 8 : 0;
 }
 

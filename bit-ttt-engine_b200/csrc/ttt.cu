@@ -112,10 +112,9 @@ __global__ void __launch_bounds__(kTttWarps * 32) ttt_chunk_kernel(float* __rest
 // not depend on the batch or on the run; only the L2 norm keeps its f64 sum.  f64 FMAs run at half the f32 rate on
 // this part and made the kernel arithmetic-bound at a sixth of the HBM bound.
 // ROWS = 2: a lane holds its 16 columns of two rows, so that a feature read from shared memory feeds four FMAs instead of
-// two.  With one row the reads bound the kernel once there are enough states to fill the GPU (17 wavefronts per token and
-// warp, 8 warps to a state): 8192 states of 64 x 64, 16 tokens 140.9 -> 118.9 us (2.8 TB/s), 7 tokens one by one 206 -> 157;
-// 2000 of 128 x 128 151.5 -> 123.8.
-
+// two.  With one row the reads bound the kernel once there are enough states to fill the GPU; with two they still take the
+// most of it (8192 states of 64 x 64, 16 tokens: shared memory and L1 at 71 % of their peak, DRAM 28 %, issue slots 55 %).
+// 8192 states of 64 x 64, 16 tokens 140 -> 118.5 us (2.8 TB/s), 7 tokens one by one 206 -> 157; 2000 of 128 x 128 150.5 -> 123.2.
 template <int LPR, int ROWS>
 __global__ void __launch_bounds__(kTttWarps / ROWS * 32, ROWS == 1 ? 3 : 4) ttt_rows_kernel(float* __restrict__ w,
                                                                     const float* __restrict__ feats,
