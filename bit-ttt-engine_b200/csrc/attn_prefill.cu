@@ -16,19 +16,20 @@
 // of the MN-major B operand.  Cache bytes only lose their offset of 128 on the way to shared memory (xor 0x80).
 // The 64 query vectors are two groups of 32 with eight softmax warps and an MMA warp each, so that one group's softmax runs
 // under the other's MMAs; four loader warps fill a ring of three K | V tiles.
-// Softmax reference of a vector: the largest score so far, or one that a score exceeds by less than what the power of two B
-// leaves free (a weight is below B then, and U below 2^32).  While it holds, the integer accumulators run on from tile to
+// Softmax reference of a vector: the largest score so far, or one that a score exceeds by less than what B leaves free above
+// its position's value scale (a weight is below B then, and U below 2^32).  While it holds, the integer accumulators run on from tile to
 // tile; where a score breaks it, that vector's four columns are read out, joined into f32 sums in shared memory and
 // rescaled, and of all vectors where B changes.
 //
-// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 227 us, 16 x 128 tokens 300 -> 57; 1B shape (heads of
-// 64), 4 x 511 tokens 298 -> 75 us, 16 x 128 tokens 231 -> 51; 2 tokens 10.7 -> 10.2; 16 tokens after 2000 51.9 -> 53.6.  Bound by the
+// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 206 us, 16 x 128 tokens 300 -> 57; 1B shape (heads of
+// 64), 4 x 511 tokens 298 -> 74 us, 16 x 128 tokens 231 -> 50; 2 tokens 10.7 -> 10.0; 16 tokens after 2000 51.9 -> 49.2.  Bound by the
 // instructions of the softmax warps (8B shape, 2048 tokens: issue slots 62 % busy, tensor pipe 15 %) and the latency of a
-// group's chain scores - vote - weights - products.  Of the 227 us about 40 are moves of references, which random
-// scores ask for in most tiles; a weight word with two bits left free for scores above the reference needed hardly any,
-// but a weight then had 30 bits.  With four softmax warps to a group (32 vectors a thread) the short items of heads of 64
-// took 1.5 times as long; scores and weights through integer conversion instructions 1.1 times; columns read out by fours of
-// vectors 235 us, by two vectors 228, unrolled 276.
+// group's chain scores - vote - weights - products.  Random scores ask for moves of references in most tiles; a weight word
+// with two bits left free for scores above the reference needed hardly any (184 us), but a weight then had 30 bits.  Room by
+// position instead of by the largest scale of the bound's tiles, and f32 sums that start at zero instead of being selected: 227 -> 206.
+// With four softmax warps to a group (32 vectors a thread) the short items of heads of 64 took 1.5 times as long; scores
+// and weights through integer conversion instructions 1.1 times; columns read out by fours of vectors 1.05 times, unrolled
+// 1.2; warps without dims (heads of 64) sent past the read-outs 1.08.
 #include <cfloat>
 #include <type_traits>
 
@@ -224,15 +225,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
             }
             float l[kHalfVec], s[kHalfVec];
 #pragma unroll
-            for (int v = 0; v < kHalfVec; ++v) l[v] = 0.0f;
-            uint32_t kept = 0;            // vectors of which osum holds something
+            for (int v = 0; v < kHalfVec; ++v) {
+                l[v] = 0.0f;
+                sm.osum[g][h0 + v][r] = 0.0f;
+            }
             uint32_t ex = 0, ex_new = 0;  // exponent of the weight bound, of these tiles and of the next kBoundTiles
             float up = 0.0f, down = 0.0f, room = 0.0f;  // room: how far a score may exceed its reference
             ptx::named_bar_sync(bar_id, kHalfThreads);
             // of vector v, whose four digit columns are b: the accumulator as f32, joined with what was read out before
             auto joined = [&](const uint32_t* b, int v) {
                 const long long sum = (long long)(int)b[3] * (1 << 24) + ((long long)(int)b[2] * (1 << 16) + ((long long)(int)b[1] * (1 << 8) + (int)b[0]));
-                return fmaf(__ll2float_rn(sum), down, kept >> v & 1 ? sm.osum[g][h0 + v][r] : 0.0f);
+                return fmaf(__ll2float_rn(sum), down, sm.osum[g][h0 + v][r]);
             };
             // lane v % 16 ends with the warp's join of vector h0 + v (x is consumed)
             auto across = [&](float (&x)[kHalfVec], auto join) {
@@ -264,6 +267,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                 }
                 wait(&sm.s_full[g], n);
                 ptx::tc_fence_after();
+                // How far this position's scores may exceed their references: its weights are below the bound while the exponential
+                // is below bound / scale (the bound of this tile, already; the first tile sets the references).  2^-16 is more than
+                // the errors of the logarithm and the exponential.
+                const float share = __fmul_rn(v_scale, __uint_as_float((270 - ex_new) << 23));  // scale / bound * 2^16
+                const float room_here = t > 0 ? fmaxf(room, fminf(11.0903549f - __logf(share) - 1.0f / 65536.0f, 0.69f)) : 0.0f;
                 const float v_most = fmaxf(fmaxf(v_look[0], v_look[1]), fmaxf(v_look[2], v_look[3]));
                 bool over = false;  // some score is too far above its reference
                 auto scores = [&](auto masked_tag) {
@@ -288,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                             float x = __fmul_rn(__fmul_rn(fmaf(hi, 16384.0f, lo), k_scale), cqv[i]);
                             if (kMasked && at > lastv[i]) x = -INFINITY;
                             s[4 * c + i] = x;
-                            over |= __fsub_rn(x, mrv[i]) > room;
+                            over |= __fsub_rn(x, mrv[i]) > room_here;
                         }
                     }
                 };
@@ -356,7 +364,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_attn_kernel(PrefillAttnAr
                         sm.osum[g][h0 + v][r] = joined(d, v) * (move ? sm.fac[g][h0 + v] : 1.0f);
                     }
                     ptx::tmem_st_wait();
-                    kept |= which;
                 }
                 if (new_bound) {
                     ex = ex_new;
