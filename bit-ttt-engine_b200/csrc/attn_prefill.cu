@@ -21,9 +21,9 @@
 // tile; where a score breaks it, that vector's four columns are read out, joined into f32 sums in shared memory and
 // rescaled, and of all vectors where B changes.
 //
-// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 206 us, 16 x 128 tokens 300 -> 57; 1B shape (heads of
-// 64), 4 x 511 tokens 298 -> 74 us, 16 x 128 tokens 231 -> 50; 2 tokens 10.7 -> 10.0; 16 tokens after 2000 51.9 -> 49.2.  Bound by the
-// instructions of the softmax warps (8B shape, 2048 tokens: issue slots 62 % busy, tensor pipe 15 %) and the latency of a
+// mma.sync form -> this (a layer's launch): 8B shape, 2048 tokens 868 -> 204 us, 16 x 128 tokens 300 -> 56; 1B shape (heads of
+// 64), 4 x 511 tokens 298 -> 73 us, 16 x 128 tokens 231 -> 50; 2 tokens 10.7 -> 10.3; 16 tokens after 2000 51.9 -> 48.5.  Bound by the
+// instructions of the softmax warps (8B shape, 2048 tokens: issue slots 63 % busy, tensor pipe 17 %) and the latency of a
 // group's chain scores - vote - weights - products.  Random scores ask for moves of references in most tiles; a weight word
 // with two bits left free for scores above the reference needed hardly any (184 us), but a weight then had 30 bits.  Room by
 // position instead of by the largest scale of the bound's tiles, and f32 sums that start at zero instead of being selected: 227 -> 206.
