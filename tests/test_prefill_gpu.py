@@ -230,6 +230,10 @@ def steered_rows(rng, kind, q, past):
         return rows_for_scores(rng, q, at / 40)
     if kind == "falling":
         return rows_for_scores(rng, q, -at / 40)
+    if kind == "creeping":   # a little more from tile to tile, value scales just below and just above a power of two
+        rows = rows_for_scores(rng, q, 3 + at / 1500)
+        rows[3] = rng.choice(np.nextafter(np.float32([2.0 ** -6, 2.0 ** -7, 0.011]), np.float32([0, 1, 1])), rows[3].shape)
+        return rows
     if kind in ("1e6", "1e7", "1e8"):  # scores of which an f32 holds the difference to the maximum in a few bits, or hardly at all
         return rows_for_scores(rng, q, float(kind) + rng.integers(0, 4, past) + at // 128)
     if kind == "small sums":  # the largest weight belongs to a row of zeros; what is left are small negative sums
@@ -248,7 +252,7 @@ def steered_rows(rng, kind, q, past):
 
 
 @pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 32), (4, 2, 64), (8, 2, 128), (8, 1, 96)])
-@pytest.mark.parametrize("kind,past", [("growing", 600), ("falling", 600), ("1e6", 600), ("1e7", 600), ("1e8", 600), ("value scales", 1400),
+@pytest.mark.parametrize("kind,past", [("growing", 600), ("falling", 600), ("creeping", 2000), ("1e6", 600), ("1e7", 600), ("1e8", 600), ("value scales", 1400),
                                        ("odd scales", 700), ("small sums", 140), ("random", 513), ("random", 33000)])
 def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, past):
     # Peaked, huge and unequal rows, where the reference of the weights and their bound move, and more tiles than the
