@@ -52,6 +52,7 @@ __host__ __device__ constexpr int tc_threads(int rs) { return (tc_lead_warps(rs)
 // Register split of the 128-token, two-row-set kernel: the epilogue warps hold a whole accumulator row (128 values) so
 // that the single accumulator set is free again after four tensor-memory loads instead of after the stores.
 constexpr int kRegsLead = 40, kRegsUnpack = 64, kRegsEpilogue = 152;
+__host__ __device__ constexpr bool tc_reg_split(int nt, int rs, int s, bool pair) { return pair || (nt == 128 && rs == 2 && s == 1); }
 __host__ __device__ constexpr int tc_abufs(int rs) { return rs == 1 ? 4 : 2; }           // unpacked-A buffers in tensor memory
 __host__ __device__ constexpr int tc_acc_sets(int nt, int rs) { return (2 * rs * nt + tc_abufs(rs) * rs * kAChunkCols <= 512) ? 2 : 1; }
 __host__ __device__ constexpr int tc_stages(int nt, int rs, int s) {
@@ -60,6 +61,17 @@ __host__ __device__ constexpr int tc_stages(int nt, int rs, int s) {
     const int n = (225 * 1024 - part) / stage;
     return n > 5 ? 5 : n;
 }
+
+// A CTA pair's tile: 256 rows x 256 tokens, an MMA of 256 x 256 x 32 over both SMs.  Each CTA unpacks 128 rows and pulls in the
+// activations of 128 of the tokens, which both tensor cores read: per product 160 bytes of a k step against the 192 of a single
+// CTA's 256 x 128 tile, and half the unpacked weights and half the MMAs, whose issue and whose contention with the stores
+// to tensor memory bound that tile (97 clocks of an MMA of 64).  A chunk of 256 inputs takes 1 400 to 1 900 clocks here, 1 032 of
+// them MMAs; without its copies, or without its stores to tensor memory, or without the stores of the results it would be 5 to
+// 20 % less (builds that are not in the tree): no single one bounds it.  Between two tiles the MMAs stop for 3 000 clocks, until
+// the accumulators are in registers.
+// Per launch, single CTAs -> pairs (us, f32 outputs): 2048 x 14336 -> 4096 129.2 -> 108.3, 4096 tokens 248 -> 202; 2048 x 4096 ->
+// 4096 43.2 -> 40.0, -> 6144 60.6 -> 56.0; 2048 x 5632 -> 2048 31.8 -> 29.6; 2048 x 2048 -> 11264 57.6 -> 57.2.
+constexpr int kPairTokens = 256;
 
 // Instruction descriptor for kind::i8: D = s32, A = u8, B = s8, both K-major, M x N tile.
 __device__ __forceinline__ uint32_t instr_desc_i8(int m, int n) {
@@ -89,22 +101,25 @@ struct TcArgs {
 
 // NT: tokens per tile (64 / 128).  RS: 128-row sets per tile (1 / 2).  S: CTAs of a cluster that share a tile
 // along k (1: no cluster work at all).
-template <int NT, int RS, int S>
-__global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
+// PAIR: the cluster is a CTA pair that works on one tile of 256 rows x 256 tokens (see kPairTokens).
+template <int NT, int RS, int S, bool PAIR>
+__global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(TcArgs a) {
     static_assert(S == 1 || (NT == 64 && (S == 2 || S == 4 || S == 8)), "k split: 64 tokens, 2 / 4 / 8 CTAs");
+    static_assert(!PAIR || (NT == 128 && RS == 1 && S == 1), "a CTA of a pair: 128 rows and the activations of 128 tokens");
     // Eight unpack warps.  RS = 2: one per (row set, TMEM lane quarter).  RS = 1: two per lane quarter, which take
     // the chunks in turn (two independent chains of load - unpack - store, four A buffers).
-    constexpr int kUnpackWarps = 8, kEpiWarps = 4 * RS, kUnpackWarp0 = tc_lead_warps(RS), kEpiWarp0 = kUnpackWarp0 + kUnpackWarps;
-    constexpr bool kRegSplit = NT == 128 && RS == 2 && S == 1;
+    constexpr int kUnpackWarps = 8, kEpiWarps = PAIR ? 8 : 4 * RS, kUnpackWarp0 = tc_lead_warps(PAIR ? 2 : RS), kEpiWarp0 = kUnpackWarp0 + kUnpackWarps;
+    constexpr bool kRegSplit = tc_reg_split(NT, RS, S, PAIR);
     constexpr int kABufs = tc_abufs(RS);
     constexpr int kReaders = RS == 1 ? 4 : 8;            // unpack warps that read one stage's weights and fill one A buffer
     constexpr int kStages = tc_stages(NT, RS, S);
-    constexpr int kAccSets = tc_acc_sets(NT, RS);
+    constexpr int kAccSets = PAIR ? 1 : tc_acc_sets(NT, RS);
     constexpr int kRawBytes = RS * kSetBytes;
     constexpr int kBBytes = 4 * NT * 64;                 // activation block of a chunk (4 residues)
     constexpr int kStageBytes = kRawBytes + kBBytes;
     constexpr int kPartBytes = S > 1 ? RS * kRows * NT * 4 : 0;  // this CTA's partial sums of a tile, read by the whole cluster
-    constexpr uint32_t kAccCols = kAccSets * RS * NT;
+    constexpr uint32_t kAccCols = PAIR ? kPairTokens : kAccSets * RS * NT;
+    constexpr int kTokSets = PAIR ? 2 : 1;               // token halves of the tile, drained by different warps
     constexpr uint32_t kTmemCols = (kAccCols + kABufs * RS * kAChunkCols) <= 256 ? 256 : 512;
     static_assert(kAccCols + kABufs * RS * kAChunkCols <= 512, "tensor memory");
     static_assert(kStages >= 3, "ring");
@@ -121,38 +136,44 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
     uint64_t* red_full = acc_empty + 2;   // every CTA of the cluster has parked its partial sums of the tile
     uint64_t* red_free = red_full + 1;    // every CTA of the cluster has read this CTA's partial sums
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_free + 1);
-    int* tok_qsum = reinterpret_cast<int*>(tmem_slot + 2);          // [2][NT] per-token sum of q and scale of the tile being drained
-    float* tok_sx = reinterpret_cast<float*>(tok_qsum + 2 * NT);    // (two copies: the row sets' warps may be one tile apart)
+    int* tok_qsum = reinterpret_cast<int*>(tmem_slot + 2);          // [2][kTokSets][NT] per-token sum of q and scale of the tile being drained
+    float* tok_sx = reinterpret_cast<float*>(tok_qsum + 2 * kTokSets * NT);  // (two copies: the row sets' warps may be one tile apart)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_tiles = (int)a.k_tiles;
-    const int row_sets = (int)((a.row_tiles + 8 * RS - 1) / (8 * RS));   // tiles along the rows
-    const int tok_blocks = (a.m + NT - 1) / NT;
-    const int rank = S > 1 ? (int)ptx::cluster_ctarank() : 0;
-    const int cid = blockIdx.x / S, n_clusters = gridDim.x / S;
+    constexpr int kTileSets = PAIR ? 2 : RS, kTileTokens = PAIR ? kPairTokens : NT, kCtas = PAIR ? 2 : S;
+    const int row_sets = (int)((a.row_tiles + 8 * kTileSets - 1) / (8 * kTileSets));   // tiles along the rows
+    const int tok_blocks = (a.m + kTileTokens - 1) / kTileTokens;
+    const int rank = kCtas > 1 ? (int)ptx::cluster_ctarank() : 0;
+    const int cid = blockIdx.x / kCtas, n_clusters = gridDim.x / kCtas;
     const int cps = (k_tiles + S - 1) / S;                 // chunks per split (the host makes every split non-empty)
-    const int kt0 = rank * cps, kt1 = min(k_tiles, kt0 + cps);
+    const int kt0 = PAIR ? 0 : rank * cps, kt1 = min(k_tiles, kt0 + cps);
     const int n_tiles = row_sets * tok_blocks;             // this CTA works on the tiles cid, cid + n_clusters, ...
+    // this CTA's row tiles of a tile begin at row_tile0(rs): rts(rs) of them exist (none, where the matrix ends in the first half)
+    auto row_tile0 = [&](int rs) -> int64_t { return (int64_t)rs * (8 * kTileSets) + (PAIR ? 8 * rank : 0); };
+    auto row_tiles_of = [&](int rs) -> int { return max(0, min(8 * RS, (int)(a.row_tiles - row_tile0(rs)))); };
 
     if (warp == 0) {  // the barriers side by side, a lane each (the set-up is on the path of every launch)
         if (lane < kStages) { ptx::mbar_init(&full[lane], 1); ptx::mbar_init(&empty[lane], 1 + kReaders); }
-        if (lane >= 8 && lane < 8 + kABufs) { ptx::mbar_init(&a_full[lane - 8], kReaders); ptx::mbar_init(&a_empty[lane - 8], 1); }
-        if (lane >= 16 && lane < 18) { ptx::mbar_init(&acc_full[lane - 16], 1); ptx::mbar_init(&acc_empty[lane - 16], kEpiWarps); }
+        // (of a pair, rank 0's a_full and acc_empty count the warps of both CTAs)
+        if (lane >= 8 && lane < 8 + kABufs) { ptx::mbar_init(&a_full[lane - 8], kReaders * (PAIR ? 2 : 1)); ptx::mbar_init(&a_empty[lane - 8], 1); }
+        if (lane >= 16 && lane < 18) { ptx::mbar_init(&acc_full[lane - 16], 1); ptx::mbar_init(&acc_empty[lane - 16], kEpiWarps * (PAIR ? 2 : 1)); }
         if (lane == 24) ptx::mbar_init(red_full, kEpiWarps * S);
         if (lane == 25) ptx::mbar_init(red_free, kEpiWarps * S);
         ptx::mbar_fence_init();
     }
     if (warp == 1) {  // one warp allocates (and later frees) the tensor memory
-        ptx::tmem_alloc(tmem_slot, kTmemCols);
-        ptx::tmem_relinquish();
+        if constexpr (PAIR) { ptx::tmem_alloc_pair(tmem_slot, kTmemCols); ptx::tmem_relinquish_pair(); }
+        else { ptx::tmem_alloc(tmem_slot, kTmemCols); ptx::tmem_relinquish(); }
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
     // The peers' barriers must exist before anybody arrives on them.  Only the epilogue warps ever touch a peer, so
     // everybody reports here and only they wait (at the top of their role): the cluster's start-up skew stays off
-    // the path of the first copies and MMAs.
-    if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // the path of the first copies and MMAs.  (Of a pair every warp waits, the producer after its first requests: the
+    // unpack warps and the commits arrive on the peer's barriers too, and the closing cluster barrier takes everybody.)
+    if (S > 1 || PAIR) ptx::cluster_arrive();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t a_col0 = kAccCols;  // the unpacked-A buffers follow the accumulators: [buffer][row set][64]
 
@@ -170,18 +191,21 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
             auto issue = [&](int tile, int kt, int slot, bool raw_part, bool b_part) {
                 const int rs = tile % row_sets, tb = tile / row_sets;
                 uint8_t* st = stage_base + (size_t)slot * kStageBytes;
-                const int rts = min(8 * RS, (int)(a.row_tiles - (int64_t)rs * 8 * RS));
+                const int rts = row_tiles_of(rs);
                 if (raw_part) {
                     if (lane == 0) ptx::mbar_arrive_expect_tx(&full[slot], (uint32_t)(rts * kTileBytes + kBBytes));
                     if (lane < rts)
-                        ptx::bulk_g2s(st + lane * kTileBytes, a.tiles + (((int64_t)rs * 8 * RS + lane) * k_tiles + kt) * kTileBytes, kTileBytes,
+                        ptx::bulk_g2s(st + lane * kTileBytes, a.tiles + ((row_tile0(rs) + lane) * k_tiles + kt) * kTileBytes, kTileBytes,
                                       &full[slot]);
                 }
-                if (b_part && lane == 0) ptx::bulk_g2s(st + kRawBytes, a.qtc + ((int64_t)tb * k_tiles + kt) * kBBytes, kBBytes, &full[slot]);
+                // (a pair's second half may lie behind the last token block: it reads that block again, nothing of it is stored)
+                const int blk = PAIR ? min(2 * tb + rank, (a.m + NT - 1) / NT - 1) : tb;
+                if (b_part && lane == 0) ptx::bulk_g2s(st + kRawBytes, a.qtc + ((int64_t)blk * k_tiles + kt) * kBBytes, kBBytes, &full[slot]);
             };
             int g = 0;
             for (int tile = cid; tile < n_tiles && g < kStages; tile += n_clusters)
                 for (int kt = kt0; kt < kt1 && g < kStages; ++kt, ++g) issue(tile, kt, g, true, false);
+            if constexpr (PAIR) { __syncwarp(); ptx::cluster_wait(); }
             ptx::pdl_wait();
             g = 0;
             for (int tile = cid; tile < n_tiles; tile += n_clusters) {
@@ -194,10 +218,17 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // ---------------- MMA issuer (of a pair: rank 0's) ----------------
+        if constexpr (PAIR) ptx::cluster_wait();
+        if (PAIR && rank != 0) {
+            if (lane == 0) ptx::pdl_launch_dependents();  // (rank 0 issues the MMAs and says when the kernel behind may start)
+        } else if (lane == 0) {
             ptx::pdl_wait();  // nothing to do before the first activation block exists; keeps the bounded waits short
-            const uint32_t idesc = instr_desc_i8(kRows, NT);
+            const uint32_t idesc = PAIR ? instr_desc_i8(2 * kRows, kPairTokens) : instr_desc_i8(kRows, NT);
+            auto commit = [&](uint64_t* bar) {
+                if constexpr (PAIR) ptx::umma_commit_pair(bar);
+                else ptx::umma_commit(bar);
+            };
             int g = 0, tl = 0;
             for (int tile = cid; tile < n_tiles; tile += n_clusters, ++tl) {
                 const int sel = tl % kAccSets, acc_use = tl / kAccSets;
@@ -220,18 +251,22 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
 #pragma unroll
                             for (int ks = 0; ks < 2; ++ks) {  // 64 k' per residue = 2 x K32 = 2 x 8 TMEM columns
                                 const uint64_t bd = ptx::smem_desc_sw64(b_addr + r * (NT * 64) + ks * 32, 512);
-                                ptx::umma_i8_ts(d_tmem, a_tmem + r * 16 + ks * 8, bd, idesc, (kt > kt0 || r > 0 || ks > 0) ? 1u : 0u);
+                                const uint32_t add = (kt > kt0 || r > 0 || ks > 0) ? 1u : 0u;
+                                if constexpr (PAIR) ptx::umma_i8_ts_pair(d_tmem, a_tmem + r * 16 + ks * 8, bd, idesc, add);
+                                else ptx::umma_i8_ts(d_tmem, a_tmem + r * 16 + ks * 8, bd, idesc, add);
                             }
                         }
                     }
-                    ptx::umma_commit(&a_empty[u]);   // unpacked buffer reusable once these MMAs are done
-                    ptx::umma_commit(&empty[slot]);  // and the stage's activation block
+                    commit(&a_empty[u]);   // unpacked buffer reusable once these MMAs are done
+                    commit(&empty[slot]);  // and the stage's activation block
                 }
-                ptx::umma_commit(&acc_full[sel]);
+                commit(&acc_full[sel]);
             }
             // every MMA of this CTA is issued: the kernel behind may start (it waits for this one's results itself)
             ptx::pdl_launch_dependents();
         }
+    } else {
+        if constexpr (PAIR) ptx::cluster_wait();  // (the idle warps of the leading warpgroup)
     }
     } else if (warp < kEpiWarp0) {
         if constexpr (kRegSplit) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsUnpack));
@@ -244,6 +279,7 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
         // 16-byte pieces t = 0..3 at ((half*32 + g*4 + t) * 16) of the row tile
         const int r8 = h * 8 + (row >> 4), half = (row >> 3) & 1, g8 = row & 7;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(sub * 32) << 16) + a_col0 + (uint32_t)h * kAChunkCols;
+        if constexpr (PAIR) ptx::cluster_wait();
         ptx::pdl_wait();
         int g = 0;
         int pending = -1;  // A buffer whose stores are issued but not yet published
@@ -254,12 +290,15 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
             ptx::tmem_st_wait();
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&a_full[pending]);
+            if (lane == 0) {
+                if constexpr (PAIR) ptx::mbar_arrive_remote(ptx::map_to_rank(&a_full[pending], 0));
+                else ptx::mbar_arrive(&a_full[pending]);
+            }
             pending = -1;
         };
         for (int tile = cid; tile < n_tiles; tile += n_clusters) {
             const int rs = tile % row_sets;
-            const int rts = min(8 * RS, (int)(a.row_tiles - (int64_t)rs * 8 * RS));
+            const int rts = row_tiles_of(rs);
             for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 if (RS == 1 && (g & 1) != set) continue;
                 const int slot = g % kStages, u = g % kABufs, a_use = g / kABufs;
@@ -301,10 +340,10 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
         if constexpr (kRegSplit) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
         // ---------------- epilogue warps (4 per row set, TMEM lanes by warp % 4) ----------------
         const int sub = warp & 3;
-        const int h = (warp - kEpiWarp0) >> 2;  // row set of the tile
+        const int h = (warp - kEpiWarp0) >> 2;  // row set of the tile; of a pair: token half
         const int lrow = sub * 32 + lane;       // row inside the set
         int32_t* pb = pbuf + (size_t)h * (kRows * NT);
-        if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (S > 1 || PAIR) ptx::cluster_wait();
         ptx::pdl_wait();  // the output (and what EPI_F32_ACCUM adds to) belongs to earlier kernels until here
         // The old value of an accumulated output is fetched apart from its update, so that a thread's loads are all
         // in flight before the first store (a store followed by a load of the same array would serialise them);
@@ -320,10 +359,11 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
         };
         // i = token inside the tile; tq / ts = the tile's staged per-token terms
         // tqi / tsi: the token's sum of q and scale (read from shared memory by the caller, ahead of its stores)
-        auto store_v = [&](int tqi, float tsi, int tb, int i, int n_tok, int64_t row, float sw, uint32_t acc, float old) {
+        // (tok0: the first token of those that this warp drains)
+        auto store_v = [&](int tqi, float tsi, int tok0, int i, int n_tok, int64_t row, float sw, uint32_t acc, float old) {
             if (i < n_tok && row < a.n_out) {
                 const int accv = (int)acc - tqi;
-                const int64_t o = (int64_t)(tb * NT + i) * a.out_stride + row;
+                const int64_t o = (int64_t)(tok0 + i) * a.out_stride + row;
                 if constexpr (EPI == EPI_I32) {
                     reinterpret_cast<int32_t*>(a.out)[o] = accv;
                 } else {
@@ -335,20 +375,27 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
                 }
             }
         };
-        auto store = [&](const int* tq, const float* ts, int tb, int i, int n_tok, int64_t row, float sw, uint32_t acc, float old) {
-            store_v(tq[i], ts[i], tb, i, n_tok, row, sw, acc, old);
+        auto store = [&](const int* tq, const float* ts, int tok0, int i, int n_tok, int64_t row, float sw, uint32_t acc, float old) {
+            store_v(tq[i], ts[i], tok0, i, n_tok, row, sw, acc, old);
+        };
+        // a set of accumulator columns has been read: the MMA issuer may write it again
+        auto free_set = [&](int sel) {
+            if constexpr (PAIR) ptx::mbar_arrive_remote(ptx::map_to_rank(&acc_empty[sel], 0));
+            else ptx::mbar_arrive(&acc_empty[sel]);
         };
         int tl = 0;
         for (int tile = cid; tile < n_tiles; tile += n_clusters, ++tl) {
             const int rs = tile % row_sets, tb = tile / row_sets;
             const int sel = tl % kAccSets;
             // the tile's per-token terms, once per row set's four warps into shared memory (named barrier 1 + h)
+            const int tok0 = PAIR ? tb * kPairTokens + h * NT : tb * NT;
+            const int tset = ((tl & 1) * kTokSets + (PAIR ? h : 0)) * NT;
             {
-                int* tq = tok_qsum + (tl & 1) * NT;
-                float* ts = tok_sx + (tl & 1) * NT;
+                int* tq = tok_qsum + tset;
+                float* ts = tok_sx + tset;
                 if (h == 0 || RS == 1) {
                     for (int i = lrow; i < NT; i += kRows) {
-                        const int token = tb * NT + i;
+                        const int token = tok0 + i;
                         tq[i] = token < a.m ? __ldg(a.qsum + token) : 0;
                         ts[i] = (token < a.m && EPI != EPI_I32) ? __ldg(a.sx + token) : 0.0f;
                     }
@@ -357,14 +404,14 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
             }
             ok &= ptx::mbar_wait_bounded(&acc_full[sel], (uint32_t)((tl / kAccSets) & 1));
             ptx::tc_fence_after();
-            const int* tq = tok_qsum + (tl & 1) * NT;
-            const float* ts = tok_sx + (tl & 1) * NT;
-            const int64_t row = ((int64_t)rs * RS + h) * kRows + lrow;
+            const int* tq = tok_qsum + tset;
+            const float* ts = tok_sx + tset;
+            const int64_t row = PAIR ? ((int64_t)rs * 2 + rank) * kRows + lrow : ((int64_t)rs * RS + h) * kRows + lrow;
             const int64_t rt = row >> 4;
             float sw = 0.f;
             if (EPI != EPI_I32 && rt < a.row_tiles) sw = __ldg(a.sw_tiles + 2 * rt + ((row >> 3) & 1));
             const uint32_t acc_addr = tmem_base + ((uint32_t)(sub * 32) << 16) + (uint32_t)(sel * RS + h) * NT;
-            const int n_tok = min(NT, a.m - tb * NT);  // tokens of this tile that exist
+            const int n_tok = min(NT, a.m - tok0);  // tokens of these that exist
             bool drained = false;
             if constexpr (kRegSplit && EPI != EPI_I32) {
                 // Whole tiles: this thread's whole accumulator row goes to registers and the set is handed back to the MMA
@@ -381,9 +428,9 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
                     ptx::tmem_ld_wait();
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&acc_empty[sel]);
+                    if (lane == 0) free_set(sel);
                     using Out = std::conditional_t<EPI == EPI_BF16 || EPI == kEpiBf16Accum, __nv_bfloat16, float>;
-                    const int64_t stride = a.out_stride, at = (int64_t)(tb * NT) * stride + row;
+                    const int64_t stride = a.out_stride, at = (int64_t)tok0 * stride + row;
                     Out* po = reinterpret_cast<Out*>(a.out) + at;
                     auto put = [&](int i, float y) {
                         if constexpr (std::is_same_v<Out, float>) po[i * stride] = y;
@@ -416,10 +463,10 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
                         float old[16];
                         ptx::tmem_ld16(acc_addr + c0, d);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) old[j] = load_old(tb * NT + c0 + j, row);
+                        for (int j = 0; j < 16; ++j) old[j] = load_old(tok0 + c0 + j, row);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) store(tq, ts, tb, c0 + j, n_tok, row, sw, d[j], old[j]);
+                        for (int j = 0; j < 16; ++j) store(tq, ts, tok0, c0 + j, n_tok, row, sw, d[j], old[j]);
                     }
                 } else {
 #pragma unroll 1
@@ -428,12 +475,12 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
                         ptx::tmem_ld32(acc_addr + c0, d);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) store(tq, ts, tb, c0 + j, n_tok, row, sw, d[j], 0.0f);
+                        for (int j = 0; j < 32; ++j) store(tq, ts, tok0, c0 + j, n_tok, row, sw, d[j], 0.0f);
                     }
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&acc_empty[sel]);
+                if (lane == 0) free_set(sel);
             } else {
                 // Reduce-scatter over the cluster: every CTA parks its partial sums of the whole tile in its own
                 // shared memory ([row set][token / 4][row][token % 4], 16 bytes per thread and step), then adds up and
@@ -474,7 +521,7 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
 #pragma unroll
                     for (int q = 0; q < kBatch; ++q)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) old[q][e] = load_old(tb * NT + (rank * kGroups + q0 + q) * 4 + e, row);
+                        for (int e = 0; e < 4; ++e) old[q][e] = load_old(tok0 + (rank * kGroups + q0 + q) * 4 + e, row);
                     // the per-token terms too: a shared-memory load between two global stores would wait for the store
                     int tqv[kBatch][4];
                     float tsv[kBatch][4];
@@ -493,10 +540,10 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
                             s.x += part[q][pr].x; s.y += part[q][pr].y; s.z += part[q][pr].z; s.w += part[q][pr].w;
                         }
                         const int i = (rank * kGroups + q0 + q) * 4;
-                        store_v(tqv[q][0], tsv[q][0], tb, i, n_tok, row, sw, s.x, old[q][0]);
-                        store_v(tqv[q][1], tsv[q][1], tb, i + 1, n_tok, row, sw, s.y, old[q][1]);
-                        store_v(tqv[q][2], tsv[q][2], tb, i + 2, n_tok, row, sw, s.z, old[q][2]);
-                        store_v(tqv[q][3], tsv[q][3], tb, i + 3, n_tok, row, sw, s.w, old[q][3]);
+                        store_v(tqv[q][0], tsv[q][0], tok0, i, n_tok, row, sw, s.x, old[q][0]);
+                        store_v(tqv[q][1], tsv[q][1], tok0, i + 1, n_tok, row, sw, s.y, old[q][1]);
+                        store_v(tqv[q][2], tsv[q][2], tok0, i + 2, n_tok, row, sw, s.z, old[q][2]);
+                        store_v(tqv[q][3], tsv[q][3], tok0, i + 3, n_tok, row, sw, s.w, old[q][3]);
                     }
                 }
                 __syncwarp();
@@ -519,7 +566,14 @@ __global__ void __launch_bounds__(tc_threads(RS), 1) gemm_tc_kernel(TcArgs a) {
     if (!ok) atomicExch(a.err, kErrTcTimeout);
     ptx::tc_fence_before();
     __syncthreads();
-    if (warp == 1) ptx::tmem_dealloc(tmem_base, kTmemCols);
+    if constexpr (PAIR) {
+        // nobody leaves while the peer may still arrive on its barriers or its MMAs touch this CTA's memory
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        if (warp == 1) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+    } else if (warp == 1) {
+        ptx::tmem_dealloc(tmem_base, kTmemCols);
+    }
     if (S > 1) {
         // Nobody leaves while a peer may still read its shared memory or arrive on its barriers: the last of both is
         // the peers' arrival on red_free for this CTA's last tile (they read the parked sums before it, and arrived on
@@ -538,20 +592,21 @@ struct TcVariant {
     cudaError_t status = cudaErrorNotReady;
 };
 
-template <int NT, int RS, int S>
+template <int NT, int RS, int S, bool PAIR = false>
 const TcVariant& tc_variant(int sm_count) {
     static TcVariant v;              // cluster limit: once per process (every device of a process is the same GPU model)
     static PerDeviceOnce attributes;  // the kernel's shared-memory limit: once per device
-    v.smem = (size_t)tc_stages(NT, RS, S) * (RS * kSetBytes + 4 * NT * 64) + (S > 1 ? RS * kRows * NT * 4 : 0) + 512 + 16 * NT;
-    auto* kernel = gemm_tc_kernel<NT, RS, S>;
+    constexpr int kCtas = PAIR ? 2 : S, kThreads = tc_threads(PAIR ? 2 : RS);
+    v.smem = (size_t)tc_stages(NT, RS, S) * (RS * kSetBytes + 4 * NT * 64) + (S > 1 ? RS * kRows * NT * 4 : 0) + 512 + (PAIR ? 32 : 16) * NT;
+    auto* kernel = gemm_tc_kernel<NT, RS, S, PAIR>;
     const size_t smem = v.smem;
     v.status = attributes.run([kernel, smem] {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess && NT == 128 && RS == 2 && S == 1) {
+        if (e == cudaSuccess && tc_reg_split(NT, RS, S, PAIR)) {
             // the register shares the warpgroups ask for must fit what the launch gives the CTA, or the asking waits for ever
             cudaFuncAttributes fa;
             e = cudaFuncGetAttributes(&fa, kernel);
-            const int have = fa.numRegs * tc_threads(RS);
+            const int have = fa.numRegs * kThreads;
             const int want = 128 * kRegsLead + 256 * kRegsUnpack + 256 * kRegsEpilogue;
             if (e == cudaSuccess && have < want) e = cudaErrorLaunchOutOfResources;
         }
@@ -561,14 +616,14 @@ const TcVariant& tc_variant(int sm_count) {
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
     if (v.max_clusters != 0) return v;
-    if (S == 1) { v.max_clusters = sm_count; return v; }
+    if (kCtas == 1) { v.max_clusters = sm_count; return v; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sm_count / S * S));
-    cfg.blockDim = dim3(tc_threads(RS));
+    cfg.gridDim = dim3((unsigned)(sm_count / kCtas * kCtas));
+    cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = v.smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = (unsigned)kCtas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
@@ -580,25 +635,26 @@ const TcVariant& tc_variant(int sm_count) {
     return v;
 }
 
-template <int NT, int RS, int S>
+template <int NT, int RS, int S, bool PAIR = false>
 cudaError_t launch_variant(TcArgs a, int sm_count, cudaStream_t stream) {
-    const TcVariant& v = tc_variant<NT, RS, S>(sm_count);
+    const TcVariant& v = tc_variant<NT, RS, S, PAIR>(sm_count);
     if (v.status != cudaSuccess) return v.status;
-    const int n_tiles = (int)((a.row_tiles + 8 * RS - 1) / (8 * RS)) * ((a.m + NT - 1) / NT);
+    constexpr int kCtas = PAIR ? 2 : S, kSets = PAIR ? 2 : RS, kTokens = PAIR ? kPairTokens : NT;
+    const int n_tiles = (int)((a.row_tiles + 8 * kSets - 1) / (8 * kSets)) * ((a.m + kTokens - 1) / kTokens);
     const int n_clusters = v.max_clusters < n_tiles ? v.max_clusters : n_tiles;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_clusters * S));
-    cfg.blockDim = dim3(tc_threads(RS));
+    cfg.gridDim = dim3((unsigned)(n_clusters * kCtas));
+    cfg.blockDim = dim3(tc_threads(kSets));
     cfg.dynamicSmemBytes = v.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)S; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.x = (unsigned)kCtas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = S > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NT, RS, S>, a);
+    cfg.numAttrs = kCtas > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NT, RS, S, PAIR>, a);
 }
 
 // Chunk steps on the busiest CTA when a tile's k range is cut over `s` CTAs (one step charged for the exchange of
@@ -616,7 +672,16 @@ cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) 
     const int n_tiles = (int)((a.row_tiles + 7) / 8) * tok_blocks;          // tiles of 128 rows
     const int n_tiles2 = (int)((a.row_tiles + 15) / 16) * tok_blocks;       // tiles of 256 rows
     if (nt == 128) {
+        // Pairs where there are tiles for most SMs and no more rounds of them than of single CTAs' tiles, which are half as large
+        // (257 x 4096 -> 28672 has one more: 59.7 -> 68.7 us).  More than 16384 rows of plain output stay with single CTAs: their
+        // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240).
+        const TcVariant& pair = tc_variant<128, 1, 1, true>(sm_count);
+        const int n_pairs = (int)((a.row_tiles + 15) / 16) * ((a.m + kPairTokens - 1) / kPairTokens);
         // 256-row tiles halve the activation traffic per weight; 128-row tiles when there is too little work for them
+        const int waves2 = (n_tiles2 + sm_count - 1) / sm_count;
+        if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && a.row_tiles <= 1024 &&
+            (n_pairs + pair.max_clusters - 1) / pair.max_clusters <= waves2)
+            return launch_variant<128, 1, 1, true>(a, sm_count, stream);
         return 2 * n_tiles2 >= sm_count ? launch_variant<128, 2, 1>(a, sm_count, stream) : launch_variant<128, 1, 1>(a, sm_count, stream);
     }
     // 64 tokens at most.  More 128-row tiles than SMs: 256-row tiles.  Fewer than half: cut k over a cluster so that
