@@ -295,11 +295,13 @@ struct SsmArgs {
     const int32_t* pos = nullptr;
     int batch = 1, q_rows = 1;
     float* conv_out = nullptr;     // prefill: x | B | C of the rows after convolution and silu
+    float* seg_s = nullptr;        // prefill, bf16: the states of a prompt's segments (ssm_segment_floats); null: no segments
     float* y = nullptr;            // [rows, inner] (S^T C + D x) * silu(z)
     int sm_count = 0;
 };
 int ssm_state_pad(int state);     // 0: not supported
 cudaError_t launch_ssm_step(const SsmArgs& a, cudaStream_t s, bool pdl);     // q_rows == 1
+int64_t ssm_segment_floats(int state_pad, int sm_count);  // whatever the batch: there are no more segments than CTA slots
 int64_t ssm_conv_floats(const SsmArgs& a);  // floats per row that conv_out needs
 // bf16: 64 tokens at a time on the tensor cores, convolution outputs in bf16; else token by token in f32
 cudaError_t launch_ssm_prefill(const SsmArgs& a, bool bf16, cudaStream_t s);

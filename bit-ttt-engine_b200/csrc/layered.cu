@@ -146,6 +146,7 @@ struct Layered {
     __nv_bfloat16* kv16 = nullptr;  // prefill: keys and values expanded from latents
     size_t kv16_elems = 0;
     float* wkv_seg = nullptr;       // prefill: states of the segments of a wkv recurrence
+    float* ssm_seg = nullptr;       // the same of a state-space recurrence
     bool loops() const { return c.loop_times > 0; }
 };
 
@@ -328,6 +329,7 @@ SsmArgs ssm_args(const bt_model* m, const LayLayer& l, const LayRun& run, const 
     a.pos = m->pos;
     a.batch = batch; a.q_rows = n;
     a.conv_out = r.conv;
+    a.seg_s = m->lay->ssm_seg;
     a.y = r.mix;
     a.sm_count = m->sm_count;
     return a;
@@ -995,6 +997,10 @@ bt_status layered_finalize(bt_model* m) {
         for (const LayLayer& l : L->layers)
             if (l.c.mixer == BT_MIX_WKV) most = std::max(most, wkv_segment_floats(l.c.heads, l.c.dim));
         if (most) BT_CUDA_TRY(dev_alloc(&L->wkv_seg, (size_t)(most * B)));
+        most = 0;
+        for (const LayLayer& l : L->layers)
+            if (l.c.mixer == BT_MIX_SSM) most = std::max(most, ssm_segment_floats(l.state_pad(), m->sm_count));
+        if (most) BT_CUDA_TRY(dev_alloc(&L->ssm_seg, (size_t)most));
     }
     m->rms_eps = L->c.norm_eps;
     m->logit_cap = L->c.logit_softcap;
@@ -1039,7 +1045,7 @@ void layered_destroy(bt_model* m) {
     for (RotTable& t : L->tables) { cudaFree(t.cos_t); cudaFree(t.sin_t); }
     L->dec.release();
     L->pf.release();
-    cudaFree(L->pos_table); cudaFree(L->h2); cudaFree(L->loop_in.tiles); cudaFree(L->loop_step); cudaFree(L->kv16); cudaFree(L->wkv_seg);
+    cudaFree(L->pos_table); cudaFree(L->h2); cudaFree(L->loop_in.tiles); cudaFree(L->loop_step); cudaFree(L->kv16); cudaFree(L->wkv_seg); cudaFree(L->ssm_seg);
     delete L;
     m->lay = nullptr;
 }

@@ -2,6 +2,8 @@
 //   S <- exp(-exp(A_log) dt) S + dt B x^T,   y = S^T C + D x,
 // x, B and C after a causal convolution per channel and silu, dt = softplus(dt + dt_bias).  The result leaves gated:
 // y * silu(z).  State, decays, step sizes and every sum of the recurrence are f32.
+#include <algorithm>
+
 #include "bt_dense.cuh"
 #include "bt_ptx.cuh"
 
@@ -249,35 +251,51 @@ cudaError_t scan_launch_n(const SsmArgs& a, cudaStream_t s, bool pdl) {
 // B, C and x are bf16 (convolution outputs); every f32 factor enters its product as bf16 hi + lo (16 significand bits):
 // the state, the weights of the pairs (t, s) and the scaled x.  The state itself, the sums and all decays stay f32.
 // A CTA owns 64 columns of one head and walks the chunks in order; the next chunk is copied while one is computed.
+// A chunk is a chain of latencies (copies, three barriers, short runs of MMAs), so two CTAs share an SM, and where one per head
+// leaves CTA slots idle the prompt is cut into segments that are walked side by side (ssm_segments): ChunkMode::kStates makes
+// what each segment but the last adds to the state, its own decays included, and ChunkMode::kOutputs starts a segment from
+// the joined states of those before it and does what ChunkMode::kAll does.  1999 tokens, 64 heads of 64 x 128: 64 CTAs with a
+// prompt each 206 us; four segments 34 (states) + 103 us.
 // Sixteen warps as 4 x 4 over (16 tokens) x (16 earlier tokens | 16 columns): each makes its tile of pair weights, leaves it
 // in shared memory and then its tile of outputs; the state is cut over the warps by rows of 16 elements and columns.
-constexpr int kChunk = 64, kChunkThreads = 512;
+constexpr int kChunk = 64, kChunkThreads = 512, kMaxSegments = 8;
+enum class ChunkMode { kAll, kStates, kOutputs };
 template <int NP>
 struct ChunkCfg {
     static constexpr int WN = NP / 16 < 8 ? NP / 16 : 8, WP = 16 / WN < 4 ? 16 / WN : 4;  // warps over state rows / columns
     static constexpr int TN = NP / 16 / WN, TP = 8 / WP;                                  // 16-row tiles, 8-column tiles per warp
     static constexpr int NS = NP * 2 + 16, PS = 64 * 2 + 16;                              // bytes per shared-memory row
-    static constexpr int kIn = kChunk * (2 * NS + PS);                                    // B, C, x of a chunk
-    static constexpr int kStages = NP <= 128 ? 2 : 1;
-    static constexpr size_t kSmem = (size_t)kStages * kIn + 2 * NP * PS + 4 * kChunk * PS + 3 * kChunk * 4;
+    static constexpr int kC = kChunk * NS, kBx = kChunk * (NS + PS);                      // C of a chunk; B and x
+    static constexpr int kOver = 2 * NP * PS > 4 * kChunk * PS ? 2 * NP * PS : 4 * kChunk * PS;  // state, then scaled x and pair weights
+    static constexpr size_t kSmem = (size_t)kC + 2 * kBx + kOver + 3 * kChunk * 4;
+    static constexpr int kSlot = NP * 64;                                                 // floats of a CTA's state
+    static constexpr int kLive = 32 * WN * WP;                                            // threads that hold it
 };
 
-template <int NP>
-__global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmArgs a, int channels) {
+// segs: segments (1: kAll), seg_chunks: chunks of each
+template <int NP, ChunkMode MODE>
+__global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_kernel(const SsmArgs a, int channels, int segs, int seg_chunks) {
     using Cfg = ChunkCfg<NP>;
     constexpr int NS = Cfg::NS, PS = Cfg::PS, TN = Cfg::TN, TP = Cfg::TP;
-    extern __shared__ __align__(16) uint8_t csm[];
-    uint8_t* s_hi = csm + Cfg::kStages * Cfg::kIn;   // state [NP][64] hi, lo
+    constexpr bool kOut = MODE != ChunkMode::kStates;
+    extern __shared__ __align__(16) uint8_t csm[];   // C | B, x of a chunk and of the next | state, scaled x, pair weights
+    uint8_t* s_hi = csm + Cfg::kC + 2 * Cfg::kBx;    // state [NP][64] hi, lo
     uint8_t* s_lo = s_hi + NP * PS;
-    uint8_t* w_hi = s_lo + NP * PS;                  // scaled x [64][64] hi, lo
+    uint8_t* w_hi = s_hi;                            // over the state, once C S is done: scaled x [64][64] hi, lo
     uint8_t* w_lo = w_hi + kChunk * PS;
     uint8_t* m_hi = w_lo + kChunk * PS;              // pair weights [64][64] hi, lo
     uint8_t* m_lo = m_hi + kChunk * PS;
-    float* dt_s = reinterpret_cast<float*>(m_lo + kChunk * PS);
+    float* dt_s = reinterpret_cast<float*>(s_hi + Cfg::kOver);
     float* cum_s = dt_s + kChunk;
     float* wt_s = cum_s + kChunk;                    // exp(c_last - c_t) dt_t
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.x, v0 = blockIdx.y * 64, b = blockIdx.z;
+    const int head = blockIdx.x, b = blockIdx.z, vblocks = (a.vdim + 63) / 64;
+    const int seg = MODE == ChunkMode::kAll ? 0 : (int)blockIdx.y / vblocks, vb = (int)blockIdx.y - seg * vblocks, v0 = vb * 64;
+    const int t_first = seg * seg_chunks * kChunk, t_end = MODE == ChunkMode::kAll ? a.q_rows : min(a.q_rows, t_first + seg_chunks * kChunk);
+    // this CTA's columns in the segments' states: [segment][thread order of the fragments]
+    const int64_t slot0 = (((int64_t)b * a.heads + head) * vblocks + vb) * segs;
+    float* seg_state = a.seg_s + slot0 * Cfg::kSlot;
+    float* seg_log = a.seg_s + (int64_t)a.batch * a.heads * vblocks * segs * Cfg::kSlot + slot0;  // logarithm of a segment's whole decay
     const int vc = min(64, a.vdim - v0), inner = a.heads * a.vdim, g = head / (a.heads / a.groups);
     const int vp = pad8(a.vdim), np = pad8(a.state), cols = conv_cols(a);
     const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(a.conv_out) + (int64_t)b * a.q_rows * cols;
@@ -292,46 +310,77 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
     const int tt = warp >> 2, qq = warp & 3;         // tokens 16 tt ..; earlier tokens / columns 16 qq ..
 
     float st[TN][TP][4];  // (n = g / g + 8 of the tile, p = 2 t, 2 t + 1)
+    auto each_state = [&](auto f) {
 #pragma unroll
-    for (int i = 0; i < TN; ++i)
+        for (int i = 0; i < TN; ++i)
 #pragma unroll
-        for (int k = 0; k < TP; ++k)
+            for (int k = 0; k < TP; ++k) f(st[i][k], (i * TP + k) * Cfg::kLive + (int)threadIdx.x, i, k);
+    };
+    auto slot = [&](int sg, int at) { return reinterpret_cast<float4*>(seg_state + (int64_t)sg * Cfg::kSlot) + at; };
+    if constexpr (MODE == ChunkMode::kOutputs) {
+        // the sequence's state as it was lies in the last segment's place; the first segment's result contains it
+        const int from = seg == 0 ? segs - 1 : 0;
+        each_state([&](float (&v)[4], int at, int, int) {
+            const float4 f = s_live ? *slot(from, at) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        });
+        for (int sg = 1; sg < seg; ++sg) {
+            const float dec = expf(seg_log[sg]);
+            each_state([&](float (&v)[4], int at, int, int) {
+                const float4 f = s_live ? *slot(sg, at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[0] = fmaf(dec, v[0], f.x); v[1] = fmaf(dec, v[1], f.y); v[2] = fmaf(dec, v[2], f.z); v[3] = fmaf(dec, v[3], f.w);
+            });
+        }
+    } else {
+        each_state([&](float (&v)[4], int at, int i, int k) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int n = (wn * TN + i) * 16 + (lane >> 2) + (e >> 1) * 8, p = (wp * TP + k) * 8 + (lane & 3) * 2 + (e & 1);
-                st[i][k][e] = s_live && p < vc && p0 > 0 ? state[(int64_t)p * a.state_pad + n] : 0.0f;
+                v[e] = s_live && p < vc && p0 > 0 && seg == 0 ? state[(int64_t)p * a.state_pad + n] : 0.0f;
             }
+            if (MODE == ChunkMode::kStates && seg == 0 && s_live) *slot(segs - 1, at) = make_float4(v[0], v[1], v[2], v[3]);
+        });
+    }
+    float seg_sum = 0.0f;  // kStates: the decays' logarithms so far
 
-    auto load = [&](int t0, int buf) {
-        const uint32_t dst = ptx::smem_u32(csm) + buf * Cfg::kIn;
+    auto load_bx = [&](int t0, int buf) {
+        const uint32_t dst = ptx::smem_u32(csm) + Cfg::kC + buf * Cfg::kBx;
         constexpr int NQ = NP / 8;
-        for (int e = threadIdx.x; e < kChunk * (2 * NQ + 8); e += kChunkThreads) {
-            const int t = e / (2 * NQ + 8), q = e - t * (2 * NQ + 8);
+        for (int e = threadIdx.x; e < kChunk * (NQ + 8); e += kChunkThreads) {
+            const int t = e / (NQ + 8), q = e - t * (NQ + 8);
             const __nv_bfloat16* row = in + (int64_t)(t0 + t) * cols;
-            const bool tok = t0 + t < a.q_rows;
+            const bool tok = t0 + t < t_end;
             if (q < NQ) {
                 const bool live = tok && q * 8 < np;
                 ptx::cp16(dst + t * NS + q * 16, live ? row + bcol + q * 8 : in, live);
-            } else if (q < 2 * NQ) {
-                const bool live = tok && (q - NQ) * 8 < np;
-                ptx::cp16(dst + kChunk * NS + t * NS + (q - NQ) * 16, live ? row + ccol + (q - NQ) * 8 : in, live);
             } else {
-                const bool live = tok && (q - 2 * NQ) * 8 < xlive;
-                ptx::cp16(dst + 2 * kChunk * NS + t * PS + (q - 2 * NQ) * 16, live ? row + xcol + (q - 2 * NQ) * 8 : in, live);
+                const bool live = tok && (q - NQ) * 8 < xlive;
+                ptx::cp16(dst + kChunk * NS + t * PS + (q - NQ) * 16, live ? row + xcol + (q - NQ) * 8 : in, live);
             }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto load_c = [&](int t0) {
+        const uint32_t dst = ptx::smem_u32(csm);
+        constexpr int NQ = NP / 8;
+        for (int e = threadIdx.x; e < kChunk * NQ; e += kChunkThreads) {
+            const int t = e / NQ, q = e - t * NQ;
+            const bool live = t0 + t < t_end && q * 8 < np;
+            ptx::cp16(dst + t * NS + q * 16, live ? in + (int64_t)(t0 + t) * cols + ccol + q * 8 : in, live);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto raw_dt = [&](int t0) {  // threads 0-63: this chunk's step-size projections
         const int t = t0 + (int)threadIdx.x;
-        return threadIdx.x < kChunk && t < a.q_rows ? a.proj[((int64_t)b * a.q_rows + t) * a.ld + inner + channels + head] : 0.0f;
+        return threadIdx.x < kChunk && t < t_end ? a.proj[((int64_t)b * a.q_rows + t) * a.ld + inner + channels + head] : 0.0f;
     };
-    load(0, 0);
-    float dt_raw = raw_dt(0);
+    if (kOut) load_c(t_first);
+    load_bx(t_first, 0);
+    float dt_raw = raw_dt(t_first);
 
     int buf = 0;
-    for (int t0 = 0; t0 < a.q_rows; t0 += kChunk) {
-        const int n = min(kChunk, a.q_rows - t0);
+    for (int t0 = t_first; t0 < t_end; t0 += kChunk, buf ^= 1) {
+        const int n = min(kChunk, t_end - t0);
         const int ta = tt * 16 + (lane >> 2), tb = ta + 8;  // this lane's tokens
         // ---- step sizes and running decay; the state as hi | lo for the products; the gates are requested ----
         if (threadIdx.x < kChunk) dt_s[threadIdx.x] = (int)threadIdx.x < n ? softplus_f(dt_raw + bias) : 0.0f;
@@ -342,9 +391,9 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int t = (e >> 1) ? tb : ta, c = qq * 16 + i * 8 + (lane & 3) * 2 + (e & 1);
-                z[i][e] = t < n && c < vc ? a.proj[((int64_t)b * a.q_rows + t0 + t) * a.ld + head * a.vdim + v0 + c] : 0.0f;
+                z[i][e] = kOut && t < n && c < vc ? a.proj[((int64_t)b * a.q_rows + t0 + t) * a.ld + head * a.vdim + v0 + c] : 0.0f;
             }
-        if (s_live)
+        if (kOut && s_live)
 #pragma unroll
             for (int i = 0; i < TN; ++i)
 #pragma unroll
@@ -358,10 +407,10 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
                     }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (Cfg::kStages == 2 && t0 + kChunk < a.q_rows) load(t0 + kChunk, buf ^ 1);
-        uint8_t* bt = csm + buf * Cfg::kIn;
-        uint8_t* xt = bt + 2 * kChunk * NS;
-        const uint32_t b_sm = ptx::smem_u32(bt), c_sm = b_sm + kChunk * NS, x_sm = b_sm + 2 * kChunk * NS;
+        if (t0 + kChunk < t_end) load_bx(t0 + kChunk, buf ^ 1);
+        uint8_t* bt = csm + Cfg::kC + buf * Cfg::kBx;
+        uint8_t* xt = bt + kChunk * NS;
+        const uint32_t c_sm = ptx::smem_u32(csm), b_sm = ptx::smem_u32(bt), x_sm = b_sm + kChunk * NS;
         // ---- running sums of the decays' logarithms, while the other warps multiply ----
         if (warp == 0) {
             const float c0 = a_neg * dt_s[2 * lane], c1 = a_neg * dt_s[2 * lane + 1];
@@ -380,7 +429,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
         }
         // ---- C S (16 tokens x 16 columns) and C B^T (16 x 16 pairs) ----
         float y[2][4] = {}, gm[2][4] = {};
-        const bool live = tt * 16 < n, pairs = live && qq <= tt;
+        const bool live = kOut && tt * 16 < n, pairs = live && qq <= tt;
         if (live) {
             const uint32_t c_addr = c_sm + (tt * 16 + (lane & 15)) * NS + (lane >> 4) * 16;
             const uint32_t b_addr = b_sm + (qq * 16 + (lane & 7) + ((lane >> 4) << 3)) * NS + ((lane >> 3) & 1) * 16;
@@ -403,7 +452,8 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
                 }
             }
         }
-        __syncthreads();  // running sums
+        __syncthreads();  // running sums; C and the state's hi | lo have been read
+        if (kOut && t0 + kChunk < t_end) load_c(t0 + kChunk);
         // ---- x scaled for the state update; pair weights ----
         for (int e = threadIdx.x; e < kChunk * 32; e += kChunkThreads) {
             const int t = e >> 5, o = t * PS + (e & 31) * 4;
@@ -462,6 +512,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
         // ---- state ----
         if (s_live) {
             const float dec = expf(cum_s[kChunk - 1]);
+            seg_sum += cum_s[kChunk - 1];
 #pragma unroll
             for (int i = 0; i < TN; ++i)
 #pragma unroll
@@ -490,28 +541,50 @@ __global__ void __launch_bounds__(kChunkThreads, 1) ssm_chunk_kernel(const SsmAr
                 }
         }
         __syncthreads();
-        if (Cfg::kStages == 1) { if (t0 + kChunk < a.q_rows) load(t0 + kChunk, 0); } else buf ^= 1;
     }
-#pragma unroll
-    for (int i = 0; i < TN; ++i)
-#pragma unroll
-        for (int k = 0; k < TP; ++k)
+    if constexpr (MODE == ChunkMode::kStates) {
+        each_state([&](float (&v)[4], int at, int, int) { if (s_live) *slot(seg, at) = make_float4(v[0], v[1], v[2], v[3]); });
+        if (threadIdx.x == 0) seg_log[seg] = seg_sum;
+    } else if (MODE == ChunkMode::kAll || seg == segs - 1) {
+        each_state([&](float (&v)[4], int, int i, int k) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int n = (wn * TN + i) * 16 + (lane >> 2) + (e >> 1) * 8, p = (wp * TP + k) * 8 + (lane & 3) * 2 + (e & 1);
-                if (s_live && p < vc) state[(int64_t)p * a.state_pad + n] = st[i][k][e];
+                if (s_live && p < vc) state[(int64_t)p * a.state_pad + n] = v[e];
             }
-    keep_inputs(a, ring, channels, b, head, v0, vc, p0);
+        });
+        keep_inputs(a, ring, channels, b, head, v0, vc, p0);
+    }
 }
 
+// Segments of a prompt: as many as there are CTA slots for every head (two CTAs an SM up to 128 state elements), of two chunks
+// at least.  Making the states apart costs a third of a segment's time (34 against 103 us above), so that two segments already
+// take 0.7 of the whole prompt's time; where a CTA per head fills the slots there is nothing to gain.
+int ssm_segments(const SsmArgs& a) {
+    const int64_t ctas = (int64_t)a.heads * ((a.vdim + 63) / 64) * a.batch, slots = (int64_t)a.sm_count * (a.state_pad <= 128 ? 2 : 1);
+    const int chunks = (a.q_rows + kChunk - 1) / kChunk;
+    const int64_t segs = std::min<int64_t>(std::min<int64_t>(slots / ctas, chunks / 2), kMaxSegments);
+    return a.seg_s && segs > 1 ? (int)segs : 1;
+}
+
+template <int NP, ChunkMode MODE>
+cudaError_t chunk_launch_mode(const SsmArgs& a, int segs, int seg_chunks, int grid_segs, cudaStream_t s) {
+    static PerDeviceOnce once;
+    cudaError_t e = once.run([] { return cudaFuncSetAttribute(ssm_chunk_kernel<NP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChunkCfg<NP>::kSmem); });
+    if (e != cudaSuccess) return e;
+    ssm_chunk_kernel<NP, MODE><<<dim3((unsigned)a.heads, (unsigned)((a.vdim + 63) / 64 * grid_segs), (unsigned)a.batch), kChunkThreads, ChunkCfg<NP>::kSmem, s>>>(
+        a, a.heads * a.vdim + 2 * a.groups * a.state, segs, seg_chunks);
+    return cudaGetLastError();
+}
 template <int NP>
 cudaError_t chunk_launch(const SsmArgs& a, cudaStream_t s) {
-    static PerDeviceOnce once;
-    cudaError_t e = once.run([] { return cudaFuncSetAttribute(ssm_chunk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChunkCfg<NP>::kSmem); });
-    if (e != cudaSuccess) return e;
-    ssm_chunk_kernel<NP><<<dim3((unsigned)a.heads, (unsigned)((a.vdim + 63) / 64), (unsigned)a.batch), kChunkThreads, ChunkCfg<NP>::kSmem, s>>>(
-        a, a.heads * a.vdim + 2 * a.groups * a.state);
-    return cudaGetLastError();
+    const int chunks = (a.q_rows + kChunk - 1) / kChunk;
+    int segs = ssm_segments(a);
+    const int seg_chunks = (chunks + segs - 1) / segs;
+    segs = (chunks + seg_chunks - 1) / seg_chunks;
+    if (segs == 1) return chunk_launch_mode<NP, ChunkMode::kAll>(a, 1, chunks, 1, s);
+    cudaError_t e = chunk_launch_mode<NP, ChunkMode::kStates>(a, segs, seg_chunks, segs - 1, s);
+    return e == cudaSuccess ? chunk_launch_mode<NP, ChunkMode::kOutputs>(a, segs, seg_chunks, segs, s) : e;
 }
 
 }  // namespace
@@ -527,6 +600,8 @@ cudaError_t launch_ssm_step(const SsmArgs& a, cudaStream_t s, bool pdl) {
     if (a.q_rows != 1) return cudaErrorInvalidValue;
     return scan_launch_n<true>(a, s, pdl);
 }
+
+int64_t ssm_segment_floats(int state_pad, int sm_count) { return (int64_t)sm_count * 2 * (state_pad * 64 + 1); }
 
 int64_t ssm_conv_floats(const SsmArgs& a) {  // per row, for either form
     const int64_t plain = a.heads * (int64_t)a.vdim + 2ll * a.groups * a.state, padded = (conv_cols(a) + 1) / 2;

@@ -162,6 +162,20 @@ def test_recurrence_alone_far_token(bt):
             assert (e.max() <= TOL["float32"][0] if dtype == "float32" else np.sqrt((e * e).mean()) <= 0.02), (sizes, e.max())
 
 
+@pytest.mark.parametrize("state", [12, 40, 128, 200])  # one and two CTAs an SM, columns beyond the state
+@pytest.mark.parametrize("n", [192, 256, 257, 449, 1030])  # one segment, two of two chunks, a last one of a token, of three and of many
+def test_recurrence_in_segments(bt, state, n):
+    cfg = lay.LayersConfig(40, 48, 1100, 1e-5, True, [ssm(3, 72, state, taps=3, norm_groups=3)])
+    t = make_tensors(cfg, seed=state)
+    t["l0.mix.A_log"] = bf16(np.array([-5.0, -2.0, 0.5], np.float32))
+    tokens = np.random.default_rng(n).integers(0, 40, n + 20).astype(np.int32)
+    logits, _ = oracle(cfg, t, tokens)
+    m = lay.build_layered(cfg, t, dtype="bfloat16")
+    assert_close(feed(m, tokens, [n, 20]), logits, "bfloat16")
+    m.reset_kv_cache()
+    assert_close(feed(m, tokens, [15, n]), logits, "bfloat16")  # a state to start from
+
+
 def needle_model(n_positions, dtype_seed=0):
     """One attention layer whose query of token 1 points at the key of token 0 (score far above all others)."""
     cfg = lay.LayersConfig(60, 96, n_positions, 1e-5, True, [attn(4, 2, 32, 24, scale=0.6, cap=18.0, coef=0.3, every=50)])
