@@ -137,11 +137,9 @@ struct DenseOut {
     const ExpertPlan* plan = nullptr;  // blocks are experts; rows by the plan
 };
 // tcgen05 product of tiled bf16 activations; f32 accumulation.  With few row tiles the inputs of a plain product are cut
-// over several CTAs, whose partial sums go through `scratch` (dense_tc_scratch floats) and are added in a fixed order.
+// over the CTAs of a cluster, whose partial sums are added in a fixed order through distributed shared memory.
 // Block-diagonal products: block b reads the columns b * halves * kpad(k) .. of the input.
-size_t dense_tc_scratch(const DenseLin& lin, int64_t m, int sm_count);
-int dense_tc_kernels(const DenseLin& lin, int64_t m, int sm_count, int act = DACT_NONE);
-cudaError_t launch_dense_tc(const DenseLin& lin, const uint8_t* x_tiles, int64_t m, const DenseOut& o, float* scratch,
+cudaError_t launch_dense_tc(const DenseLin& lin, const uint8_t* x_tiles, int64_t m, const DenseOut& o,
                             unsigned int* err, int sm_count, cudaStream_t s);
 
 // f32 product of f32 rows (no tensor cores), for 32-bit models; block b reads the columns b * x_block ..

@@ -1,6 +1,8 @@
 // Dense bf16 projections: streaming product for up to 8 rows (f32 activations), tcgen05 product for more (bf16
 // activations), f32 product for 32-bit models; each also block-diagonal, the last two also over rows grouped by expert.  And
 // the row kernels around them (embedding with learned positions, output norm + residual + next norm, norm in equal parts).
+#include <mutex>
+
 #include "bt_dense.cuh"
 #include "bt_ptx.cuh"
 
@@ -349,7 +351,7 @@ struct TcArgs {
     int splits, blocks;
     int64_t w_block, x_block;        // bytes from one block to the next
     float* out;
-    int64_t ld, part_stride, out_block;
+    int64_t ld, out_block;
     const float* bias;
     uint8_t* out_tiles;
     __nv_bfloat16* out_rows16;
@@ -359,6 +361,8 @@ struct TcArgs {
     unsigned int* err;
 };
 
+// TC_SPLIT: the splits of a tile are the CTAs of a cluster (their rank the split); a CTA has one tile, and its partial sums lie
+// over the ring, [token][row], until every CTA has added up its share of the tokens.
 template <int NT>
 struct TcCfg {
     static constexpr int kStageBytes = (kTcRows + NT) * 128;
@@ -369,7 +373,7 @@ struct TcCfg {
 
 // What the epilogue does is a constant of the kernel: f32 rows as they are, f32 rows with bias and activation, tiled bf16
 // (squared relu), gate and up pairs to tiled bf16, bf16 rows.
-enum TcEpi : int { TC_ROWS, TC_ROWS_ACT, TC_TILES, TC_PAIRS, TC_ROWS16 };
+enum TcEpi : int { TC_ROWS, TC_ROWS_ACT, TC_TILES, TC_PAIRS, TC_ROWS16, TC_SPLIT };
 
 template <int NT, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a) {
@@ -402,6 +406,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
     struct Tile { int blk, rs, c0, c1, sp; int64_t tok0, tok_end; };
     auto decode = [&](int t) {
         Tile d;
+        if (EPI == TC_SPLIT) {  // t = row set * splits + split, one token block
+            d.blk = 0; d.rs = t / a.splits; d.sp = t - d.rs * a.splits; d.tok0 = 0; d.tok_end = a.m;
+            d.c0 = (int)((int64_t)a.chunks * d.sp / a.splits);
+            d.c1 = (int)((int64_t)a.chunks * (d.sp + 1) / a.splits);
+            return d;
+        }
         const int per = row_sets * tok_blocks, q = t / per, u = t - q * per, tb = u / row_sets;
         d.rs = u - tb * row_sets;
         if (a.plan) {
@@ -409,10 +419,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
             d.blk = e.expert; d.tok0 = e.row0; d.tok_end = e.row_end; d.sp = 0; d.c0 = 0; d.c1 = a.chunks;
             return d;
         }
-        d.blk = a.splits > 1 ? 0 : q;
-        d.sp = a.splits > 1 ? q : 0;
-        d.c0 = (int)((int64_t)a.chunks * d.sp / a.splits);
-        d.c1 = (int)((int64_t)a.chunks * (d.sp + 1) / a.splits);
+        d.blk = q;
+        d.sp = 0;
+        d.c0 = 0;
+        d.c1 = a.chunks;
         d.tok0 = (int64_t)tb * NT;
         d.tok_end = a.m;
         return d;
@@ -488,7 +498,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
                 uint32_t v[32];
                 ptx::tmem_ld32(tmem_base + ((uint32_t)(sub * 32) << 16) + set * NT + q, v);
                 ptx::tmem_ld_wait();
-                if (EPI == TC_PAIRS) {
+                if (EPI == TC_SPLIT) {
+                    // every MMA of the CTA's only tile is done: the ring is free
+                    float* part = reinterpret_cast<float*>(smem) + q * kTcRows + sub * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) part[j * kTcRows] = __uint_as_float(v[j]);
+                } else if (EPI == TC_PAIRS) {
                     // neighbouring lanes hold gate and up: the even one finishes the first 16 tokens, the odd one the others;
                     // pieces of (one token, 8 features) through shared memory, [token group][8 features][token]
 #pragma unroll
@@ -533,7 +548,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
                     }
                     __syncwarp();
                 } else if (f < a.n) {
-                    float* o = a.out + (int64_t)d.sp * a.part_stride + (a.plan ? 0 : d.blk * a.out_block) + (tok0 + q) * a.ld + f;
+                    float* o = a.out + (a.plan ? 0 : d.blk * a.out_block) + (tok0 + q) * a.ld + f;
                     if (tok0 + q + 32 <= tok_end) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) o[j * a.ld] = finish(__uint_as_float(v[j]));
@@ -554,33 +569,43 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 1) ptx::tmem_dealloc(tmem_base, 2 * NT);
-}
-
-// sum of the partial products in the order of the splits, activation, f32 rows or tiled bf16
-__global__ void __launch_bounds__(256) dense_reduce_kernel(const float* __restrict__ parts, int splits, int64_t part_stride,
-                                                           int64_t pld, int64_t m, int n, int n_out, int act, float* __restrict__ out,
-                                                           int64_t ld, uint8_t* __restrict__ tiles, int64_t m_pad, const float* __restrict__ bias) {
-    const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    const int64_t r = blockIdx.y;
-    if (c0 >= n_out) return;
-    float v[8];
+    if constexpr (EPI == TC_SPLIT) {
+        // The partial sums of a tile meet through distributed shared memory: token t is added up by CTA t mod splits, in the
+        // order of the splits, and finished there, four rows to a thread.  A second launch that read them from global memory
+        // took 3.0 to 4.1 us behind every such product.
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        const int rank = (int)ptx::cluster_ctarank(), rs = (int)blockIdx.x / a.splits;
+        constexpr int kPieces = kTcRows / 4;
+        for (int i = threadIdx.x;; i += kTcThreads) {
+            const int64_t tok = rank + (int64_t)a.splits * (i / kPieces);
+            if (tok >= a.m) break;
+            const int r0 = i % kPieces * 4, c0 = rs * kTcRows + r0;
+            const float* at = reinterpret_cast<const float*>(smem) + tok * kTcRows + r0;
+            uint4 p[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-    for (int s = 0; s < splits; ++s) {
-        const float* p = parts + s * part_stride + r * pld + c0;  // pld: multiple of 128, rows 16-byte aligned
-        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-        v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+            for (int sp = 0; sp < 8; ++sp)
+                if (sp < a.splits) p[sp] = ptx::ld_dsmem_v4(ptx::map_to_rank(at, (uint32_t)sp));
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp)
+                if (sp < a.splits) {
+                    v[0] += __uint_as_float(p[sp].x); v[1] += __uint_as_float(p[sp].y);
+                    v[2] += __uint_as_float(p[sp].z); v[3] += __uint_as_float(p[sp].w);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = c0 + j < a.n ? act_fn(a.act, v[j] + (a.bias ? a.bias[c0 + j] : 0.0f)) : 0.0f;
+            if (a.out_tiles) {
+                if (c0 < dense_kpad(a.n)) *reinterpret_cast<uint2*>(a.out_tiles + dense_off(tok, c0, a.m_pad)) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (c0 + j < a.n) a.out[tok * a.ld + c0 + j] = v[j];
+            }
+        }
+        ptx::cluster_arrive();  // nobody leaves while a peer reads its sums
+        ptx::cluster_wait();
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = c0 + j < n ? act_fn(act, v[j] + (bias ? bias[c0 + j] : 0.0f)) : 0.0f;
-    if (tiles)
-        *reinterpret_cast<uint4*>(tiles + dense_off(r, c0, m_pad)) =
-            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-    else
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (c0 + j < n) out[r * ld + c0 + j] = v[j];
 }
 
 template <int NT, int EPI>
@@ -591,6 +616,49 @@ cudaError_t tc_launch_e(const TcArgs& a, int sm_count, cudaStream_t s) {
     const int64_t tiles = (int64_t)(a.n_pad / kTcRows) * ((a.m + NT - 1) / NT) * a.splits * a.blocks;  // a.m: the plan's upper bound
     dense_tc_kernel<NT, EPI><<<(unsigned)(tiles < sm_count ? tiles : sm_count), kTcThreads, TcCfg<NT>::kSmem, s>>>(a);
     return cudaGetLastError();
+}
+// How many clusters of `splits` CTAs of the split product the GPU holds at once (a cluster lives inside one GPC); 0: none.
+template <int NT>
+int tc_clusters(int splits, int sm_count) {
+    static std::mutex mu;
+    static int known[9] = {};  // (every device of a process is the same GPU model)
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[splits] == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(sm_count / splits * splits));
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = TcCfg<NT>::kSmem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(dense_tc_kernel<NT, TC_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<NT>::kSmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, dense_tc_kernel<NT, TC_SPLIT>, &cfg) != cudaSuccess || n < 1) {
+            (void)cudaGetLastError();
+            n = -1;
+        }
+        known[splits] = n;
+    }
+    return known[splits] < 0 ? 0 : known[splits];
+}
+template <int NT>
+cudaError_t tc_launch_split(const TcArgs& a, cudaStream_t s) {
+    static PerDeviceOnce once;
+    cudaError_t e = once.run([] { return cudaFuncSetAttribute(dense_tc_kernel<NT, TC_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<NT>::kSmem); });
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.n_pad / kTcRows * a.splits));
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = TcCfg<NT>::kSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)a.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, dense_tc_kernel<NT, TC_SPLIT>, a);
 }
 template <int NT>
 cudaError_t tc_launch(const TcArgs& a, int sm_count, cudaStream_t s) {
@@ -613,7 +681,10 @@ int tc_splits(const DenseLin& lin, int64_t m, int sm_count) {
     const int tiles = lin.n_pad / kTcRows, chunks = lin.k_pad / kDenseK;
     int s = sm_count / tiles;
     if (s > chunks / 4) s = chunks / 4;
-    return s < 1 ? 1 : (s > 8 ? 8 : s);
+    if (s > 8) s = 8;
+    // all clusters at once: with a second wave of them a product takes as long again, while a split less costs an eighth to a half
+    while (s > 1 && (m <= 64 ? tc_clusters<64>(s, sm_count) : tc_clusters<128>(s, sm_count)) < tiles) --s;
+    return s < 1 ? 1 : s;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -975,14 +1046,8 @@ cudaError_t launch_dense_stream_segs(const DenseSeg* segs, int nseg, const Dense
     }
 }
 
-size_t dense_tc_scratch(const DenseLin& lin, int64_t m, int sm_count) {
-    const int sp = tc_splits(lin, m, sm_count);
-    return sp > 1 ? (size_t)sp * (size_t)m * lin.n_pad : 0;
-}
-int dense_tc_kernels(const DenseLin& lin, int64_t m, int sm_count, int act) { return act < DACT_SWIGLU && tc_splits(lin, m, sm_count) > 1 ? 2 : 1; }
-
-cudaError_t launch_dense_tc(const DenseLin& lin, const uint8_t* x_tiles, int64_t m, const DenseOut& o, float* scratch,
-                            unsigned int* err, int sm_count, cudaStream_t s) {
+cudaError_t launch_dense_tc(const DenseLin& lin, const uint8_t* x_tiles, int64_t m, const DenseOut& o, unsigned int* err,
+                            int sm_count, cudaStream_t s) {
     const int blocks = o.shared_weights ? o.blocks : lin.blocks, n_out = dense_outputs(lin, o.act);
     const bool whole = o.act == DACT_SWIGLU || o.out_rows16 || o.plan || blocks > 1;  // never cut
     const int sp = whole ? 1 : tc_splits(lin, m, sm_count);
@@ -997,23 +1062,13 @@ cudaError_t launch_dense_tc(const DenseLin& lin, const uint8_t* x_tiles, int64_t
     a.blocks = o.plan ? 1 : blocks; a.w_block = o.shared_weights ? 0 : (int64_t)lin.block_bytes();
     a.x_block = o.shared_weights ? o.x_block : (int64_t)a.chunks * a.m_pad * 128;
     a.out_block = o.out_block; a.bias = o.bias; a.plan = nullptr; a.n_plan = nullptr; a.out_rows16 = nullptr;
-    if (sp > 1) {
-        a.out = scratch; a.ld = lin.n_pad; a.part_stride = m * (int64_t)lin.n_pad; a.out_tiles = nullptr; a.act = DACT_NONE;
-        a.bias = nullptr;
-        a.n = lin.n_pad;  // the padded rows are zero weights: the reduction may read whole vectors
-    } else {
-        a.out = o.out; a.ld = o.ld; a.part_stride = 0; a.out_tiles = o.out_tiles; a.out_rows16 = o.out_rows16; a.act = o.act;
-    }
+    a.out = o.out; a.ld = o.ld; a.out_tiles = o.out_tiles; a.out_rows16 = o.out_rows16; a.act = o.act;
+    if (sp > 1) return nt == 64 ? tc_launch_split<64>(a, s) : tc_launch_split<128>(a, s);
     if (o.plan) {
         a.plan = o.plan->tiles; a.n_plan = o.plan->n_tiles;
         a.m = (int64_t)o.plan->max_tiles * nt;
     }
-    cudaError_t e = nt == 64 ? tc_launch<64>(a, sm_count, s) : (nt == 128 ? tc_launch<128>(a, sm_count, s) : tc_launch<256>(a, sm_count, s));
-    if (e != cudaSuccess || sp == 1) return e;
-    const int cols = o.out_tiles ? dense_kpad(lin.n) : lin.n;
-    dense_reduce_kernel<<<dim3((unsigned)((cols + 2047) / 2048), (unsigned)m), 256, 0, s>>>(
-        scratch, sp, a.part_stride, a.ld, m, lin.n, cols, o.act, o.out, o.ld, o.out_tiles, a.m_pad, o.bias);
-    return cudaGetLastError();
+    return nt == 64 ? tc_launch<64>(a, sm_count, s) : (nt == 128 ? tc_launch<128>(a, sm_count, s) : tc_launch<256>(a, sm_count, s));
 }
 
 cudaError_t launch_dense_f32(const DenseLin& lin, const float* x, int64_t ldx, int64_t x_block, int64_t m, const DenseOut& o, cudaStream_t s) {

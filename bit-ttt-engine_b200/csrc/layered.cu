@@ -52,7 +52,6 @@ struct RowBuffers {
     uint8_t* ft = nullptr;
     uint8_t* t1 = nullptr;
     uint8_t* t2 = nullptr;
-    float* scratch = nullptr;  // partial sums of the tcgen05 product
     // mixture of experts
     float* logits = nullptr;
     int* choice = nullptr;     // chosen expert, place, destination per row; counts, starts, tiles
@@ -63,7 +62,7 @@ struct RowBuffers {
     int64_t grouped = 0;
     void release() {
         for (void* p : {(void*)proj, (void*)mix, (void*)y, (void*)ff, (void*)conv, (void*)v_first, (void*)hn, (void*)cat, (void*)a, (void*)b, (void*)c, (void*)wkv_pre, q,
-                        (void*)xt, (void*)mt, (void*)ft, (void*)t1, (void*)t2, (void*)scratch, (void*)logits, (void*)choice, (void*)wt, (void*)xe, (void*)fe, (void*)ye})
+                        (void*)xt, (void*)mt, (void*)ft, (void*)t1, (void*)t2, (void*)logits, (void*)choice, (void*)wt, (void*)xe, (void*)fe, (void*)ye})
             cudaFree(p);
         *this = RowBuffers();
     }
@@ -255,15 +254,6 @@ bt_status alloc_rows(const bt_model* m, RowBuffers& r, int rows, bool wide) {
             for (const LayLayer& l : L->layers)
                 if (l.c.mixer == BT_MIX_WKV) pre = std::max(pre, wkv_prefix_floats(l.c.heads, l.c.dim, rows, L->c.max_batch));
             BT_CUDA_TRY(dev_alloc(&r.wkv_pre, (size_t)pre));
-            size_t scratch = 0;
-            for (const LayLayer& l : L->layers) {
-                size_t count;
-                const DenseLin* const* all = l.lins(&count);
-                for (size_t i = 0; i < count; ++i)
-                    if (all[i]->tiles) scratch = std::max(scratch, dense_tc_scratch(*all[i], std::min(rows, 128), m->sm_count));
-            }
-            if (L->loops()) scratch = std::max(scratch, dense_tc_scratch(L->loop_in, std::min(rows, 128), m->sm_count));
-            BT_CUDA_TRY(dev_alloc(&r.scratch, scratch));
             struct { uint8_t** p; int k; } tiles[] = {{&r.xt, L->loops() ? 2 * kpw : W}, {&r.mt, q.mt}, {&r.ft, q.ft}, {&r.t1, q.t1}, {&r.t2, q.t2}};
             for (auto& t : tiles) {  // zeroed once: rows and columns of the padding stay finite
                 const size_t bytes = mp * dense_kpad(std::max(t.k, 1)) * 2;
@@ -563,7 +553,7 @@ struct RowPass {
     }
     cudaError_t product(int part, const DenseLin& lin, const uint8_t* xt, const float* x, int64_t ldx, const DenseOut& o, int64_t x_block = 0) {
         if (!(parts & part)) return cudaSuccess;
-        return f32 ? launch_dense_f32(lin, x, ldx, x_block, M, o, s) : launch_dense_tc(lin, xt, M, o, r.scratch, err, sm, s);
+        return f32 ? launch_dense_f32(lin, x, ldx, x_block, M, o, s) : launch_dense_tc(lin, xt, M, o, err, sm, s);
     }
     // f32 rows a sublayer reads (f32 models)
     const float* in_rows() const { return L->c.pre_norm ? r.hn : h; }
@@ -648,7 +638,7 @@ struct RowPass {
                 o.out_rows16 = L->kv16; o.ld = l.expand.n; o.out_block = seq; o.shared_weights = true; o.blocks = nb; o.x_block = tile_bytes; o.m_pad = tile_rows;
                 if (parts & PART_MID) {
                     BT_CUDA_TRY(launch_latent_tiles(a.kv, b0, nb, past + n, tiles, tile_rows, s));
-                    BT_CUDA_TRY(launch_dense_tc(l.expand, tiles, past + n, o, nullptr, err, sm, s));
+                    BT_CUDA_TRY(launch_dense_tc(l.expand, tiles, past + n, o, err, sm, s));
                 }
                 if (parts & PART_CORE) BT_CUDA_TRY(launch_latent_tile(a, L->kv16, rows, b0, nb, tiled(r.mt), s));
             }
@@ -1065,22 +1055,21 @@ int layered_launches(const bt_model* m, int batch) {
     const Layered* L = m->lay;
     const bool fused = step_is_fused(m, batch);
     int n = 1 + (fused ? 1 : 0);  // embedding; fused: the last residual sum
-    auto product = [&](const DenseLin& d, int act = DACT_NONE) { return fused || L->f32 ? 1 : dense_tc_kernels(d, batch, m->sm_count, act); };
     if (!fused && L->c.pre_norm && L->runs[0].pass < 0) ++n;
     for (const LayRun& run : L->runs) {
         const LayLayer& l = L->layers[(size_t)run.layer];
         const bool b16 = !L->f32;
-        if (run.pass >= 0) n += product(L->loop_in) + (fused ? 0 : 1);
-        n += product(l.in) + 1 + product(l.o);  // with attention or recurrence
+        if (run.pass >= 0) n += 1 + (fused ? 0 : 1);
+        n += 3;  // with attention or recurrence
         switch (l.c.mixer) {
             case BT_MIX_SSM: n += fused ? 0 : 1; break;
-            case BT_MIX_LATENT: n += product(l.mid) + product(l.mid2) + (fused ? 0 : 1 + (b16 && l.c.vdim % 8 ? 1 : 0)); break;
-            case BT_MIX_WKV: n += fused ? 0 : 2 + product(l.mid) + product(l.mid2) + (b16 ? 1 : 0); break;
-            case BT_MIX_RGLRU: n += fused ? 0 : 1 + product(l.mid); break;
+            case BT_MIX_LATENT: n += 2 + (fused ? 0 : 1 + (b16 && l.c.vdim % 8 ? 1 : 0)); break;
+            case BT_MIX_WKV: n += fused ? 0 : 4 + (b16 ? 1 : 0); break;
+            case BT_MIX_RGLRU: n += fused ? 0 : 2; break;
         }
-        if (l.c.mlp == BT_MLP_DENSE_RELU2) n += product(l.up) + product(l.down);
+        if (l.c.mlp == BT_MLP_DENSE_RELU2) n += 2;
         if (l.c.mlp == BT_MLP_MOE_SWIGLU)
-            n += fused ? 3 : product(l.router) + 3 + 2 + (l.c.shared_ff ? product(l.s_up, DACT_SWIGLU) + product(l.s_down) : 0);
+            n += fused ? 3 : 6 + (l.c.shared_ff ? 2 : 0);
         if (!fused) n += 1 + (l.c.mlp != BT_MLP_NONE ? 1 : 0);
     }
     if (m->lm_tiles && batch > 8) return n + 4;  // prepare, product, arg-max, position advance
