@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row_sets = a.n_pad / kTcRows;
+    if (a.plan) ptx::pdl_wait();  // (written by the kernel in front)
     const int tok_blocks = a.plan ? *a.n_plan : (int)((a.m + NT - 1) / NT);
     const int tiles = row_sets * tok_blocks * a.splits * a.blocks;
 
@@ -432,19 +433,32 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(const TcArgs a)
 
     if (warp == 0) {
         if (lane == 0) {
+            // The weights do not depend on earlier kernels: those of the first stages are requested before the wait on the
+            // kernel in front (a row kernel as a rule, which leaves room beside it), their activations after it.
+            auto issue = [&](const Tile& d, int kc, int slot, bool weights, bool inputs) {
+                const uint32_t x_bytes = tile_rows(d) * 128;
+                uint8_t* st = smem + (size_t)slot * Cfg::kStageBytes;
+                if (weights) {
+                    const int wc = kc >= a.w_chunks ? kc - a.w_chunks : kc;  // hi and lo halves meet the same weights
+                    ptx::mbar_arrive_expect_tx(&full[slot], kTcRows * 128 + x_bytes);
+                    ptx::bulk_g2s(st, a.w + (int64_t)d.blk * a.w_block + (int64_t)d.rs * kTcRows * 128 + (int64_t)wc * a.n_pad * 128, kTcRows * 128, &full[slot]);
+                }
+                if (inputs)
+                    ptx::bulk_g2s(st + kTcRows * 128, a.x + (a.plan ? 0 : (int64_t)d.blk * a.x_block) + d.tok0 * 128 + (int64_t)kc * a.m_pad * 128, x_bytes, &full[slot]);
+            };
+            int ahead = 0;
+            for (int t = blockIdx.x; t < tiles && ahead < S; t += gridDim.x) {
+                const Tile d = decode(t);
+                for (int kc = d.c0; kc < d.c1 && ahead < S; ++kc, ++ahead) issue(d, kc, ahead, true, false);
+            }
+            ptx::pdl_wait();
+            ptx::pdl_launch_dependents();
             int slot = 0, issued = 0; uint32_t par = 1; bool first = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const Tile d = decode(t);
-                const uint8_t* wp = a.w + (int64_t)d.blk * a.w_block + (int64_t)d.rs * kTcRows * 128;
-                const uint8_t* xp = a.x + (a.plan ? 0 : (int64_t)d.blk * a.x_block) + d.tok0 * 128;
-                const uint32_t x_bytes = tile_rows(d) * 128;
                 for (int kc = d.c0; kc < d.c1; ++kc) {
-                    const int wc = kc >= a.w_chunks ? kc - a.w_chunks : kc;  // hi and lo halves meet the same weights
                     if (!first) { if (!ptx::mbar_wait_bounded(&empty[slot], par)) { ok = false; break; } }
-                    uint8_t* st = smem + (size_t)slot * Cfg::kStageBytes;
-                    ptx::mbar_arrive_expect_tx(&full[slot], kTcRows * 128 + x_bytes);
-                    ptx::bulk_g2s(st, wp + (int64_t)wc * a.n_pad * 128, kTcRows * 128, &full[slot]);
-                    ptx::bulk_g2s(st + kTcRows * 128, xp + (int64_t)kc * a.m_pad * 128, x_bytes, &full[slot]);
+                    issue(d, kc, slot, issued >= ahead, true);
                     ++issued;
                     if (++slot == S) { slot = 0; first = false; par ^= 1; }
                 }
@@ -614,8 +628,7 @@ cudaError_t tc_launch_e(const TcArgs& a, int sm_count, cudaStream_t s) {
     cudaError_t e = once.run([] { return cudaFuncSetAttribute(dense_tc_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<NT>::kSmem); });
     if (e != cudaSuccess) return e;
     const int64_t tiles = (int64_t)(a.n_pad / kTcRows) * ((a.m + NT - 1) / NT) * a.splits * a.blocks;  // a.m: the plan's upper bound
-    dense_tc_kernel<NT, EPI><<<(unsigned)(tiles < sm_count ? tiles : sm_count), kTcThreads, TcCfg<NT>::kSmem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(dense_tc_kernel<NT, EPI>, dim3((unsigned)(tiles < sm_count ? tiles : sm_count)), dim3(kTcThreads), TcCfg<NT>::kSmem, s, true, a);
 }
 // How many clusters of `splits` CTAs of the split product the GPU holds at once (a cluster lives inside one GPC); 0: none.
 template <int NT>
@@ -653,11 +666,13 @@ cudaError_t tc_launch_split(const TcArgs& a, cudaStream_t s) {
     cfg.blockDim = dim3(kTcThreads);
     cfg.dynamicSmemBytes = TcCfg<NT>::kSmem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)a.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, dense_tc_kernel<NT, TC_SPLIT>, a);
 }
 template <int NT>
@@ -959,6 +974,8 @@ __global__ void __launch_bounds__(512) row_op_kernel(const RowArgs a) {
 // f32 rows in parts -> tiled bf16 (hi | lo): a thread per 8 columns of one row
 __global__ void __launch_bounds__(256) rows_tile_kernel(const float* __restrict__ x, int64_t ld, int64_t x_block, int blocks, int k, int halves,
                                                         int act, int64_t rows, uint8_t* __restrict__ tiles, int64_t m_pad) {
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const int kp = dense_kpad(k), per = kp / 8;
     const int64_t total = rows * blocks * per;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1087,8 +1104,8 @@ cudaError_t launch_rows_tile(const float* x, int64_t ld, int64_t x_block, int bl
                              uint8_t* tiles, int64_t m_pad, cudaStream_t s) {
     if (halves < 1 || halves > 2 || act >= DACT_SWIGLU) return cudaErrorInvalidValue;
     const int64_t total = rows * blocks * (dense_kpad(k) / 8);
-    rows_tile_kernel<<<(unsigned)((total + 255) / 256 < 4736 ? (total + 255) / 256 : 4736), 256, 0, s>>>(x, ld, x_block, blocks, k, halves, act, rows, tiles, m_pad);
-    return cudaGetLastError();
+    return launch_pdl(rows_tile_kernel, dim3((unsigned)((total + 255) / 256 < 4736 ? (total + 255) / 256 : 4736)), dim3(256), 0, s, true, x, ld, x_block, blocks, k,
+                      halves, act, rows, tiles, m_pad);
 }
 
 cudaError_t launch_embed_pos(const int32_t* tokens, const __nv_bfloat16* table, const __nv_bfloat16* pos_table,

@@ -57,10 +57,12 @@ __device__ __forceinline__ float latent_inv(const LatentAttn& a, const float* c,
 __global__ void __launch_bounds__(256) latent_prep_kernel(const LatentAttn a) {
     __shared__ float red[32];
     const int64_t r = blockIdx.x;
-    const int b = (int)(r / a.q_rows), p = a.pos[b] + (int)(r % a.q_rows);
+    const int b = (int)(r / a.q_rows), p = a.pos[b] + (int)(r % a.q_rows);  // (positions are set before the step's first kernel)
     const float* row = a.proj + r * a.ld;
     const int H = a.heads, hd = a.dim + a.rot, kr = a.kv.rot_col();
     const float* c = row + H * hd;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const float inv = latent_inv(a, c, red);
     if (p < 0 || p >= a.kv.max_seq) return;
     uint8_t* seq = reinterpret_cast<uint8_t*>(a.kv.rows) + b * a.kv.seq_bytes();
@@ -102,6 +104,8 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(const LatentAttn a) {
 }
 
 __global__ void __launch_bounds__(256) latent_tiles_kernel(const LatentView v, int b0, int64_t n, uint8_t* __restrict__ tiles, int64_t m_pad) {
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const int per = dense_kpad(v.rank) / 8;  // pieces per position
     const int64_t groups = (n + 7) / 8, total = groups * per * 8;
     const uint8_t* src = reinterpret_cast<const uint8_t*>(v.rows) + (b0 + (int64_t)blockIdx.y) * v.seq_bytes();
@@ -621,13 +625,11 @@ int latent_max_rot() { return kMaxRot; }
 cudaError_t launch_latent_tiles(const LatentView& v, int b0, int nb, int64_t n, uint8_t* tiles, int64_t m_pad, cudaStream_t s) {
     if (v.f32) return cudaErrorInvalidValue;
     const int64_t total = (n + 7) / 8 * dense_kpad(v.rank);
-    latent_tiles_kernel<<<dim3((unsigned)((total + 255) / 256 < 592 ? (total + 255) / 256 : 592), (unsigned)nb), 256, 0, s>>>(v, b0, n, tiles, m_pad);
-    return cudaGetLastError();
+    return launch_pdl(latent_tiles_kernel, dim3((unsigned)((total + 255) / 256 < 592 ? (total + 255) / 256 : 592), (unsigned)nb), dim3(256), 0, s, true, v, b0, n, tiles, m_pad);
 }
 
 cudaError_t launch_latent_prep(const LatentAttn& a, cudaStream_t s) {
-    latent_prep_kernel<<<(unsigned)(a.batch * a.q_rows), 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(latent_prep_kernel, dim3((unsigned)(a.batch * a.q_rows)), dim3(256), 0, s, true, a);
 }
 
 cudaError_t launch_latent_span(const LatentAttn& a, bool prepared, const ActOut& out, cudaStream_t s, bool pdl) {

@@ -581,7 +581,7 @@ struct RowPass {
             a.op = ROW_GROUPNORM; a.y = h; a.ld = W; a.w = w; a.eps = eps; a.rows = M; a.k = W;
             const bool rows = f32 || L->layers[(size_t)run.layer].c.mixer == BT_MIX_WKV;
             a.act = rows ? plain(r.hn, W) : tiled(r.xt);
-            if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(a, s, false));
+            if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(a, s, true));
         } else if (L->layers[(size_t)run.layer].c.mixer == BT_MIX_WKV) {
             BT_CUDA_TRY(cudaMemcpyAsync(r.hn, h, (size_t)M * W * sizeof(float), cudaMemcpyDeviceToDevice, s));
         } else if (!f32) {
@@ -615,7 +615,7 @@ struct RowPass {
         g.op = ROW_GROUPNORM; g.y = r.mix; g.ld = l.inner(); g.w = l.vec[BT_LT_SSM_NORM]; g.eps = eps; g.groups = l.c.norm_groups;
         g.rows = M; g.k = l.inner();
         g.act = f32 ? plain(r.proj, l.inner()) : tiled(r.mt);  // the projection rows are used up
-        if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(g, s, false));
+        if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(g, s, true));
         return BT_OK;
     }
     bt_status latent(LayLayer& l, LayRun& run) {
@@ -681,7 +681,7 @@ struct RowPass {
         g.op = ROW_GROUPNORM; g.y = r.mix; g.ld = HD; g.w = l.vec[BT_LT_WKV_NORM]; g.eps = eps; g.groups = l.c.heads; g.rows = M; g.k = HD;
         g.gate = r.proj + 3ll * HD; g.gate_ld = 4ll * HD;
         g.act = f32 ? plain(r.c, HD) : tiled(r.mt);
-        if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(g, s, false));
+        if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(g, s, true));
         return BT_OK;
     }
     bt_status rglru(LayLayer& l, LayRun& run) {
@@ -771,7 +771,7 @@ struct RowPass {
             res.w = l.vec[BT_LT_NORM1];
             const bool mlp = l.c.mlp != BT_MLP_NONE;
             next_input(mlp ? ri : ri + 1, mlp, res);
-            if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(res, s, false));
+            if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(res, s, true));
             if (mlp) {
                 if (l.c.mlp == BT_MLP_DENSE_RELU2) {
                     DenseOut up = rows_out(f32 ? r.ff : nullptr, l.c.ff, DACT_RELU2);
@@ -783,7 +783,7 @@ struct RowPass {
                 }
                 res.w = l.vec[BT_LT_NORM2];
                 next_input(ri + 1, false, res);
-                if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(res, s, false));
+                if (parts & PART_ROWS) BT_CUDA_TRY(launch_row_op(res, s, true));
             }
             BT_CUDA_TRY(trace_stream(m, (int)ri, h, M, s));
         }

@@ -16,7 +16,9 @@ namespace {
 constexpr int kRows = 128, kChunk = 64, kTok = 64, kCols = 2 * kTok;  // N = hi | lo
 constexpr int kATile = kRows * kChunk * 2;                              // 16 KB
 constexpr int kBTile = kCols * kChunk * 2;                              // 16 KB
-constexpr int kStages = 4;
+// As many chunks of weights and activations in flight as fit: bound by the reads of the weights, and 16 tokens bring a quarter of
+// the activations of 64, so that eleven stages fit instead of four (32000 x 2560, 16 tokens: 34 -> 29 us).
+constexpr int kRingBytes = 224 * 1024, kMaxStages = 12;
 constexpr int kThreads = 6 * 32;
 constexpr unsigned kErrLmTimeout = 0x4c4d4844u;  // 'LMHD'
 
@@ -58,47 +60,93 @@ __global__ void lm_retile_kernel(const __nv_bfloat16* __restrict__ w, int64_t vo
 // RMSNorm of up to 64 tokens, split into bf16 hi | lo, laid out as the B tiles of every k-chunk
 // f16: the pieces are IEEE halves (hi + lo = 11 + 11 significand bits; a lo piece below 6e-5 is subnormal and
 // keeps an absolute accuracy of 2^-25) to match weights stored as halves; otherwise bf16 (8 + 8 bits).
-__global__ void __launch_bounds__(256) lm_prep_kernel(const float* __restrict__ h, const float* __restrict__ norm_w,
-                                                      float eps, int hidden, int m, uint8_t* __restrict__ btiles, bool f16) {
+// cols: columns of the product, hi | lo of cols / 2 tokens.  A thread takes eight inputs at a time (one 16-byte piece of either
+// part), and up to kPrepKeep of them stay in registers between the two passes (64 x 4096: 12.5 us with a value a thread, 3 us).
+constexpr int kPrepThreads = 256, kPrepKeep = 2;
+__global__ void __launch_bounds__(kPrepThreads) lm_prep_kernel(const float* __restrict__ h, const float* __restrict__ norm_w,
+                                                               float eps, int hidden, int m, int cols, uint8_t* __restrict__ btiles, bool f16) {
     __shared__ double red[32];
-    const int token = blockIdx.x;  // 0..63
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    const int token = blockIdx.x;  // 0 .. cols / 2 - 1
     const bool real = token < m;
     const float* hr = h + (int64_t)(real ? token : 0) * hidden;
+    const bool vec = ((reinterpret_cast<uintptr_t>(hr) | reinterpret_cast<uintptr_t>(norm_w)) & 15) == 0;
+    auto get = [&](const float* p, int c0, float (&v)[8]) {
+        if (vec && c0 + 8 <= hidden) {
+            const float4 x = *reinterpret_cast<const float4*>(p + c0), y = *reinterpret_cast<const float4*>(p + c0 + 4);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = c0 + j < hidden ? p[c0 + j] : 0.0f;
+        }
+    };
+    const int padded = (hidden + kChunk - 1) / kChunk * kChunk;
+    float keep[kPrepKeep][8];
     double ss = 0.0;
+    auto squares = [&](const float (&v)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss = fma((double)v[j], (double)v[j], ss);
+    };
+#pragma unroll
+    for (int i = 0; i < kPrepKeep; ++i) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) keep[i][j] = 0.0f;
+        if (real) get(hr, (i * kPrepThreads + (int)threadIdx.x) * 8, keep[i]);
+        squares(keep[i]);
+    }
     if (real)
-        for (int c = threadIdx.x; c < hidden; c += blockDim.x) ss = fma((double)hr[c], (double)hr[c], ss);
+        for (int c0 = (kPrepKeep * kPrepThreads + (int)threadIdx.x) * 8; c0 < hidden; c0 += kPrepThreads * 8) {
+            float v[8];
+            get(hr, c0, v);
+            squares(v);
+        }
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
     ss = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) ss += red[w];
+    for (int w = 0; w < kPrepThreads / 32; ++w) ss += red[w];
     const float denom = sqrtf(__fadd_rn((float)(ss / (double)hidden), eps));
-    for (int c = threadIdx.x; c < (hidden + kChunk - 1) / kChunk * kChunk; c += blockDim.x) {
-        const float v = real && c < hidden ? __fmul_rn(__fdiv_rn(hr[c], denom), norm_w[c]) : 0.0f;
-        uint8_t* tile = btiles + (int64_t)(c / kChunk) * kBTile;
-        if (f16) {
-            const __half hi = __float2half_rn(v);
-            const __half lo = __float2half_rn(v - __half2float(hi));
-            *reinterpret_cast<__half*>(tile + tile_off(token, c % kChunk, kChunk)) = hi;
-            *reinterpret_cast<__half*>(tile + tile_off(kTok + token, c % kChunk, kChunk)) = lo;
-        } else {
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-            const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-            *reinterpret_cast<__nv_bfloat16*>(tile + tile_off(token, c % kChunk, kChunk)) = hi;
-            *reinterpret_cast<__nv_bfloat16*>(tile + tile_off(kTok + token, c % kChunk, kChunk)) = lo;
+    auto put = [&](int c0, const float (&x)[8]) {
+        if (c0 >= padded) return;
+        float w[8];
+        uint32_t hi[4], lo[4];
+        get(norm_w, c0, w);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            const float a = real ? __fmul_rn(__fdiv_rn(x[j], denom), w[j]) : 0.0f, b = real ? __fmul_rn(__fdiv_rn(x[j + 1], denom), w[j + 1]) : 0.0f;
+            if (f16) {
+                const __half2 u = __floats2half2_rn(a, b), l = __floats2half2_rn(a - __low2float(u), b - __high2float(u));
+                hi[j / 2] = *reinterpret_cast<const uint32_t*>(&u);
+                lo[j / 2] = *reinterpret_cast<const uint32_t*>(&l);
+            } else {
+                hi[j / 2] = ptx::pack2(a, b);
+                lo[j / 2] = ptx::pack2(a - __uint_as_float(hi[j / 2] << 16), b - __uint_as_float(hi[j / 2] & 0xffff0000u));
+            }
         }
+        uint8_t* tile = btiles + (int64_t)(c0 / kChunk) * (cols * kChunk * 2);
+        *reinterpret_cast<uint4*>(tile + tile_off(token, c0 % kChunk, kChunk)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(tile + tile_off(cols / 2 + token, c0 % kChunk, kChunk)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    };
+#pragma unroll
+    for (int i = 0; i < kPrepKeep; ++i) put((i * kPrepThreads + (int)threadIdx.x) * 8, keep[i]);
+    for (int c0 = (kPrepKeep * kPrepThreads + (int)threadIdx.x) * 8; c0 < padded; c0 += kPrepThreads * 8) {
+        float v[8];
+        get(hr, c0, v);
+        put(c0, v);
     }
 }
 
 __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* __restrict__ wtiles,
                                                                  const uint8_t* __restrict__ btiles, int64_t vocab,
-                                                                 int hidden, int m, float* __restrict__ logits,
+                                                                 int hidden, int m, int cols, int stages, float* __restrict__ logits,
                                                                  unsigned int* err, bool w_f16, float cap) {
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* stage_base = smem;  // kStages x (A tile | B tile)
-    uint64_t* full = reinterpret_cast<uint64_t*>(stage_base + (size_t)kStages * (kATile + kBTile));
-    uint64_t* empty = full + kStages;
-    uint64_t* acc_full = empty + kStages;
+    const int b_tile = cols * kChunk * 2, stage_bytes = kATile + b_tile;  // cols: hi | lo of the tokens, padded to 16 each
+    uint8_t* stage_base = smem;  // stages x (A tile | B tile)
+    uint64_t* full = reinterpret_cast<uint64_t*>(stage_base + (size_t)stages * stage_bytes);
+    uint64_t* empty = full + kMaxStages;
+    uint64_t* acc_full = empty + kMaxStages;
     uint64_t* acc_empty = acc_full + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -106,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* 
     const int64_t row_sets = (vocab + kRows - 1) / kRows;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
         ptx::mbar_init(acc_full, 1);
         ptx::mbar_init(acc_empty, 128);
         ptx::mbar_fence_init();
@@ -120,20 +168,28 @@ __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* 
 
     if (warp == 0) {
         if (lane == 0) {
-            int slot = 0; uint32_t par = 1; bool first = true;
+            // the weights of the first stages are requested before the wait on the kernel in front, which wrote the activations
+            int ahead = 0;
+            auto weights = [&](int64_t rs, int kc, int slot) {
+                ptx::mbar_arrive_expect_tx(&full[slot], stage_bytes);
+                ptx::bulk_g2s(stage_base + (size_t)slot * stage_bytes, wtiles + (rs * chunks + kc) * (int64_t)kATile, kATile, &full[slot]);
+            };
+            for (int64_t rs = blockIdx.x; rs < row_sets && ahead < stages; rs += gridDim.x)
+                for (int kc = 0; kc < chunks && ahead < stages; ++kc, ++ahead) weights(rs, kc, ahead);
+            ptx::pdl_wait();
+            ptx::pdl_launch_dependents();
+            int slot = 0, issued = 0; uint32_t par = 1; bool first = true;
             for (int64_t rs = blockIdx.x; rs < row_sets; rs += gridDim.x)
                 for (int kc = 0; kc < chunks; ++kc) {
                     if (!first) ok &= ptx::mbar_wait_bounded(&empty[slot], par);
-                    uint8_t* st = stage_base + (size_t)slot * (kATile + kBTile);
-                    ptx::mbar_arrive_expect_tx(&full[slot], kATile + kBTile);
-                    ptx::bulk_g2s(st, wtiles + (rs * chunks + kc) * (int64_t)kATile, kATile, &full[slot]);
-                    ptx::bulk_g2s(st + kATile, btiles + (int64_t)kc * kBTile, kBTile, &full[slot]);
-                    if (++slot == kStages) { slot = 0; first = false; par ^= 1; }
+                    if (issued++ >= ahead) weights(rs, kc, slot);
+                    ptx::bulk_g2s(stage_base + (size_t)slot * stage_bytes + kATile, btiles + (int64_t)kc * b_tile, b_tile, &full[slot]);
+                    if (++slot == stages) { slot = 0; first = false; par ^= 1; }
                 }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = instr_desc_bf16(kRows, kCols, w_f16);
+            const uint32_t idesc = instr_desc_bf16(kRows, cols, w_f16);
             int slot = 0; uint32_t par = 0, acc_par = 0; bool first_tile = true;
             for (int64_t rs = blockIdx.x; rs < row_sets; rs += gridDim.x) {
                 if (!first_tile) { ok &= ptx::mbar_wait_bounded(acc_empty, acc_par); acc_par ^= 1; }
@@ -142,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* 
                 for (int kc = 0; kc < chunks; ++kc) {
                     ok &= ptx::mbar_wait_bounded(&full[slot], par);
                     ptx::tc_fence_after();
-                    const uint32_t a_addr = ptx::smem_u32(stage_base + (size_t)slot * (kATile + kBTile));
+                    const uint32_t a_addr = ptx::smem_u32(stage_base + (size_t)slot * stage_bytes);
                     const uint32_t b_addr = a_addr + kATile;
 #pragma unroll
                     for (int ks = 0; ks < kChunk / 16; ++ks) {  // K = 16 bf16 = 2 core matrices per MMA
@@ -151,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* 
                         ptx::umma_f16(tmem_base, ad, bd, idesc, (kc > 0 || ks > 0) ? 1u : 0u);
                     }
                     ptx::umma_commit(&empty[slot]);
-                    if (++slot == kStages) { slot = 0; par ^= 1; }
+                    if (++slot == stages) { slot = 0; par ^= 1; }
                 }
                 ptx::umma_commit(acc_full);
             }
@@ -165,14 +221,14 @@ __global__ void __launch_bounds__(kThreads, 1) lm_head_tc_kernel(const uint8_t* 
             ptx::tc_fence_after();
             const int64_t v = rs * kRows + sub * 32 + lane;
 #pragma unroll 1
-            for (int c0 = 0; c0 < kTok; c0 += 32) {
-                uint32_t hi[32], lo[32];
+            for (int c0 = 0; c0 < cols / 2; c0 += 16) {
+                uint32_t hi[16], lo[16];
                 const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16) + c0;
-                ptx::tmem_ld32(taddr, hi);
-                ptx::tmem_ld32(taddr + kTok, lo);
+                ptx::tmem_ld16(taddr, hi);
+                ptx::tmem_ld16(taddr + cols / 2, lo);
                 ptx::tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
+                for (int j = 0; j < 16; ++j) {
                     const int token = c0 + j;
                     if (token < m && v < vocab) {
                         float r = __fadd_rn(__uint_as_float(hi[j]), __uint_as_float(lo[j]));
@@ -207,21 +263,22 @@ cudaError_t launch_lm_retile(const __nv_bfloat16* w, int64_t vocab, int hidden, 
 cudaError_t launch_lm_head_tc(const void* wtiles, const float* h, const float* norm_w, float eps, int batch, int hidden,
                               int64_t vocab, void* btiles, float* logits, unsigned int* err, int sm_count,
                               cudaStream_t stream, bool w_f16, float cap) {
-    const size_t smem = (size_t)kStages * (kATile + kBTile) + 256;
+    constexpr size_t most = kRingBytes + 256;
     static PerDeviceOnce once;
-    cudaError_t ce = once.run([smem] { return cudaFuncSetAttribute(lm_head_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-    if (ce != cudaSuccess) return ce;
+    cudaError_t ce = once.run([] { return cudaFuncSetAttribute(lm_head_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most); });
     const int64_t row_sets = (vocab + kRows - 1) / kRows;
     const int grid = (int)(row_sets < sm_count ? row_sets : sm_count);
-    for (int b0 = 0; b0 < batch; b0 += kTok) {
+    for (int b0 = 0; b0 < batch && ce == cudaSuccess; b0 += kTok) {
         const int bc = batch - b0 < kTok ? batch - b0 : kTok;
-        lm_prep_kernel<<<kTok, 256, 0, stream>>>(h + (size_t)b0 * hidden, norm_w, eps, hidden, bc,
-                                                 reinterpret_cast<uint8_t*>(btiles), w_f16);
-        lm_head_tc_kernel<<<grid, kThreads, smem, stream>>>(reinterpret_cast<const uint8_t*>(wtiles),
-                                                           reinterpret_cast<const uint8_t*>(btiles), vocab, hidden, bc,
-                                                           logits + (size_t)b0 * vocab, err, w_f16, cap);
+        const int cols = (bc + 15) / 16 * 32, stage = kATile + cols * kChunk * 2;  // a product as wide as the tokens need
+        const int stages = kRingBytes / stage < kMaxStages ? kRingBytes / stage : kMaxStages;
+        ce = launch_pdl(lm_prep_kernel, dim3((unsigned)(cols / 2)), dim3(kPrepThreads), 0, stream, true, h + (size_t)b0 * hidden, norm_w, eps, hidden, bc, cols,
+                        reinterpret_cast<uint8_t*>(btiles), w_f16);
+        if (ce == cudaSuccess)
+            ce = launch_pdl(lm_head_tc_kernel, dim3((unsigned)grid), dim3(kThreads), (size_t)stages * stage + 256, stream, true, reinterpret_cast<const uint8_t*>(wtiles),
+                            reinterpret_cast<const uint8_t*>(btiles), vocab, hidden, bc, cols, stages, logits + (size_t)b0 * vocab, err, w_f16, cap);
     }
-    return cudaGetLastError();
+    return ce;
 }
 
 }  // namespace bt

@@ -213,6 +213,8 @@ __global__ void __launch_bounds__(256) moe_choose_kernel(const MoeRoute a) {
     extern __shared__ float zs[];  // [8][experts], then choices and weights
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 8 + warp;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if (r >= a.rows) return;
     float* z = zs + warp * a.experts;
     int* sel = reinterpret_cast<int*>(zs + 8 * a.experts) + warp * a.top;
@@ -232,6 +234,8 @@ __global__ void __launch_bounds__(256) moe_choose_kernel(const MoeRoute a) {
 __global__ void __launch_bounds__(kMaxExperts) moe_plan_kernel(const MoeRoute a) {
     __shared__ int rows_s[32], tiles_s[32];
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const int n = e < a.experts ? a.counts[e] : 0;
     const int padded = (n + 7) / 8 * 8, nt = (n + a.tile - 1) / a.tile;
     int rs = padded, ts = nt;
@@ -275,6 +279,8 @@ __global__ void __launch_bounds__(kMaxExperts) moe_plan_kernel(const MoeRoute a)
 __global__ void __launch_bounds__(256) moe_group_kernel(const MoeRoute a) {
     __shared__ int dst[kMaxTop];
     const int64_t r = blockIdx.x;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if ((int)threadIdx.x < a.top) {
         const int d = a.row_start[a.sel[r * a.top + threadIdx.x]] + a.rank[r * a.top + threadIdx.x];
         dst[threadIdx.x] = d;
@@ -341,10 +347,9 @@ int64_t moe_grouped_rows(int64_t rows, int top, int experts) { return (rows * to
 cudaError_t launch_moe_route(const MoeRoute& a, cudaStream_t s) {
     if (a.experts > kMaxExperts || a.top > kMaxTop || a.top > a.experts) return cudaErrorInvalidValue;
     const size_t smem = (size_t)8 * (a.experts + 2 * a.top) * sizeof(float);
-    moe_choose_kernel<<<(unsigned)((a.rows + 7) / 8), 256, smem, s>>>(a);
-    moe_plan_kernel<<<1, kMaxExperts, 0, s>>>(a);
-    moe_group_kernel<<<(unsigned)a.rows, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    cudaError_t e = launch_pdl(moe_choose_kernel, dim3((unsigned)((a.rows + 7) / 8)), dim3(256), smem, s, true, a);
+    if (e == cudaSuccess) e = launch_pdl(moe_plan_kernel, dim3(1), dim3(kMaxExperts), 0, s, true, a);
+    return e == cudaSuccess ? launch_pdl(moe_group_kernel, dim3((unsigned)a.rows), dim3(256), 0, s, true, a) : e;
 }
 
 }  // namespace bt

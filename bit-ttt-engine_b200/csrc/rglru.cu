@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(256) rglru_conv_kernel(const RgluArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kb = a.channels / a.blocks, kp = dense_kpad(kb);
     const int cg = blockIdx.x * 8 + warp;  // group of 32 padded columns
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if (cg * 32 >= a.blocks * kp) return;
     const int blk = cg * 32 / kp, c = cg * 32 - blk * kp + lane, ch = blk * kb + c;
     const bool live = c < kb;
@@ -117,7 +119,9 @@ __global__ void __launch_bounds__(kScanThreads, 1) rglru_scan_kernel(const RgluA
     const int c = lane % CH, seg = warp * TW + lane / CH;
     const int b = blockIdx.y, ch = blockIdx.x * CH + c, C = a.channels;
     const bool live = ch < C;
-    const int p0 = a.pos[b];
+    const int p0 = a.pos[b];  // (set before the step's first kernel: no kernel in front of this one writes positions)
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if (threadIdx.x < CH) carry[threadIdx.x] = blockIdx.x * CH + threadIdx.x < C && p0 > 0 ? a.state[(int64_t)b * C + blockIdx.x * CH + threadIdx.x] : 0.0f;
     const float lam8 = live ? -8.0f * softplus_f(a.lam[ch]) : 0.0f;
     const int64_t row0 = (int64_t)b * a.q_rows;
@@ -200,6 +204,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) rglru_scan_kernel(const RgluA
 // one token per sequence, gates and convolution done: a thread per channel and sequence
 __global__ void __launch_bounds__(128) rglru_one_kernel(const RgluArgs a, const ActOut out) {
     const int ch = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y, C = a.channels;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if (ch >= C) return;
     const int p = a.pos[b];
     const float2 g = *reinterpret_cast<const float2*>(a.gates + ((int64_t)b * C + ch) * 2);
@@ -219,19 +225,14 @@ __global__ void __launch_bounds__(128) rglru_one_kernel(const RgluArgs a, const 
 cudaError_t launch_rglru_conv(const RgluArgs& a, cudaStream_t s) {
     const int groups = a.blocks * dense_kpad(a.channels / a.blocks) / 32;
     const dim3 grid((unsigned)((groups + 7) / 8), (unsigned)((a.q_rows + kConvTokens - 1) / kConvTokens), (unsigned)a.batch);
-    if (a.taps <= 4) rglru_conv_kernel<4><<<grid, 256, 0, s>>>(a);
-    else rglru_conv_kernel<0><<<grid, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(a.taps <= 4 ? rglru_conv_kernel<4> : rglru_conv_kernel<0>, grid, dim3(256), 0, s, true, a);
 }
 
 cudaError_t launch_rglru_scan(const RgluArgs& a, const ActOut& out, cudaStream_t s) {
-    if (a.q_rows == 1)
-        rglru_one_kernel<<<dim3((unsigned)((a.channels + 127) / 128), (unsigned)a.batch), 128, 0, s>>>(a, out);
-    else if ((int64_t)a.channels * a.batch < 4096)
-        rglru_scan_kernel<16><<<dim3((unsigned)((a.channels + 15) / 16), (unsigned)a.batch), kScanThreads, 0, s>>>(a, out);
-    else
-        rglru_scan_kernel<32><<<dim3((unsigned)((a.channels + 31) / 32), (unsigned)a.batch), kScanThreads, 0, s>>>(a, out);
-    return cudaGetLastError();
+    if (a.q_rows == 1) return launch_pdl(rglru_one_kernel, dim3((unsigned)((a.channels + 127) / 128), (unsigned)a.batch), dim3(128), 0, s, true, a, out);
+    const int ch = (int64_t)a.channels * a.batch < 4096 ? 16 : 32;
+    return launch_pdl(ch == 16 ? rglru_scan_kernel<16> : rglru_scan_kernel<32>, dim3((unsigned)((a.channels + ch - 1) / ch), (unsigned)a.batch), dim3(kScanThreads), 0, s, true,
+                      a, out);
 }
 
 }  // namespace bt

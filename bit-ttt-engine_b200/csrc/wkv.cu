@@ -22,6 +22,8 @@ __global__ void __launch_bounds__(256) wkv_mix_kernel(const WkvMix a) {
     const int64_t r = blockIdx.x;
     const int b = (int)(r / a.q_rows), i = (int)(r % a.q_rows), W = a.width;
     const int p0 = a.pos[b];
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const float* h = a.hn + r * W;
     const float* before = i > 0 ? h - W : (p0 > 0 ? a.shift + (int64_t)((p0 + 1) & 1) * a.shift_slot + (int64_t)b * W : nullptr);
     for (int c = threadIdx.x; c < W; c += 256) {
@@ -30,9 +32,12 @@ __global__ void __launch_bounds__(256) wkv_mix_kernel(const WkvMix a) {
         for (int s = 0; s < 5; ++s) a.rows5[(r * 5 + s) * W + c] = fmaf(d, a.mu[s][c], v);
     }
 }
-// the same into tiles: a CTA per 8 rows, eight lanes per piece of 8 columns, so that a piece of the rows is one run of 128 bytes
+// the same into tiles: a CTA per 8 rows and 256 columns, eight lanes per piece of 8 columns, so that a piece of the rows is one
+// run of 128 bytes
 __global__ void __launch_bounds__(256) wkv_mix_tiles_kernel(const WkvMix a) {
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x & 7);
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     if (r >= (int64_t)a.batch * a.q_rows) return;
     const int b = (int)(r / a.q_rows), i = (int)(r % a.q_rows), W = a.width, kp = dense_kpad(W);
     const int p0 = a.pos[b];
@@ -48,27 +53,27 @@ __global__ void __launch_bounds__(256) wkv_mix_tiles_kernel(const WkvMix a) {
             for (int j = 0; j < 8; ++j) v[j] = p && c0 + j < W ? p[c0 + j] : 0.0f;
         }
     };
-    for (int c0 = (threadIdx.x >> 3) * 8; c0 < kp; c0 += 32 * 8) {
-        float v[8], d[8];
-        get(h, c0, v);
-        get(before, c0, d);
+    const int c0 = ((int)blockIdx.y * 32 + (int)(threadIdx.x >> 3)) * 8;
+    if (c0 >= kp) return;
+    float v[8], d[8];
+    get(h, c0, v);
+    get(before, c0, d);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) d[j] -= v[j];
+    for (int j = 0; j < 8; ++j) d[j] -= v[j];
 #pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            float m[8];
-            get(a.mu[s], c0, m);
-            uint32_t hi[4], lo[4];
+    for (int s = 0; s < 5; ++s) {
+        float m[8];
+        get(a.mu[s], c0, m);
+        uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                const float x = fmaf(d[j], m[j], v[j]), y = fmaf(d[j + 1], m[j + 1], v[j + 1]);
-                hi[j / 2] = ptx::pack2(x, y);
-                lo[j / 2] = ptx::pack2(x - __uint_as_float(hi[j / 2] << 16), y - __uint_as_float(hi[j / 2] & 0xffff0000u));
-            }
-            uint8_t* dst = s < 4 ? a.tiles4 + dense_off(r, s * kp + c0, a.m_pad) : a.tiles_w + dense_off(r, c0, a.m_pad);
-            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (s == 4) *reinterpret_cast<uint4*>(a.tiles_w + dense_off(r, kp + c0, a.m_pad)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        for (int j = 0; j < 8; j += 2) {
+            const float x = fmaf(d[j], m[j], v[j]), y = fmaf(d[j + 1], m[j + 1], v[j + 1]);
+            hi[j / 2] = ptx::pack2(x, y);
+            lo[j / 2] = ptx::pack2(x - __uint_as_float(hi[j / 2] << 16), y - __uint_as_float(hi[j / 2] & 0xffff0000u));
         }
+        uint8_t* dst = s < 4 ? a.tiles4 + dense_off(r, s * kp + c0, a.m_pad) : a.tiles_w + dense_off(r, c0, a.m_pad);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (s == 4) *reinterpret_cast<uint4*>(a.tiles_w + dense_off(r, kp + c0, a.m_pad)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
 }
 
@@ -752,9 +757,8 @@ int64_t wkv_prefix_floats(int heads, int dim, int64_t rows, int batch) { return 
 
 cudaError_t launch_wkv_mix(const WkvMix& a, cudaStream_t s) {
     const unsigned rows = (unsigned)(a.batch * a.q_rows);
-    if (a.rows5) wkv_mix_kernel<<<rows, 256, 0, s>>>(a);
-    else wkv_mix_tiles_kernel<<<(rows + 7) / 8, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    if (a.rows5) return launch_pdl(wkv_mix_kernel, dim3(rows), dim3(256), 0, s, true, a);
+    return launch_pdl(wkv_mix_tiles_kernel, dim3((rows + 7) / 8, (unsigned)(dense_kpad(a.width) + 255) / 256), dim3(256), 0, s, true, a);
 }
 
 cudaError_t launch_wkv_step(const WkvArgs& a, cudaStream_t s, bool pdl) {
@@ -766,7 +770,7 @@ cudaError_t launch_wkv_step(const WkvArgs& a, cudaStream_t s, bool pdl) {
 
 cudaError_t launch_wkv_prefill(const WkvArgs& a, cudaStream_t s) {
     if (a.dim > wkv_max_dim() || !a.w) return cudaErrorInvalidValue;
-    if (a.q_rows == 1) return step_launch(a, s, false);
+    if (a.q_rows == 1) return step_launch(a, s, true);
     if (takes_blocks(a)) return block_launch(a, s);
     if (a.dim <= 32) return scan_launch<1>(a, s);
     if (a.dim <= 64) return scan_launch<2>(a, s);
