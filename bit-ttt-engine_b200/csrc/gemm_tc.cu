@@ -96,6 +96,9 @@ struct TcArgs {
     int64_t out_stride;
     int epilogue;              // EPI_I32 / EPI_F32 / EPI_F32_ACCUM / EPI_BF16 / kEpiBf16Accum
     const float* acc_in;       // what the accumulating epilogues add to: [m, out_stride] f32
+    int bases;                 // up to 64 tokens: bases in this launch, one behind the other
+    int64_t basis_bytes;       // from one basis' weights to the next
+    float* sum;                // several bases and a bf16 output: [m, out_stride] f32, the bases so far
     unsigned int* err;
 };
 
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
     const int cid = blockIdx.x / kCtas, n_clusters = gridDim.x / kCtas;
     const int cps = (k_tiles + S - 1) / S;                 // chunks per split (the host makes every split non-empty)
     const int kt0 = PAIR ? 0 : rank * cps, kt1 = min(k_tiles, kt0 + cps);
+    const int bases = NT == 64 ? a.bases : 1;              // a tile's bases are worked through like tiles of their own
     const int n_tiles = row_sets * tok_blocks;             // this CTA works on the tiles cid, cid + n_clusters, ...
     // this CTA's row tiles of a tile begin at row_tile0(rs): rts(rs) of them exist (none, where the matrix ends in the first half)
     auto row_tile0 = [&](int rs) -> int64_t { return (int64_t)rs * (8 * kTileSets) + (PAIR ? 8 * rank : 0); };
@@ -188,14 +192,14 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         {
             // The weights do not depend on earlier kernels: the first stages' weight tiles are requested before the
             // dependency wait, their activation blocks (written by the quantiser just before) after it.
-            auto issue = [&](int tile, int kt, int slot, bool raw_part, bool b_part) {
+            auto issue = [&](int tile, int basis, int kt, int slot, bool raw_part, bool b_part) {
                 const int rs = tile % row_sets, tb = tile / row_sets;
                 uint8_t* st = stage_base + (size_t)slot * kStageBytes;
                 const int rts = row_tiles_of(rs);
                 if (raw_part) {
                     if (lane == 0) ptx::mbar_arrive_expect_tx(&full[slot], (uint32_t)(rts * kTileBytes + kBBytes));
                     if (lane < rts)
-                        ptx::bulk_g2s(st + lane * kTileBytes, a.tiles + ((row_tile0(rs) + lane) * k_tiles + kt) * kTileBytes, kTileBytes,
+                        ptx::bulk_g2s(st + lane * kTileBytes, a.tiles + basis * a.basis_bytes + ((row_tile0(rs) + lane) * k_tiles + kt) * kTileBytes, kTileBytes,
                                       &full[slot]);
                 }
                 // (a pair's second half may lie behind the last token block: it reads that block again, nothing of it is stored)
@@ -204,16 +208,18 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             };
             int g = 0;
             for (int tile = cid; tile < n_tiles && g < kStages; tile += n_clusters)
-                for (int kt = kt0; kt < kt1 && g < kStages; ++kt, ++g) issue(tile, kt, g, true, false);
+                for (int basis = 0; basis < bases; ++basis)
+                    for (int kt = kt0; kt < kt1 && g < kStages; ++kt, ++g) issue(tile, basis, kt, g, true, false);
             if constexpr (PAIR) { __syncwarp(); ptx::cluster_wait(); }
             ptx::pdl_wait();
             g = 0;
-            for (int tile = cid; tile < n_tiles; tile += n_clusters) {
+            for (int tile = cid; tile < n_tiles; tile += n_clusters)
+            for (int basis = 0; basis < bases; ++basis) {
                 for (int kt = kt0; kt < kt1; ++kt, ++g) {
                     const int slot = g % kStages, use = g / kStages;
-                    if (use == 0) { issue(tile, kt, slot, false, true); continue; }
+                    if (use == 0) { issue(tile, basis, kt, slot, false, true); continue; }
                     ok &= ptx::mbar_wait_bounded(&empty[slot], (uint32_t)((use - 1) & 1));
-                    issue(tile, kt, slot, true, true);
+                    issue(tile, basis, kt, slot, true, true);
                 }
             }
         }
@@ -230,7 +236,8 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                 else ptx::umma_commit(bar);
             };
             int g = 0, tl = 0;
-            for (int tile = cid; tile < n_tiles; tile += n_clusters, ++tl) {
+            for (int tile = cid; tile < n_tiles; tile += n_clusters)
+            for (int basis = 0; basis < bases; ++basis, ++tl) {
                 const int sel = tl % kAccSets, acc_use = tl / kAccSets;
                 if (acc_use > 0) ok &= ptx::mbar_wait_bounded(&acc_empty[sel], (uint32_t)((acc_use - 1) & 1));
                 ptx::tc_fence_after();
@@ -296,7 +303,8 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             }
             pending = -1;
         };
-        for (int tile = cid; tile < n_tiles; tile += n_clusters) {
+        for (int tile = cid; tile < n_tiles; tile += n_clusters)
+        for (int basis = 0; basis < bases; ++basis) {
             const int rs = tile % row_sets;
             const int rts = row_tiles_of(rs);
             for (int kt = kt0; kt < kt1; ++kt, ++g) {
@@ -351,11 +359,18 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         // The epilogue kind is a compile-time constant of everything below (one copy of the role per kind, chosen once):
         // the unrolled store sequences are long, and a kind switch inside every element made them four times as long -
         // code that is fetched once per tile and does not stay in the instruction cache.
-        auto epilogue_role = [&](auto kind) {
+        // MULTI: several bases, added up in basis order in f32 rows (the output, or aside before a bf16 output); the thread that
+        // adds a basis is the one that stored the one before.
+        auto epilogue_role = [&](auto kind, auto multi) {
         constexpr int EPI = decltype(kind)::value;
-        constexpr bool accum = EPI == EPI_F32_ACCUM || EPI == kEpiBf16Accum;
+        constexpr bool MULTI = decltype(multi)::value;
+        constexpr bool accum = MULTI || EPI == EPI_F32_ACCUM || EPI == kEpiBf16Accum;
+        int basis = 0;
         auto load_old = [&](int token, int64_t row) -> float {
-            return (accum && token < a.m && row < a.n_out) ? a.acc_in[(int64_t)token * a.out_stride + row] : 0.0f;
+            const int64_t o = (int64_t)token * a.out_stride + row;
+            if (!accum || token >= a.m || row >= a.n_out) return 0.0f;
+            if constexpr (MULTI) return basis == 0 ? 0.0f : (EPI == EPI_BF16 ? a.sum[o] : reinterpret_cast<const float*>(a.out)[o]);
+            else return a.acc_in[o];
         };
         // i = token inside the tile; tq / ts = the tile's staged per-token terms
         // tqi / tsi: the token's sum of q and scale (read from shared memory by the caller, ahead of its stores)
@@ -368,7 +383,12 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                     reinterpret_cast<int32_t*>(a.out)[o] = accv;
                 } else {
                     const float y = __fmul_rn(__fmul_rn((float)accv, sw), tsi);
-                    if constexpr (EPI == EPI_F32) reinterpret_cast<float*>(a.out)[o] = y;
+                    if constexpr (MULTI) {
+                        const float v = basis == 0 ? y : __fadd_rn(old, y);
+                        if (EPI == EPI_F32) reinterpret_cast<float*>(a.out)[o] = v;
+                        else if (basis + 1 < a.bases) a.sum[o] = v;
+                        else reinterpret_cast<__nv_bfloat16*>(a.out)[o] = __float2bfloat16_rn(v);
+                    } else if constexpr (EPI == EPI_F32) reinterpret_cast<float*>(a.out)[o] = y;
                     else if constexpr (EPI == EPI_F32_ACCUM) reinterpret_cast<float*>(a.out)[o] = __fadd_rn(old, y);
                     else if constexpr (EPI == kEpiBf16Accum) reinterpret_cast<__nv_bfloat16*>(a.out)[o] = __float2bfloat16_rn(__fadd_rn(old, y));
                     else reinterpret_cast<__nv_bfloat16*>(a.out)[o] = __float2bfloat16_rn(y);
@@ -384,7 +404,8 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             else ptx::mbar_arrive(&acc_empty[sel]);
         };
         int tl = 0;
-        for (int tile = cid; tile < n_tiles; tile += n_clusters, ++tl) {
+        for (int tile = cid; tile < n_tiles; tile += n_clusters)
+        for (basis = 0; basis < (MULTI ? a.bases : 1); ++basis, ++tl) {
             const int rs = tile % row_sets, tb = tile / row_sets;
             const int sel = tl % kAccSets;
             // the tile's per-token terms, once per row set's four warps into shared memory (named barrier 1 + h)
@@ -409,7 +430,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             const int64_t row = PAIR ? ((int64_t)rs * 2 + rank) * kRows + lrow : ((int64_t)rs * RS + h) * kRows + lrow;
             const int64_t rt = row >> 4;
             float sw = 0.f;
-            if (EPI != EPI_I32 && rt < a.row_tiles) sw = __ldg(a.sw_tiles + 2 * rt + ((row >> 3) & 1));
+            if (EPI != EPI_I32 && rt < a.row_tiles) sw = __ldg(a.sw_tiles + 2 * (basis * a.row_tiles + rt) + ((row >> 3) & 1));
             const uint32_t acc_addr = tmem_base + ((uint32_t)(sub * 32) << 16) + (uint32_t)(sel * RS + h) * NT;
             const int n_tok = min(NT, a.m - tok0);  // tokens of these that exist
             bool drained = false;
@@ -555,12 +576,22 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             }
         }
         };
-        switch (a.epilogue) {
-            case EPI_I32: epilogue_role(std::integral_constant<int, EPI_I32>{}); break;
-            case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}); break;
-            case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}); break;
-            case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}); break;
-            default: epilogue_role(std::integral_constant<int, EPI_BF16>{}); break;
+        constexpr std::false_type one{};
+        if constexpr (NT == 64) {
+            constexpr std::true_type several{};
+            if (a.bases > 1) {
+                if (a.epilogue == EPI_F32) epilogue_role(std::integral_constant<int, EPI_F32>{}, several);
+                else epilogue_role(std::integral_constant<int, EPI_BF16>{}, several);
+            }
+        }
+        if (bases == 1) {
+            switch (a.epilogue) {
+                case EPI_I32: epilogue_role(std::integral_constant<int, EPI_I32>{}, one); break;
+                case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}, one); break;
+                case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}, one); break;
+                case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}, one); break;
+                default: epilogue_role(std::integral_constant<int, EPI_BF16>{}, one); break;
+            }
         }
     }
     if (!ok) atomicExch(a.err, kErrTcTimeout);
@@ -578,7 +609,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         // Nobody leaves while a peer may still read its shared memory or arrive on its barriers: the last of both is
         // the peers' arrival on red_free for this CTA's last tile (they read the parked sums before it, and arrived on
         // red_full before that).  One warp waits for it; the CTA lives as long as that warp.
-        const int my_tiles = cid < n_tiles ? (n_tiles - cid + n_clusters - 1) / n_clusters : 0;
+        const int my_tiles = cid < n_tiles ? (n_tiles - cid + n_clusters - 1) / n_clusters * bases : 0;
         if (warp == 2 && my_tiles > 0 && !ptx::mbar_wait_cluster_bounded(red_free, (uint32_t)((my_tiles - 1) & 1)))
             atomicExch(a.err, kErrTcTimeout);
     }
@@ -708,8 +739,8 @@ cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) 
 }  // namespace
 
 int gemm_tc_kernels(const LinearDev& lin, int64_t m, int sm_count) {
-    (void)m; (void)sm_count;
-    return lin.w.n_bases;  // one launch per basis; a k split is reduced inside the launch
+    (void)sm_count;
+    return m <= 64 ? 1 : lin.w.n_bases;  // above 64 tokens one launch per basis; a k split is reduced inside the launch
 }
 
 size_t gemm_tc_act_bytes(int64_t m, int64_t k_tiles) {
@@ -736,8 +767,14 @@ cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride
                              nullptr, stream, qtc, kts);
     }
     if (e != cudaSuccess) return e;
-    for (int b = 0; b < lin.w.n_bases; ++b) {
+    // Up to 64 tokens the bases of a product are one launch: three launches in turn took 9 us each for 16 x 4096 -> 4096, of
+    // which most is start-up and drain; the call 28.7 -> 18.5 us.  (Larger products fill the GPU one by one.)
+    const bool together = nt == 64 && lin.w.n_bases > 1 && (epilogue == EPI_F32 || epilogue == EPI_BF16);
+    for (int b = 0; b < (together ? 1 : lin.w.n_bases); ++b) {
         TcArgs a = {};
+        a.bases = together ? lin.w.n_bases : 1;
+        a.basis_bytes = lin.w.basis_stride();
+        a.sum = sum;
         a.tiles = lin.w.tiles + (size_t)b * lin.w.basis_stride();
         a.row_tiles = lin.w.row_tiles;
         a.k_tiles = lin.w.k_tiles;
@@ -749,7 +786,7 @@ cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride
         a.m = (int)m;
         // Several bases: the first stores, the others add to it, in basis order.  With a bf16 output all but the last work
         // on f32 rows aside, and the last one rounds the whole sum.
-        const bool aside = lin.w.n_bases > 1 && epilogue == EPI_BF16, last = b + 1 == lin.w.n_bases;
+        const bool aside = !together && lin.w.n_bases > 1 && epilogue == EPI_BF16, last = b + 1 == lin.w.n_bases;
         a.out = aside && !last ? (void*)sum : out;
         a.out_stride = out_stride;
         a.epilogue = aside ? (last ? kEpiBf16Accum : (b > 0 ? EPI_F32_ACCUM : EPI_F32)) : ((b > 0 && epilogue == EPI_F32) ? EPI_F32_ACCUM : epilogue);

@@ -222,3 +222,24 @@ def test_tensor_core_path_cta_pairs(bt, oracle, m, n, k, dtype, bases):
     ref = torch.from_numpy(oracle.bitlinear_q(x.float().numpy(), packed, scales, n, bases)).to(x.dtype)
     assert torch.equal(y, ref)
     assert bt.lib().bt_device_check(0) == 0
+
+
+
+
+@pytest.mark.parametrize("m,n,k,bases", [
+    (9, 128, 256, 2), (40, 300, 516, 8),                     # one row tile; eight bases, rows that fill no tile
+    (16, 4096, 4096, 3), (33, 1000, 8192, 3), (64, 600, 2048, 2),  # inputs cut over clusters
+    (64, 19100, 260, 2)])                                    # more row tiles than SMs
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_bases_in_one_launch(bt, oracle, m, n, k, bases, dtype):
+    # 9 to 64 tokens: the bases of a projection are worked through in one launch and added up in basis order
+    rng = np.random.default_rng(m + n)
+    packed = np.stack([ternary_packed(rng, n, k) for _ in range(bases)], -1)
+    scales = np.array([0.5 / 3 ** b for b in range(bases)], np.float32)
+    x = torch.from_numpy(rng.normal(0, 1, (m, k)).astype(np.float32)).to(getattr(torch, dtype))
+    lin = bt.BitLinear.from_packed(packed, scales, n, k)
+    ref = torch.from_numpy(oracle.bitlinear_q(x.float().numpy(), packed, scales, n, bases)).to(x.dtype)
+    for _ in range(2):  # (the second time over an output that is not zero)
+        y = lin.forward(x.cuda()).cpu()
+        assert torch.equal(y, ref)
+    assert bt.lib().bt_device_check(0) == 0
