@@ -398,6 +398,14 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         auto store = [&](const int* tq, const float* ts, int tok0, int i, int n_tok, int64_t row, float sw, uint32_t acc, float old) {
             store_v(tq[i], ts[i], tok0, i, n_tok, row, sw, acc, old);
         };
+        // EPI_SWIGLU: rows 0-7 of a row tile are gate rows, rows 8-15 the matching up rows, eight lanes further on.  Of `half` + half
+        // tokens in a lane's registers the gate lane finishes the first half and the up lane the second, so that both compute:
+        // each sends what the other needs.  f32 as in the quantiser that did this before (silu(g) * u, layers/swiglu.rs:31-33).
+        auto swiglu = [&](uint32_t mine, uint32_t other, int tqi, float tsi, float sw_gate, float sw_up, bool up) -> float {
+            const float g = __fmul_rn(__fmul_rn((float)((int)(up ? other : mine) - tqi), sw_gate), tsi);
+            const float u = __fmul_rn(__fmul_rn((float)((int)(up ? mine : other) - tqi), sw_up), tsi);
+            return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
+        };
         // a set of accumulator columns has been read: the MMA issuer may write it again
         auto free_set = [&](int sel) {
             if constexpr (PAIR) ptx::mbar_arrive_remote(ptx::map_to_rank(&acc_empty[sel], 0));
@@ -452,6 +460,18 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                     if (lane == 0) free_set(sel);
                     using Out = std::conditional_t<EPI == EPI_BF16 || EPI == kEpiBf16Accum, __nv_bfloat16, float>;
                     const int64_t stride = a.out_stride, at = (int64_t)tok0 * stride + row;
+                    if constexpr (EPI == EPI_SWIGLU) {
+                        const bool up = lane & 8;
+                        const float sw_other = __shfl_xor_sync(0xffffffffu, sw, 8), sw_gate = up ? sw_other : sw, sw_up = up ? sw : sw_other;
+                        const int *tqh = tq + (up ? NT / 2 : 0);
+                        const float *tsh = ts + (up ? NT / 2 : 0);
+                        float* po = reinterpret_cast<float*>(a.out) + (int64_t)(tok0 + (up ? NT / 2 : 0)) * stride + (row >> 4) * 8 + (row & 7);
+#pragma unroll
+                        for (int i = 0; i < NT / 2; ++i) {
+                            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? d[i] : d[NT / 2 + i], 8);
+                            po[i * stride] = swiglu(up ? d[NT / 2 + i] : d[i], got, tqh[i], tsh[i], sw_gate, sw_up, up);
+                        }
+                    } else {
                     Out* po = reinterpret_cast<Out*>(a.out) + at;
                     auto put = [&](int i, float y) {
                         if constexpr (std::is_same_v<Out, float>) po[i * stride] = y;
@@ -472,12 +492,31 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
 #pragma unroll
                         for (int i = 0; i < NT; ++i) put(i, __fmul_rn(__fmul_rn((float)((int)d[i] - tq[i]), sw), ts[i]));
                     }
+                    }
                 }
             }
             if (drained) {
                 // nothing left to do for this tile
             } else if constexpr (S == 1) {
-                if (accum) {
+                if constexpr (EPI == EPI_SWIGLU) {
+                    const bool up = lane & 8;
+                    const float sw_other = __shfl_xor_sync(0xffffffffu, sw, 8), sw_gate = up ? sw_other : sw, sw_up = up ? sw : sw_other;
+                    const int64_t col = (row >> 4) * 8 + (row & 7);
+#pragma unroll 1
+                    for (int c0 = 0; c0 < NT; c0 += 32) {
+                        uint32_t d[32];
+                        ptx::tmem_ld32(acc_addr + c0, d);
+                        ptx::tmem_ld_wait();
+                        const int i0 = c0 + (up ? 16 : 0);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? d[j] : d[16 + j], 8);
+                            if (i0 + j < n_tok && row < a.n_out)
+                                reinterpret_cast<float*>(a.out)[(int64_t)(tok0 + i0 + j) * a.out_stride + col] = swiglu(up ? d[16 + j] : d[j], got, tq[i0 + j], ts[i0 + j], sw_gate, sw_up, up);
+                        }
+                        __syncwarp();
+                    }
+                } else if (accum) {
 #pragma unroll 1
                     for (int c0 = 0; c0 < NT; c0 += 16) {
                         uint32_t d[16];
@@ -590,6 +629,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                 case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}, one); break;
                 case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}, one); break;
                 case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}, one); break;
+                case EPI_SWIGLU: if constexpr (NT == 128) epilogue_role(std::integral_constant<int, EPI_SWIGLU>{}, one); break;
                 default: epilogue_role(std::integral_constant<int, EPI_BF16>{}, one); break;
             }
         }
@@ -705,12 +745,13 @@ cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) 
     if (nt == 128) {
         // Pairs where there are tiles for most SMs and no more rounds of them than of single CTAs' tiles, which are half as large
         // (257 x 4096 -> 28672 has one more: 59.7 -> 68.7 us).  More than 16384 rows of plain output stay with single CTAs: their
-        // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240).
+        // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240);
+        // with SiLU * up, which stores half of that, pairs are ahead again (prefill of 2048 tokens, 8B: 3 242 us and 3 290).
         const TcVariant& pair = tc_variant<128, 1, 1, true>(sm_count);
         const int n_pairs = (int)((a.row_tiles + 15) / 16) * ((a.m + kPairTokens - 1) / kPairTokens);
         // 256-row tiles halve the activation traffic per weight; 128-row tiles when there is too little work for them
         const int waves2 = (n_tiles2 + sm_count - 1) / sm_count;
-        if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && a.row_tiles <= 1024 &&
+        if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && (a.row_tiles <= 1024 || a.epilogue == EPI_SWIGLU) &&
             (n_pairs + pair.max_clusters - 1) / pair.max_clusters <= waves2)
             return launch_variant<128, 1, 1, true>(a, sm_count, stream);
         return 2 * n_tiles2 >= sm_count ? launch_variant<128, 2, 1>(a, sm_count, stream) : launch_variant<128, 1, 1>(a, sm_count, stream);
@@ -748,13 +789,19 @@ size_t gemm_tc_act_bytes(int64_t m, int64_t k_tiles) {
     return (size_t)((m + nt - 1) / nt * k_tiles * 4 * nt * 64);
 }
 
+// More than 64 tokens, where tiles follow one another and the exponentials of one are worked out under the MMAs of the next (2048 x
+// 4096 -> 28672 with the quantiser behind it, 32 layers: 3 428 -> 3 274 us a prefill).  With fewer a CTA has one tile, and its eight
+// epilogue warps are the last thing the launch waits for: the decode step of 64 sequences became slower, and keeps the quantiser's.
+bool gemm_tc_swiglu(const LinearDev& lin, int64_t m) { return m > 64 && lin.w.n_bases == 1 && lin.w.n_out % kTileRows == 0; }
+
 cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride, int64_t m, int8_t* qtc, float* sx,
                            int32_t* qsum, void* out, int64_t out_stride, int epilogue, unsigned int* err, int sm_count,
                            cudaStream_t stream, bool prequantised, bt_dtype x_dtype, float* sum) {
     if (lin.w.n_bases != 1 && epilogue == EPI_BF16 && !sum) return cudaErrorInvalidValue;
-    if (epilogue != EPI_I32 && epilogue != EPI_F32 && epilogue != EPI_F32_ACCUM && epilogue != EPI_BF16)
-        return cudaErrorInvalidValue;  // (the SiLU*up epilogue exists in the streaming kernel only)
     const int nt = m <= 64 ? 64 : 128;
+    if (epilogue != EPI_I32 && epilogue != EPI_F32 && epilogue != EPI_F32_ACCUM && epilogue != EPI_BF16 &&
+        !(epilogue == EPI_SWIGLU && gemm_tc_swiglu(lin, m)))
+        return cudaErrorInvalidValue;
     const int k = (int)lin.w.k_in, kts = (int)lin.w.k_tiles;
     cudaError_t e = cudaSuccess;
     if (prequantised) {

@@ -911,10 +911,18 @@ bt_status enqueue_prefill_chunk(bt_model* m, int batch, int n, int past, int ttt
         }
         BT_CUDA_TRY(trace_copy(m, li, TR_H_MID, m->pf_h, M, s));
         BT_CUDA_TRY(launch_row_quant(PRE_RMSNORM, m->pf_h, H, L.norm2, kRmsEps, M, H, nullptr, 0, m->pf_sx, m->pf_qsum, nullptr, s, m->pf_qtc, kt_h));
-        BT_CUDA_TRY(launch_gemm_tc(L.gate_up_il->dev(), nullptr, H, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_gu, 2 * I, EPI_F32, err, sm, s, true));
-        BT_CUDA_TRY(launch_row_quant(PRE_SWIGLU, m->pf_gu, 2 * I, nullptr, 0.f, M, I, nullptr, 0, m->pf_sx, m->pf_qsum,
-                                     m->trace ? m->pf_act : nullptr, s, m->pf_qtc, kt_i));
-        if (m->trace) BT_CUDA_TRY(trace_copy(m, li, TR_ACT, m->pf_act, M, s));
+        if (gemm_tc_swiglu(L.gate_up_il->dev(), M)) {
+            // silu(gate) * up in the product's epilogue, under the next tile's MMAs: half the output bytes, and a quantiser without the
+            // exponential
+            BT_CUDA_TRY(launch_gemm_tc(L.gate_up_il->dev(), nullptr, H, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_gu, I, EPI_SWIGLU, err, sm, s, true));
+            BT_CUDA_TRY(launch_row_quant(PRE_NONE, m->pf_gu, I, nullptr, 0.f, M, I, nullptr, 0, m->pf_sx, m->pf_qsum, nullptr, s, m->pf_qtc, kt_i));
+            BT_CUDA_TRY(trace_copy(m, li, TR_ACT, m->pf_gu, M, s));
+        } else {
+            BT_CUDA_TRY(launch_gemm_tc(L.gate_up_il->dev(), nullptr, H, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_gu, 2 * I, EPI_F32, err, sm, s, true));
+            BT_CUDA_TRY(launch_row_quant(PRE_SWIGLU, m->pf_gu, 2 * I, nullptr, 0.f, M, I, nullptr, 0, m->pf_sx, m->pf_qsum,
+                                         m->trace ? m->pf_act : nullptr, s, m->pf_qtc, kt_i));
+            if (m->trace) BT_CUDA_TRY(trace_copy(m, li, TR_ACT, m->pf_act, M, s));
+        }
         if (m->multi_basis) {
             BT_CUDA_TRY(launch_gemm_tc(L.down->dev(), nullptr, I, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_att, H, EPI_F32, err, sm, s, true));
             BT_CUDA_TRY(launch_residual_add(m->pf_h, m->pf_att, (int64_t)M * H, s));

@@ -289,3 +289,15 @@ def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, pa
         assert np.isfinite(want).all()
         assert (np.linalg.norm(got - want, axis=-1) <= 16 * 2.0 ** -22 * np.linalg.norm(want, axis=-1)).all(), (kind, i)
     assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("hidden,ff,batch,n", [(256, 176, 1, 65), (256, 1040, 1, 129), (1024, 4112, 3, 90), (512, 5008, 5, 199)])
+def test_prefill_silu_in_the_product(bt, oracle, syn, hidden, ff, batch, n):
+    # more than 64 rows: silu(gate) * up leaves the gate|up product itself; few row tiles, row tiles that end inside a set of
+    # 128, tiles without some of their tokens, CTA pairs (the last)
+    cfg = syn.BitLlamaConfig("llama", 64, hidden, 1, hidden // 64, hidden // 128, ff, max_position_embeddings=256)
+    w = syn.make_weights(cfg, seed=ff, from_latent=False)
+    gpu, ref = syn.build_model(w, max_batch=batch), oracle.model_from_weights(w)
+    states = [ref.new_state() for _ in range(batch)]
+    staged_prefill(oracle, ref, gpu, cfg, np.random.default_rng(n).integers(0, 64, size=(batch, n)), states)
+    assert bt.lib().bt_device_check(0) == 0
