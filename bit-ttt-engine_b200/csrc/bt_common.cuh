@@ -101,6 +101,7 @@ enum Prologue : int {
     PRO_Q8 = 0,       // already quantised in global memory (q, qsum, sx)
     PRO_RMSNORM = 1,  // x f32 -> RMSNorm with norm_w -> per-token absmax quantisation, in the kernel
     PRO_ABSMAX = 2,   // x f32 with its per-token max|x| already known (absmax_in) -> quantisation
+    PRO_ROW = 3,      // x f32 or bf16 -> per-token absmax quantisation, in the kernel
 };
 
 // Ternary product for up to 8 tokens per launch.
@@ -113,7 +114,8 @@ struct GemvArgs {
     int64_t q_stride;
     const int32_t* qsum;    // PRO_Q8: [m]
     const float* sx;        // PRO_Q8: [m] (unused for EPI_I32)
-    const float* x;         // PRO_RMSNORM / PRO_ABSMAX: [m, x_stride] f32
+    const float* x;         // PRO_RMSNORM / PRO_ABSMAX / PRO_ROW: [m, x_stride] f32
+    bool x_bf16;            // PRO_ROW: bf16 instead
     int64_t x_stride;
     const float* norm_w;    // PRO_RMSNORM: [k_in]
     float eps;
@@ -150,13 +152,16 @@ cudaError_t linear_product(const LinearDev& lin, const int8_t* q, int64_t q_stri
 
 // Single-basis product for m <= 8 tokens whose quantisation happens inside the kernel.
 struct FusedIn {
-    int prologue;                   // PRO_RMSNORM or PRO_ABSMAX
+    int prologue;                   // PRO_RMSNORM, PRO_ABSMAX or PRO_ROW
     const float* x;
     int64_t x_stride;
     const float* norm_w;
     float eps;
     const unsigned int* absmax_in;
+    bool x_bf16 = false;            // PRO_ROW
 };
+// Whether PRO_ROW takes rows of this many inputs from this address.
+bool gemv_takes_rows(const void* x, int64_t k_in);
 cudaError_t linear_product_fused(const LinearDev& lin, const FusedIn& in, int m, void* out,
                                  int64_t out_stride, int epilogue, unsigned int* absmax_out,
                                  unsigned int* err, int sm_count, cudaStream_t stream);

@@ -139,6 +139,19 @@ __device__ __forceinline__ int quant_store_half(const float (&v)[8], float inv, 
     return sum;
 }
 
+// The definition of the quantiser to the letter (act_quant.cu), values that are no numbers included: they become -127, and so
+// do products with an infinite 127 / max|x| that are none.
+__device__ __forceinline__ float clamp127(float v) { return fminf(fmaxf(v, -127.0f), 127.0f); }
+
+__device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&v)[16]) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const uint4 u = *reinterpret_cast<const uint4*>(p + 8 * b);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { v[8 * b + 2 * i] = __uint_as_float(w[i] << 16); v[8 * b + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    }
+}
 __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
@@ -254,6 +267,39 @@ __device__ __forceinline__ void stage_activations(const GemvArgs& a, uint8_t* ac
             if (h0) local += quant_store_group(v0, inv, dst, j0);
             if (h1) local += quant_store_group(v1, inv, dst, j1);
             for (int j = groups + tid; j < groups_pad; j += kMathThreads) {
+                const float z[16] = {0};
+                quant_store_group(z, 0.0f, dst, j);
+            }
+        } else if (PRO == PRO_ROW) {
+            // up to two 16-groups per thread held in registers (k_in <= 16384); zeros behind the row
+            float v0[16], v1[16];
+            const int j0 = tid, j1 = tid + kMathThreads;
+            const bool h0 = j0 < groups, h1 = j1 < groups;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v0[e] = v1[e] = 0.0f;
+            if (a.x_bf16) {
+                const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(a.x) + (int64_t)n * a.x_stride;
+                if (h0) load16(xb + 16 * j0, v0);
+                if (h1) load16(xb + 16 * j1, v1);
+            } else {
+                if (h0) load16(xr + 16 * j0, v0);
+                if (h1) load16(xr + 16 * j1, v1);
+            }
+            if (n == 0) loads_issued();
+            float amax = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fmaxf(fabsf(v0[e]), fabsf(v1[e])));
+            amax = math_max_f(amax, sl_f + (n & 1) * kMathWarps, warp, lane);  // (two places: one barrier a token)
+            s = __fdiv_rn(amax, 127.0f);
+            const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                v0[e] = amax > 0.0f && h0 ? clamp127(__fmul_rn(v0[e], inv)) : 0.0f;
+                v1[e] = amax > 0.0f && h1 ? clamp127(__fmul_rn(v1[e], inv)) : 0.0f;
+            }
+            if (j0 < groups_pad) local += quant_store_group(v0, 1.0f, dst, j0);
+            if (j1 < groups_pad) local += quant_store_group(v1, 1.0f, dst, j1);
+            for (int j = j1 + kMathThreads; j < groups_pad; j += kMathThreads) {
                 const float z[16] = {0};
                 quant_store_group(z, 0.0f, dst, j);
             }
@@ -729,6 +775,7 @@ template <int TPW>
 static cudaError_t launch_gemv_t(const GemvArgs& a, int grid, size_t smem, int nstages, int act_stride, cudaStream_t stream) {
     switch (a.prologue) {
         case PRO_RMSNORM: return launch_pdl(gemv_kernel<PRO_RMSNORM, TPW>, dim3(grid), dim3(kThreads), smem, stream, a.pdl, a, nstages, act_stride);
+        case PRO_ROW: return launch_pdl(gemv_kernel<PRO_ROW, TPW>, dim3(grid), dim3(kThreads), smem, stream, a.pdl, a, nstages, act_stride);
         case PRO_ABSMAX: return launch_pdl(gemv_kernel<PRO_ABSMAX, TPW>, dim3(grid), dim3(kThreads), smem, stream, a.pdl, a, nstages, act_stride);
         default: return launch_pdl(gemv_kernel<PRO_Q8, TPW>, dim3(grid), dim3(kThreads), smem, stream, a.pdl, a, nstages, act_stride);
     }
@@ -738,6 +785,7 @@ cudaError_t launch_gemv(const GemvArgs& a, int sm_count, cudaStream_t stream) {
     if (a.m < 1 || a.m > 8) return cudaErrorInvalidValue;
     if (a.prologue != PRO_Q8 && (a.k_in % 16 != 0)) return cudaErrorInvalidValue;
     if (a.prologue == PRO_RMSNORM && a.k_in > 16 * 2 * kMathThreads) return cudaErrorInvalidValue;
+    if (a.prologue == PRO_ROW && !gemv_takes_rows(a.x, a.k_in)) return cudaErrorInvalidValue;
     if (a.epilogue == EPI_SWIGLU && (!a.absmax_out || a.n_out % 16 != 0)) return cudaErrorInvalidValue;
     const int act_stride = (int)(a.k_tiles * kTileK + 64);
     const size_t fixed = gemv_fixed_smem(a.m, a.k_tiles);
@@ -772,6 +820,8 @@ cudaError_t launch_gemv(const GemvArgs& a, int sm_count, cudaStream_t stream) {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<PRO_Q8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<PRO_RMSNORM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<PRO_ABSMAX, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<PRO_ROW, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<PRO_ROW, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
             if (e != cudaSuccess) return e;
             g_configured[dev] = 1;
         }
@@ -861,6 +911,7 @@ cudaError_t linear_product_fused(const LinearDev& lin, const FusedIn& in, int m,
     a.norm_w = in.norm_w;
     a.eps = in.eps;
     a.absmax_in = in.absmax_in;
+    a.x_bf16 = in.x_bf16;
     a.absmax_out = absmax_out;
     a.sw_tiles = lin.scale_tiles;
     a.m = m;
@@ -870,6 +921,11 @@ cudaError_t linear_product_fused(const LinearDev& lin, const FusedIn& in, int m,
     a.err = err;
     a.pdl = true;
     return launch_gemv(a, sm_count, stream);
+}
+
+// (Rows of a multiple of 16 values start on 16-byte boundaries in either type.)
+bool gemv_takes_rows(const void* x, int64_t k_in) {
+    return k_in % 16 == 0 && k_in <= 16 * 2 * kMathThreads && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 }
 
 }  // namespace bt

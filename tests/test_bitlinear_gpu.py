@@ -243,3 +243,29 @@ def test_bases_in_one_launch(bt, oracle, m, n, k, bases, dtype):
         y = lin.forward(x.cuda()).cpu()
         assert torch.equal(y, ref)
     assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("k", [16, 272, 8192, 16384, 16400, 516])  # the last two stay with the quantiser kernel
+@pytest.mark.parametrize("m", [1, 2, 3, 4])  # the last count too
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_rows_quantised_in_the_product(bt, oracle, m, k, dtype):
+    n = 100
+    rng = np.random.default_rng(m * k)
+    packed = ternary_packed(rng, n, k)
+    x = rng.normal(0, 1, (m, k)).astype(np.float32)
+    x[0, :5] = [127, 0.5, -0.5, 126.5, -1.5]
+    if m > 1:
+        x[1] = 0
+    if m > 2:
+        x[2] *= 1e-39  # 127 / max|x| overflows: every value saturates
+    x = torch.from_numpy(x).to(getattr(torch, dtype))
+    lin = bt.BitLinear.from_packed(packed, [0.5], n, k)
+    ref = torch.from_numpy(oracle.bitlinear_q(x.float().numpy(), packed, [0.5], n)).to(x.dtype)
+    assert torch.equal(lin.forward(x.cuda()).cpu(), ref)
+    apart = torch.empty(m * k + 1, dtype=x.dtype, device="cuda")[1:].view(m, k).copy_(x)  # rows that start on no 16-byte boundary
+    assert torch.equal(lin.forward(apart).cpu(), ref)
+    # values that are no numbers, as the quantiser kernel has them (more tokens than the product quantises itself)
+    x[0, 3], x[0, k // 2] = float("nan"), float("inf")
+    many = x[:1].expand(4, k).contiguous().cuda()
+    assert torch.equal(lin.forward(x[:1].cuda()).nan_to_num(7.0), lin.forward(many)[:1].nan_to_num(7.0))
+    assert bt.lib().bt_device_check(0) == 0
