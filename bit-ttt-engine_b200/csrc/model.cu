@@ -809,7 +809,11 @@ extern "C" bt_status bt_model_forward_one(bt_model* m, const int32_t* tokens_hos
 
 namespace {
 
-constexpr int kPrefillRowsMax = 2048;  // rows (sequences x tokens) one prefill chunk works on
+// Rows (sequences x tokens) that one prefill pass works on.  Ternary models: with 2048 rows the products of a 2048-wide model have
+// 64 to 160 tiles for 74 CTA pairs, and every pass ends in a wait of the host (16 prompts of 511 tokens, 1B: 5 156 us in passes
+// of 2048, 3 874 in one).  Layer-list models keep more buffers a row, and a ternary model without the memory for 8192 (1.5 GB
+// at 4096 x 14336) works on 2048 as well.
+constexpr int kPrefillRows = 8192, kPrefillRowsLeast = 2048;
 
 bt_status prefill_buffers(bt_model* m, int rows) {
     if (m->lay) return layered_prefill_buffers(m, rows);
@@ -818,8 +822,9 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     const int64_t H = c.hidden_dim, I = m->i_l;
     const int64_t qw = c.arch == 1 ? m->qkv_dim : m->d_small;  // q|k|v, or the TTT features and predictions (two slots)
     BT_CUDA_TRY(cudaDeviceSynchronize());
-    for (void* p : {(void*)m->pf_tokens, (void*)m->pf_h, (void*)m->pf_qkv, (void*)m->pf_att, (void*)m->pf_gu, (void*)m->pf_qtc,
-                    (void*)m->pf_sx, (void*)m->pf_qsum, (void*)m->pf_qs}) cudaFree(p);
+    auto drop = [](auto*& p) { cudaFree(p); p = nullptr; };
+    drop(m->pf_tokens); drop(m->pf_h); drop(m->pf_qkv); drop(m->pf_att); drop(m->pf_gu); drop(m->pf_qtc);
+    drop(m->pf_sx); drop(m->pf_qsum); drop(m->pf_qs);
     m->pf_rows = 0;
     const int64_t kmax = H > I ? H : I;
     BT_CUDA_TRY(dev_alloc(&m->pf_tokens, (size_t)rows));
@@ -956,13 +961,22 @@ bt_status prefill_impl(bt_model* m, const int32_t* tokens_host, int batch, int n
     DeviceGuard guard(m->device);
     cudaStream_t s = m->stream;
     // tokens per sequence and chunk: as many as keep sequences x tokens within the scratch (a TTT chunk is never cut)
-    int per = kPrefillRowsMax / batch;
-    if (per < 1) per = 1;
-    if (per > n_tokens) per = n_tokens;
-    if (c.arch == 0 && per < n_tokens && per > ttt_chunk) per -= per % ttt_chunk;
-    if (m->trace && (int64_t)batch * per > m->trace_rows) per = m->trace_rows / batch;
+    int per = 0;
+    auto cut = [&](int rows) {
+        per = rows / batch;
+        if (per < 1) per = 1;
+        if (per > n_tokens) per = n_tokens;
+        if (c.arch == 0 && per < n_tokens && per > ttt_chunk) per -= per % ttt_chunk;
+        if (m->trace && (int64_t)batch * per > m->trace_rows) per = m->trace_rows / batch;
+    };
+    cut(m->lay ? kPrefillRowsLeast : kPrefillRows);
     if (per < 1) return set_error(BT_ERR_NOMEM, "bt_model_prefill: the trace buffer holds fewer rows than sequences");
     bt_status st = prefill_buffers(m, batch * per);
+    if (st != BT_OK && batch * per > kPrefillRowsLeast) {
+        cudaGetLastError();  // (an allocation that failed leaves the context as it was)
+        cut(kPrefillRowsLeast);
+        st = prefill_buffers(m, batch * per);
+    }
     if (st != BT_OK) return st;
     if (m->trace && !m->lay && m->pf_act_rows < batch * per) {
         BT_CUDA_TRY(cudaDeviceSynchronize());
