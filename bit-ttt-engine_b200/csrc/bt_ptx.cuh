@@ -175,12 +175,10 @@ __device__ __forceinline__ uint32_t pack4_sat_s8(int q0, int q1, int q2, int q3)
 }
 
 // round(v) with halves away from zero as an int, for |v| < 2^22: equal to (int)roundf(v).
-// trunc(v + copysign(0.5, v)) is exact except when |v| < 0.5 (the sum can round up to 1),
-// which is answered directly.
+// trunc(v + copysign(0.5, v)): the sum is taken towards zero too, so that it never reaches the next integer by rounding.
 __device__ __forceinline__ int round_half_away(float v) {
     const float h = __uint_as_float((__float_as_uint(v) & 0x80000000u) | 0x3f000000u);  // copysign(0.5, v)
-    const int r = __float2int_rz(__fadd_rn(v, h));
-    return fabsf(v) < 0.5f ? 0 : r;
+    return __float2int_rz(__fadd_rz(v, h));
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {

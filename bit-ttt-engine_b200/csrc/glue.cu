@@ -285,6 +285,8 @@ __global__ void __launch_bounds__(1024) row_quant_kernel(const T* __restrict__ x
 // memory directly.
 // Per launch before -> after (us): 2048 x 4096 RMSNorm 54.8 -> 17.8, identity 27.3 -> 10.5; 2048 x 14336 SiLU 82.2 -> 70.9
 // (264 MB: 3.7 TB/s); 2001 x 14336 bf16 56.8 -> 39.7; 2044 x 2048 RMSNorm 21.1 -> 10.6; 64 x 4096 RMSNorm 4.9 -> 4.3.
+// What is left is the instructions of the rounding: integers by one addition towards zero, without clamps, and their sum by dp4a
+// took 2001 x 14336 bf16 from 41.2 to 34.9 and 2048 x 4096 RMSNorm from 17.9 to 16.4.
 template <int PRE, typename T, int V>
 __global__ void __launch_bounds__(512, V == 8 ? 2 : 3)
 row_quant_many_kernel(const T* __restrict__ x, int64_t x_stride, const float* __restrict__ w, float eps, int k,
@@ -365,6 +367,8 @@ row_quant_many_kernel(const T* __restrict__ x, int64_t x_stride, const float* __
     const float s = __fdiv_rn(amax, 127.0f);
     const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
     int local = 0;
+    // |v * inv| is 127 at most, up to two roundings, so that its integer needs no clamp; only where 127 / max|v| overflows it does
+    const bool clamp = inv > 3.0e38f;
     const int lane = tid & 31, tin = b % tc_nt;
     int8_t* blk = qtc + (int64_t)(b / tc_nt) * k_tiles * (4 * tc_nt * 64) + (lane & 3) * (tc_nt * 64) + tin * 64;
     const uint32_t turn1 = lane & 1 ? 0x3715u : 0x6240u, turn2 = lane & 2 ? 0x3276u : 0x5410u;
@@ -372,16 +376,16 @@ row_quant_many_kernel(const T* __restrict__ x, int64_t x_stride, const float* __
     for (int j = 0; j < V; ++j) {
         const int gi = tid + j * nthr;
         if (gi >= groups_pad) break;  // whole warps: groups_pad is a multiple of 64
-        int q[4] = {0, 0, 0, 0};
-        if (amax > 0.0f && gi < groups) {
-            q[0] = max(-127, min(127, ptx::round_half_away(__fmul_rn(v[j].x, inv))));
-            q[1] = max(-127, min(127, ptx::round_half_away(__fmul_rn(v[j].y, inv))));
-            q[2] = max(-127, min(127, ptx::round_half_away(__fmul_rn(v[j].z, inv))));
-            q[3] = max(-127, min(127, ptx::round_half_away(__fmul_rn(v[j].w, inv))));
+        // (zeros behind the row, and all values of a row of zeros, whose inv is 0)
+        int q[4] = {ptx::round_half_away(__fmul_rn(v[j].x, inv)), ptx::round_half_away(__fmul_rn(v[j].y, inv)),
+                    ptx::round_half_away(__fmul_rn(v[j].z, inv)), ptx::round_half_away(__fmul_rn(v[j].w, inv))};
+        if (clamp) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) q[e] = max(-127, min(127, q[e]));
         }
-        local += q[0] + q[1] + q[2] + q[3];
         // this lane has the residues 0 .. 3 of one k'; afterwards residue lane % 4 of four k'
-        const uint32_t own = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+        const uint32_t own = ptx::pack4_sat_s8(q[0], q[1], q[2], q[3]);
+        local = ptx::dp4a_s8s8(own, 0x01010101u, local);
         const uint32_t half = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), turn1);
         const uint32_t word = __byte_perm(half, __shfl_xor_sync(0xffffffffu, half, 2), turn2);
         const int kp = gi & 60;

@@ -269,3 +269,15 @@ def test_rows_quantised_in_the_product(bt, oracle, m, k, dtype):
     many = x[:1].expand(4, k).contiguous().cuda()
     assert torch.equal(lin.forward(x[:1].cuda()).nan_to_num(7.0), lin.forward(many)[:1].nan_to_num(7.0))
     assert bt.lib().bt_device_check(0) == 0
+
+
+def test_row_quantisers_of_tiny_rows(bt, oracle):
+    # rows whose 127 / max|x| overflows, among ordinary ones, through the kernel of many rows
+    n, k, m = 48, 1024, 300
+    rng = np.random.default_rng(5)
+    packed = ternary_packed(rng, n, k)
+    x = rng.normal(0, 1, (m, k)).astype(np.float32)
+    x[7] *= 1e-39
+    x[250] = np.where(np.arange(k) % 3, 1e-40, -2e-40)
+    lin = bt.BitLinear.from_packed(packed, [0.5], n, k)
+    assert np.array_equal(lin.forward(torch.from_numpy(x).cuda()).cpu().numpy(), oracle.bitlinear_q(x, packed, [0.5], n))
