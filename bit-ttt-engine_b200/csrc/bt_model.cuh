@@ -49,6 +49,26 @@ cudaError_t launch_lm_head_tc(const void* wtiles, const float* h, const float* n
                               cudaStream_t stream, bool w_f16 = false,   // w_f16: the weight tiles hold IEEE halves
                               float cap = 0.f);                          // logits <- cap * tanh(logits / cap); 0: none
 
+// One decode step of a small TTT model up to the residual stream, in one launch (ttt_step.cu)
+struct TttStepLayer {
+    const uint8_t *down, *up, *gate_up, *mlp_down;                      // weight tiles (gate and up interleaved by 8 rows)
+    const float *sw_down, *sw_up, *sw_gate_up, *sw_mlp_down;            // [row_tiles][2] weight scales
+    const float *norm1, *norm2;
+    float* w_state;                                                     // [max_batch, small, small]
+};
+struct TttStepArgs {
+    const TttStepLayer* layers;  // device
+    int num_layers;
+    const int32_t* tokens;
+    const __nv_bfloat16* embed;
+    bool f16;                    // embed holds IEEE halves
+    int vocab, hidden, ff, batch;
+    float lr, eps;
+    float* h;                    // [batch, hidden]
+};
+bool ttt_step_fits(int hidden, int small, int ff, int batch);
+cudaError_t launch_ttt_model_step(const TttStepArgs& a, int small, cudaStream_t s);
+
 // Q8 KV cache of one layer: u8 data [batch, n_kv, max_seq, head_dim] and f32 scales
 // [batch, n_kv, max_seq] for K and V (layers/kv_cache.rs:14-24).
 struct KvCacheView {

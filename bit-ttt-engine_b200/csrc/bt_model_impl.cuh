@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "bt_handles.cuh"
+#include "bt_model.cuh"
 
 namespace bt {
 
@@ -88,6 +89,7 @@ struct bt_model {
     void* lm_btiles = nullptr;       // normalised hidden states as bf16 hi|lo tiles
     float* lm_gather = nullptr;      // tensor parallelism: the ranks' vocabulary slices of the logits, [tp][batch][vl]
     int64_t vl = 0;                  // rows of the head per rank (multiple of 128)
+    bt::TttStepLayer* ttt_layers = nullptr;  // what the one-launch step of a small TTT model reads of its layers
     unsigned int* absmax = nullptr;  // [num_layers][2][max_batch] max|x| cells of the fused path
     float* cand_val = nullptr;
     int32_t* cand_idx = nullptr;

@@ -366,6 +366,9 @@ __device__ __forceinline__ uint4 ld_dsmem_v4(uint32_t remote_addr) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote_addr) : "memory");
     return v;
 }
+__device__ __forceinline__ void st_dsmem_f32(uint32_t remote_addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_addr), "f"(v) : "memory");
+}
 // arrive on an mbarrier of another CTA of the cluster; release: this thread's earlier writes are visible
 // to whoever observes the arrival with acquire semantics
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar_addr) {

@@ -30,6 +30,7 @@
 
 #include "bt_common.cuh"
 #include "bt_ptx.cuh"
+#include "bt_tile_mma.cuh"
 
 namespace bt {
 
@@ -52,31 +53,6 @@ constexpr int kEarlyBytes = 64 * 1024;  // weight bytes a CTA requests before it
 constexpr int kTokBytes = 128;  // per-token scale and sum, shared with the epilogue warp
 constexpr int kScratchBytes = 512;  // block-reduction scratch of the prologue
 constexpr unsigned kErrGemvTimeout = 0x47454d56u;  // 'GEMV'
-
-__device__ __forceinline__ void red_add_s32(int* p, int v) {
-    asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(ptx::smem_u32(p)), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
-
-// One 1 KB tile: 2 A loads, 4 B loads, 32 ANDs, 8 MMAs.  The four field positions are four
-// independent accumulator chains: their first MMAs are issued back to back, then the second.
-// FIRST: the tile opens a row tile, its first MMAs start from the zero register (the
-// accumulators need no clearing between row tiles).
-template <bool FIRST>
-__device__ __forceinline__ void tile_mma_r(int (&acc)[4][4], const uint4& w4, const uint4& v4, const uint4 (&b4)[4]) {
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        const uint32_t mask = 0x03030303u << (2 * f);
-        if (FIRST) ptx::mma_u8s8_zero(acc[f], w4.x & mask, v4.x & mask, w4.z & mask, v4.z & mask, b4[f].x, b4[f].z);
-        else ptx::mma_u8s8(acc[f], w4.x & mask, v4.x & mask, w4.z & mask, v4.z & mask, b4[f].x, b4[f].z);
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        const uint32_t mask = 0x03030303u << (2 * f);
-        ptx::mma_u8s8(acc[f], w4.y & mask, v4.y & mask, w4.w & mask, v4.w & mask, b4[f].y, b4[f].w);
-    }
-}
 
 // ---- reductions over the 256 math threads (named barrier 1) ----------------------------
 __device__ __forceinline__ double math_sum_d(double v, double* slot, int warp, int lane) {

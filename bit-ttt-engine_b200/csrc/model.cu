@@ -145,6 +145,11 @@ cudaError_t trace_copy(const bt_model* m, int layer, int slot, const float* src,
 
 bt_status enqueue_head(bt_model* m, int rows, cudaStream_t s, bool fused_launches, bool advance = true);
 
+// (a trace wants the stages' results, which the one launch keeps to itself)
+bool ttt_in_one_launch(const bt_model* m, int batch) {
+    return m->ttt_layers && !m->trace && ttt_step_fits(m->cfg.hidden_dim, m->d_small, m->i_l, batch);
+}
+
 bt_status enqueue_step_fused(bt_model* m, int batch, cudaStream_t s) {
     const bt_model_config& c = m->cfg;
     const int H = c.hidden_dim, I = m->i_l, B = c.max_batch;
@@ -153,6 +158,13 @@ bt_status enqueue_step_fused(bt_model* m, int batch, cudaStream_t s) {
     const int sm = m->sm_count;
     const bool split_quant = m->tp == 1 && c.arch == 1 && batch >= kSplitQuantBatch;
     bt_status qst;
+    if (ttt_in_one_launch(m, batch)) {
+        TttStepArgs a = {};
+        a.layers = m->ttt_layers; a.num_layers = c.num_layers; a.tokens = m->tokens; a.embed = m->embed; a.f16 = m->embed_f16;
+        a.vocab = c.vocab_size; a.hidden = H; a.ff = I; a.batch = batch; a.lr = c.inner_lr; a.eps = kRmsEps; a.h = m->h;
+        BT_CUDA_TRY(launch_ttt_model_step(a, m->d_small, s));
+        return enqueue_head(m, batch, s, true);
+    }
     BT_CUDA_TRY(launch_embed(m->tokens, m->embed, batch, H, c.vocab_size, m->h, s, m->absmax, c.num_layers * 2 * B, true, m->embed_f16));
     for (int li = 0; li < c.num_layers; ++li) {
         Layer& L = m->layers[(size_t)li];
@@ -650,6 +662,14 @@ extern "C" bt_status bt_model_finalize(bt_model* m) {
     } else {
         BT_CUDA_TRY(dev_alloc(&m->feat, (size_t)B * m->d_small));
         BT_CUDA_TRY(dev_alloc(&m->z, (size_t)B * m->d_small));
+        if (m->tp == 1 && !m->multi_basis && ttt_step_fits(H, m->d_small, I, 1)) {
+            std::vector<TttStepLayer> layers;
+            for (const Layer& L : m->layers)
+                layers.push_back({L.ttt_down->w.tiles, L.ttt_up->w.tiles, L.gate_up_il->w.tiles, L.down->w.tiles, L.ttt_down->scale_tiles, L.ttt_up->scale_tiles,
+                                  L.gate_up_il->scale_tiles, L.down->scale_tiles, L.norm1, L.norm2, L.w_state});
+            BT_CUDA_TRY(dev_alloc(&m->ttt_layers, layers.size()));
+            BT_CUDA_TRY(cudaMemcpy(m->ttt_layers, layers.data(), layers.size() * sizeof(TttStepLayer), cudaMemcpyHostToDevice));
+        }
     }
     BT_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&m->tokens_pinned), (size_t)B * sizeof(int32_t)));
     BT_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&m->next_pinned), (size_t)B * sizeof(int32_t)));
@@ -675,7 +695,7 @@ extern "C" bt_status bt_model_destroy(bt_model* m) {
         cudaFree(L.norm1); cudaFree(L.norm2); cudaFree(L.w_state);
     }
     void* bufs[] = {m->embed, m->lm_head, m->norm_f, m->inv_freq, m->tokens, m->pos, m->h, m->q, m->sx, m->qsum,
-                    m->qkv, m->att, m->gu, m->feat, m->z, m->xn, m->logits, m->next, m->act, m->absmax, m->cand_val, m->cand_idx, m->rope_cos, m->rope_sin, m->acc_i32, m->xt, m->qtc, m->lm_tiles, m->lm_btiles, m->lm_gather};
+                    m->qkv, m->att, m->gu, m->feat, m->z, m->xn, m->logits, m->next, m->act, m->absmax, m->cand_val, m->cand_idx, m->rope_cos, m->rope_sin, m->acc_i32, m->xt, m->qtc, m->lm_tiles, m->lm_btiles, m->lm_gather, m->ttt_layers};
     for (void* p : bufs) cudaFree(p);
     for (void* p : {(void*)m->pf_tokens, (void*)m->pf_h, (void*)m->pf_qkv, (void*)m->pf_att, (void*)m->pf_gu, (void*)m->pf_qtc,
                     (void*)m->pf_sx, (void*)m->pf_qsum, (void*)m->pf_act, (void*)m->pf_qs}) cudaFree(p);
@@ -1124,6 +1144,7 @@ extern "C" int bt_model_launches_per_step(const bt_model* m, int batch) {
         // NCCL all-reduces, or + 2 max-exchange and 2 sum-exchange kernels over peer memory;
         // embedding, lm_head per 4 tokens, pick (split head: gathered-rows copy, arg-max, position advance instead)
         int per_layer = 4 + 1 + (m->tp > 1 ? (tp_peer_ready(m->peer) ? 4 : 2) : 0);
+        if (ttt_in_one_launch(m, batch)) return 1 + (batch + 3) / 4 + 1;
         if (m->tp == 1 && m->cfg.arch == 1 && batch >= kSplitQuantBatch) per_layer += 4;  // a quantiser kernel in front of every product
         return m->cfg.num_layers * per_layer + 1 + (batch + 3) / 4 + (split_head ? 3 : 1);
     }

@@ -114,3 +114,24 @@ def test_models_with_several_bases_per_projection(bt, oracle, arch, batch):
     for t in range(4):
         staged_decode_step(oracle, ref, gpu, cfg, tokens[t], states)
     assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("hidden,ff,layers,batch", [
+    (128, 256, 3, 1), (256, 688, 2, 2),   # less than a row tile to a CTA; MLP rows that fill no tile of 256 inputs
+    (256, 16, 1, 8), (512, 2048, 2, 8),   # the smallest and the largest sizes
+    (512, 1040, 2, 5), (128, 2048, 2, 3)])
+def test_small_ttt_step_in_one_launch(bt, hidden, ff, layers, batch):
+    # the step of a small model as one launch, and launch by launch as a trace has it: the same logits, picks and states,
+    # whichever of the two moved a state on before
+    syn = importlib.import_module("bit-ttt-engine_b200.synthetic")
+    cfg = syn.BitLlamaConfig("ttt", 500, hidden, layers, 4, 4, ff, inner_lr=0.3)
+    one, by_launch = (syn.build_model(syn.make_weights(cfg, seed=hidden + ff), max_batch=batch) for _ in range(2))
+    rng = np.random.default_rng(ff)
+    for step in range(6):
+        tokens = rng.integers(0, cfg.vocab_size, batch)
+        by_launch.set_trace(step != 4)
+        want, got = by_launch.forward_one(tokens), one.forward_one(tokens)
+        assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1]), step
+    for layer in range(layers):
+        assert torch.equal(one.ttt_state(layer), by_launch.ttt_state(layer))
+    assert bt.lib().bt_device_check(0) == 0
