@@ -135,3 +135,17 @@ def test_small_ttt_step_in_one_launch(bt, hidden, ff, layers, batch):
     for layer in range(layers):
         assert torch.equal(one.ttt_state(layer), by_launch.ttt_state(layer))
     assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("hidden,vocab", [(256, 40), (256, 5000), (512, 2369), (768, 2500), (8192, 700), (320, 900)])
+def test_head_of_one_token(bt, oracle, hidden, vocab):
+    # fewer rows than warps, runs of rows that end inside a slot, rows longer than a warp's ring, a width the streamed form refuses
+    syn = importlib.import_module("bit-ttt-engine_b200.synthetic")
+    heads = hidden // 64
+    cfg = syn.BitLlamaConfig("llama", vocab, hidden, 1, heads, heads // 4 if heads % 4 == 0 else heads, 64, max_position_embeddings=8)
+    w = syn.make_weights(cfg, seed=vocab, from_latent=False)
+    gpu, ref = syn.build_model(w), oracle.model_from_weights(w)
+    states = [ref.new_state()]
+    for token in (1, vocab - 1):
+        staged_decode_step(oracle, ref, gpu, cfg, [token], states)
+    assert bt.lib().bt_device_check(0) == 0
