@@ -259,12 +259,16 @@ def test_rows_quantised_in_the_product(bt, oracle, m, k, dtype):
     if m > 2:
         x[2] *= 1e-39  # 127 / max|x| overflows: every value saturates
     x = torch.from_numpy(x).to(getattr(torch, dtype))
+    if m > 2:  # (but for zeros, whose product with infinity is no number: the oracle's conversion of it to an integer is not defined)
+        x[2][x[2] == 0] = 2.0 ** -130
     lin = bt.BitLinear.from_packed(packed, [0.5], n, k)
     ref = torch.from_numpy(oracle.bitlinear_q(x.float().numpy(), packed, [0.5], n)).to(x.dtype)
     assert torch.equal(lin.forward(x.cuda()).cpu(), ref)
     apart = torch.empty(m * k + 1, dtype=x.dtype, device="cuda")[1:].view(m, k).copy_(x)  # rows that start on no 16-byte boundary
     assert torch.equal(lin.forward(apart).cpu(), ref)
     # values that are no numbers, as the quantiser kernel has them (more tokens than the product quantises itself)
+    tiny = torch.cat([torch.zeros(1, k // 2), torch.full((1, k // 2), 2.0 ** -130)], 1).to(x.dtype)
+    assert torch.equal(lin.forward(tiny.cuda()), lin.forward(tiny.expand(4, k).contiguous().cuda())[:1])
     x[0, 3], x[0, k // 2] = float("nan"), float("inf")
     many = x[:1].expand(4, k).contiguous().cuda()
     assert torch.equal(lin.forward(x[:1].cuda()).nan_to_num(7.0), lin.forward(many)[:1].nan_to_num(7.0))
