@@ -3,7 +3,7 @@
 // Scores, softmax and the running sums are f32 throughout.
 #include <cooperative_groups.h>
 
-#include "bt_dense.cuh"
+#include "attn_dense.cuh"
 #include "bt_ptx.cuh"
 
 namespace cg = cooperative_groups;
@@ -396,32 +396,6 @@ cudaError_t span_launch_r(const DenseAttn& a, bool prepared, const ActOut& out, 
 // Rows in shared memory are padded by 16 bytes, so that the eight rows of an ldmatrix fall into different banks.
 constexpr int kTileQ = 64, kTileKeys = 64, kTileThreads = 128;
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-// A raw score in units of ln 2, so that its exponential is one ex2: s * scale, or capped: cap * tanh(s * scale / cap) with
-// tanh(u) = 1 - 2 / (e^2u + 1), whose absolute error is of the order of 1e-7 cap.
-struct ScoreMap {
-    float k, cap2;  // factor on the raw score; 2 cap / ln 2, 0: no cap
-    __device__ __forceinline__ ScoreMap(float scale, float cap) {
-        const float log2e = 1.4426950408889634f;
-        k = cap > 0.0f ? scale / cap * (2.0f * log2e) : scale * log2e;
-        cap2 = cap > 0.0f ? 2.0f * cap * log2e : 0.0f;
-    }
-    __device__ __forceinline__ float operator()(float s) const {
-        const float u = s * k;
-        return cap2 > 0.0f ? fmaf(-cap2, rcp(ex2(u) + 1.0f), 0.5f * cap2) : u;
-    }
-};
-constexpr float kLn2 = 0.6931471805599453f;
-
 // ---------------------------------------------------------------------------------------
 // one query position per CTA group on the tensor cores (bf16 cache, decode)
 // ---------------------------------------------------------------------------------------
@@ -692,16 +666,6 @@ cudaError_t span_mma_launch_v(const DenseAttn& a, bool prepared, const ActOut& o
     return span_mma_launch<DK, 256>(a, prepared, out, s, pdl);
 }
 
-// LATENT: keys and values are bf16 rows expanded from the latents, the last key columns the rotated part all heads share.
-struct LatentTile {
-    const __nv_bfloat16* kv = nullptr;  // [sequence][kv_rows][heads k_main | heads v_stride]
-    int64_t kv_ld = 0, kv_seq = 0;      // elements between positions and between sequences
-    int k_main = 0;                     // columns of a head's own key part
-    LatentView latent;
-    int b0 = 0;
-    const float* gate = nullptr;        // output gates of the rows
-    int64_t gate_ld = 0;
-};
 template <int DK, int DV, bool LATENT>  // upper bounds of the (padded) head sizes
 __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(const DenseAttn a, const LatentTile lt, const ActOut out) {
     extern __shared__ __align__(16) uint8_t tsm[];
@@ -899,6 +863,15 @@ cudaError_t tile_launch_k(const DenseAttn& a, const LatentTile& lt, const ActOut
 }
 int pad8(int n) { return (n + 7) / 8 * 8; }
 
+// Tiles of 128 positions pay from this many rows on.  Their first tile takes 14 us (set-up, 128 queries, the sum of the groups at
+// the end), each further one of 128 keys 2.2 to 3.2; a tile of 64 keys of the kernel above takes 2.4 us for heads of 64 and 6 for
+// keys of 192.  64-position tiles and these, us: 32 heads of 64 with a cap, 512 rows 23.6 and 24.2, 1024 58.6 and 50.5; of 32, 512
+// rows 20.4 and 22.7, 768 36.3 and 31.0; 16 heads of 128 with a cap, 320 rows 24.5 and 25.2, 512 35.5 and 27.5; of 80 + 64, 384 rows
+// 16.4 and 17.4, 512 20.3 and 18.8; of 192 + 128, 128 rows 17.4 and 18.4, 256 26.1 and 18.3.
+bool attn_flash_pays(const DenseAttn& a) {
+    return attn_flash_fits(a) && a.q_rows >= (a.kv.k_stride <= 64 ? 640 : (a.kv.k_stride <= 128 ? 448 : 192));
+}
+
 }  // namespace
 
 int attn_max_dim() { return 256; }
@@ -923,6 +896,7 @@ bool attn_tile_fits(const DenseAttn& a) { return !a.kv.f32 && a.kv.k_stride <= 2
 
 cudaError_t launch_attn_tile(const DenseAttn& a, const ActOut& out, cudaStream_t s) {
     if (!attn_tile_fits(a) || !a.q_bf16 || !out.tiles) return cudaErrorInvalidValue;
+    if (attn_flash_pays(a)) return launch_attn_flash(a, nullptr, out, s);
     return tile_launch_k<false>(a, LatentTile(), out, s);
 }
 
@@ -934,12 +908,13 @@ cudaError_t launch_latent_tile(const LatentAttn& l, const __nv_bfloat16* kv16, i
     a.q_buf = l.q_buf; a.q_bf16 = true;
     a.scale = l.scale; a.pos = l.pos; a.batch = nb; a.q_rows = l.q_rows; a.heads = l.heads; a.n_kv = l.heads;
     a.kv.k_stride = pad8(l.dim) + pad8(l.rot); a.kv.v_stride = pad8(l.vdim); a.kv.max_seq = l.kv.max_seq;
-    a.dk = a.kv.k_stride; a.dv = l.vdim;
+    a.dk = a.kv.k_stride; a.dv = l.vdim; a.err = l.err;
     LatentTile t;
     t.kv = kv16; t.k_main = pad8(l.dim); t.kv_ld = (int64_t)l.heads * (t.k_main + a.kv.v_stride); t.kv_seq = kv_rows * t.kv_ld;
     t.latent = l.kv; t.b0 = b0;
     t.gate = l.gate ? l.proj + l.heads * (l.dim + l.rot) + l.rank + l.rot : nullptr;
     t.gate_ld = l.ld;
+    if (attn_flash_pays(a)) return launch_attn_flash(a, &t, out, s);
     return tile_launch_k<true>(a, t, out, s);
 }
 

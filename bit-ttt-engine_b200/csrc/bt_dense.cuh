@@ -214,8 +214,9 @@ struct DenseAttn {
     const int32_t* pos = nullptr;   // [batch] position of the first new token
     int batch = 1, q_rows = 1, heads = 1, n_kv = 1, dk = 0, dv = 0;
     int sm_count = 0;
-    void* q_buf = nullptr;          // prefill: prepared queries [rows, H, k_stride], bf16 (tile kernel) or f32
+    void* q_buf = nullptr;          // prefill: prepared queries [rows, H, k_stride], bf16 (tile kernels) or f32
     bool q_bf16 = false;
+    unsigned int* err = nullptr;    // the device's error word
 };
 // Query and key norm, temperature, value mixing; keys and values go to the cache, queries to q_buf.
 cudaError_t launch_attn_prep(const DenseAttn& a, cudaStream_t s);
@@ -257,7 +258,8 @@ struct LatentAttn {
     float* q_rot = nullptr;        // prepared: rotated parts [rows][heads][rot]
     uint8_t* q_tiles = nullptr;    // prepared: unrotated parts as tiled hi | lo blocks (bf16) ...
     float* q_rows32 = nullptr;     // ... or f32 rows [rows][heads][dim]
-    __nv_bfloat16* q_buf = nullptr;  // tile kernel: [rows][heads][pad8(dim) + pad8(rot)]
+    __nv_bfloat16* q_buf = nullptr;  // tile kernels: [rows][heads][pad8(dim) + pad8(rot)]
+    unsigned int* err = nullptr;     // the device's error word
     int64_t m_pad = 0;
 };
 // latents of positions [0, n) of `nb` sequences -> tiled activations [nb][kpad(rank) / 64][m_pad][64]

@@ -305,6 +305,7 @@ DenseAttn attn_args(const bt_model* m, const LayLayer& l, const LayRun& run, con
     a.batch = batch; a.q_rows = n; a.heads = c.heads; a.n_kv = c.kv_heads; a.dk = c.dim; a.dv = c.vdim;
     a.sm_count = m->sm_count;
     a.q_buf = r.q;
+    a.err = device_error_word(m->device);
     return a;
 }
 SsmArgs ssm_args(const bt_model* m, const LayLayer& l, const LayRun& run, const RowBuffers& r, int batch, int n) {
@@ -334,7 +335,7 @@ LatentAttn latent_args(const bt_model* m, const LayLayer& l, const LayRun& run, 
     if (l.table >= 0) { a.cos_t = L->tables[(size_t)l.table].cos_t; a.sin_t = L->tables[(size_t)l.table].sin_t; }
     a.heads = c.heads; a.dim = c.dim; a.rot = c.rot_dim; a.rot_dims = c.rot_dims; a.vdim = c.vdim; a.rank = c.kv_rank;
     a.kv = run.kv->latent;
-    a.pos = m->pos; a.batch = batch; a.q_rows = n; a.sm_count = m->sm_count;
+    a.pos = m->pos; a.batch = batch; a.q_rows = n; a.sm_count = m->sm_count; a.err = device_error_word(m->device);
     a.q_abs = r.a;
     a.m_pad = dense_mpad((int64_t)batch * n);
     return a;

@@ -188,6 +188,20 @@ def test_recurrence_carries_a_far_token(bt, mixer):
             assert_close(feed(m, tokens, sizes), logits, dtype, sizes)
 
 
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank", [(2, 128, 64, 128, 96), (3, 20, 6, 12, 40), (2, 96, 16, 100, 64), (2, 160, 64, 32, 72)])
+@pytest.mark.parametrize("n", [191, 192, 641])  # rows on both sides of where the tiles of 128 begin
+def test_latent_attention_by_tiles(bt, heads, dim, rot, vdim, rank, n):
+    """Prompts through the tiles of 128 positions (heads up to 192 + 128) and of 64, with positions before them and without."""
+    cfg = config(48, 64, [latent(heads, dim, rot, vdim, rank, scale=(dim + rot) ** -0.5)])
+    t = make_tensors(cfg, seed=dim)
+    tokens = np.random.default_rng(n).integers(0, 48, n + 70).astype(np.int32)
+    logits, _ = oracle(cfg, t, tokens)
+    m = lay.build_layered(cfg, t, dtype="bfloat16", max_seq_len=768)
+    for sizes in ([n, 70], [70, n]):
+        m.reset_kv_cache()
+        assert_close(feed(m, tokens, sizes), logits, "bfloat16", sizes)
+
+
 def needle_model(heads, rank):
     """One latent attention layer whose query of token 1 points at the key of token 0 (score far above all others)."""
     cfg = config(60, 96, [latent(heads, 32, 8, 24, rank, scale=0.5)])

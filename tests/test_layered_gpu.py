@@ -219,6 +219,36 @@ def test_far_keys_at_tile_borders(bt, dtype):
         assert_close(got, want[-1:], dtype)
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim,cap", [
+    (2, 1, 16, 8, 0.0), (4, 2, 64, 64, 15.0), (3, 3, 72, 7, 0.0), (2, 1, 128, 128, 6.0), (2, 2, 192, 100, 0.0),  # up to the largest heads
+    (2, 1, 200, 128, 4.0)])  # of the 128-position tiles, and beyond
+@pytest.mark.parametrize("n", [447, 448, 639, 640, 769])  # rows on both sides of where they begin, and of their size
+def test_attention_by_tiles(bt, heads, kv, dim, vdim, cap, n):
+    cfg = lay.LayersConfig(50, 64, 1000, 1e-5, True, [attn(heads, kv, dim, vdim, scale=dim ** -0.5, cap=cap)])
+    t = make_tensors(cfg, seed=dim)
+    tokens = np.random.default_rng(n).integers(0, 50, n + 130).astype(np.int32)
+    logits, _ = oracle(cfg, t, tokens, None if cap else "no_cap")
+    m = lay.build_layered(cfg, t, dtype="bfloat16")
+    assert_close(feed(m, tokens, [n, 130]), logits, "bfloat16")
+    m.reset_kv_cache()
+    assert_close(feed(m, tokens, [100, n, 64]), logits, "bfloat16")  # positions before the prompt, in whole tiles and not
+
+
+def test_attention_references_that_move(bt):
+    """A row's largest score far above that of the tiles before it: the sums so far are rescaled."""
+    cfg, t = needle_model(700, 1)
+    rng = np.random.default_rng(3)
+    m = lay.build_layered(cfg, t, dtype="bfloat16")
+    for place, asks in ((257, (258, 400, 650)), (390, (391, 640)), (520, (521, 600))):
+        tokens = rng.integers(2, 60, 660).astype(np.int32)
+        tokens[place] = 0
+        for a in asks:
+            tokens[a] = 1
+        logits, _ = oracle(cfg, t, tokens)
+        m.reset_kv_cache()
+        assert_close(m.prefill_logits(tokens, np.arange(660)), logits, "bfloat16", place)
+
+
 @pytest.mark.parametrize("dtype,batch", [("float32", 3), ("bfloat16", 2), ("bfloat16", 8), ("bfloat16", 9), ("float32", 12), ("bfloat16", 21)])
 def test_batch_equals_each_alone(bt, dtype, batch):
     cfg, t = CONFIGS["odd"], make_tensors(CONFIGS["odd"], seed=6)
