@@ -81,6 +81,44 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const DenseAttn a) {
     float inv_q, inv_k;
     qk_sums(a, row, red, inv_q, inv_k);
     inv_q *= temperature(a, p);
+    if constexpr (QBF16) {
+        // a piece of eight columns a thread, of a query, a key or a value (a warp a head and a column a lane: 1999 rows of 32 + 2 x 4 heads
+        // of 64 23.2 us, now 14.2; the products are read twice, once for the norms' sums)
+        const int per = ks / 8, pv = vs / 8, n_q = a.heads * per, n_k = p >= 0 && p < a.kv.max_seq ? a.n_kv * per : 0, n_v = n_k ? a.n_kv * pv : 0;
+        auto norm8 = [&](float (&v)[8], const float* norm, int s, int c0, float inv) {
+            float w[8];
+            if (norm) piece8(norm + s, c0, dk, w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = v[j] * inv * (norm ? w[j] : 1.0f);
+        };
+        for (int t = threadIdx.x; t < n_q + n_k + n_v; t += 256) {
+            float v[8];
+            __nv_bfloat16* dst;
+            if (t < n_q) {
+                const int h = t / per, c0 = (t - h * per) * 8;
+                piece8(row + h * dk, c0, dk, v);
+                norm8(v, a.q_norm, h * dk, c0, inv_q);
+                dst = reinterpret_cast<__nv_bfloat16*>(a.q_buf) + (r * a.heads + h) * ks + c0;
+            } else if (t < n_q + n_k) {
+                const int g = (t - n_q) / per, c0 = (t - n_q - g * per) * 8;
+                piece8(row + nq + g * dk, c0, dk, v);
+                norm8(v, a.k_norm, g * dk, c0, inv_k);
+                dst = reinterpret_cast<__nv_bfloat16*>(a.kv.k) + (((int64_t)b * a.n_kv + g) * a.kv.max_seq + p) * ks + c0;
+            } else {
+                const int g = (t - n_q - n_k) / pv, c0 = (t - n_q - n_k - g * pv) * 8, s = g * dv + c0;
+                piece8(row + nq + nk + g * dv, c0, dv, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (c0 + j < dv) {
+                        if (a.v_first_out) a.v_first_out[r * nv + s + j] = v[j];
+                        if (a.v_first_in) v[j] = (1.0f - a.v_lambda) * v[j] + a.v_lambda * a.v_first_in[r * nv + s + j];
+                    }
+                dst = reinterpret_cast<__nv_bfloat16*>(a.kv.v) + (((int64_t)b * a.n_kv + g) * a.kv.max_seq + p) * vs + c0;
+            }
+            *reinterpret_cast<uint4*>(dst) = make_uint4(ptx::pack2(v[0], v[1]), ptx::pack2(v[2], v[3]), ptx::pack2(v[4], v[5]), ptx::pack2(v[6], v[7]));
+        }
+        return;
+    }
     // a warp per head and turn
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int h = warp; h < a.heads; h += 8)
@@ -89,8 +127,7 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const DenseAttn a) {
             const int s = h * dk + c;
             const float v = c < dk ? row[s] * inv_q * (a.q_norm ? a.q_norm[s] : 1.0f) : 0.0f;
             const int64_t o = (r * a.heads + h) * ks + c;
-            if (QBF16) reinterpret_cast<__nv_bfloat16*>(a.q_buf)[o] = __float2bfloat16_rn(v);
-            else reinterpret_cast<float*>(a.q_buf)[o] = v;
+            reinterpret_cast<float*>(a.q_buf)[o] = v;
         }
     if (p < 0 || p >= a.kv.max_seq) return;
     for (int g = warp; g < a.n_kv; g += 8) {

@@ -20,6 +20,19 @@ __host__ __device__ inline int64_t dense_off(int64_t row, int c, int64_t rows_pa
 }
 __host__ __device__ inline int dense_kpad(int k) { return (k + kDenseK - 1) / kDenseK * kDenseK; }
 
+#ifdef __CUDACC__
+// eight of n columns, zeros behind them
+__device__ __forceinline__ void piece8(const float* x, int c0, int n, float (&v)[8]) {
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0 && c0 + 8 <= n) {
+        const float4 a = *reinterpret_cast<const float4*>(x + c0), b = *reinterpret_cast<const float4*>(x + c0 + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = c0 + j < n ? x[c0 + j] : 0.0f;
+    }
+}
+#endif
+
 // One matrix, or `blocks` matrices of one shape behind one another: the diagonal blocks of a block-diagonal matrix, the
 // experts of a mixture.
 struct DenseLin {
