@@ -9,10 +9,10 @@
 // bits whatever the power of two).
 // Bound: the special-function unit (ex2 per score, with a score cap ex2 + rcp + ex2: 3 x 16384 of 16 a clock and tile = 3072
 // clocks, against 770 of MMAs for heads of 64), then the softmax warps' instructions.
-// 1999 tokens, us a layer, with mma.sync tiles of 64 x 64 before -> now: 32 heads of 64 with a cap 175 -> 111, 16 heads of 192 + 128
-// 279 -> 67.  What the loop comes to is 3.2 and 2.6 us a tile; a CTA's beginning and end, 5 us once the code is in the caches, are
-// what is left, and the last round of CTAs.  Every second exponential by a polynomial on the FMA units: 130 -> 155 at the time (the
-// softmax warps are bound by issue too).  Warpgroups that trade registers (no spills of the 128 of a launch): 117 -> 112.
+// 1999 tokens, us a layer, with mma.sync tiles of 64 x 64 before -> now: 32 heads of 64 with a cap 175 -> 92, 16 heads of 192 + 128
+// 279 -> 59.  What is left beside the loop is a CTA's beginning and end and the last round of CTAs.  Every second exponential by a
+// polynomial on the FMA units: 130 -> 155 at the time (the softmax warps are bound by issue too).  Warpgroups that trade registers
+// (no spills of the 128 of a launch): 117 -> 112.
 #include <type_traits>
 
 #include "attn_dense.cuh"
@@ -47,17 +47,17 @@ __device__ __forceinline__ void ld_wait32(uint32_t (&v)[32]) {
                    "+r"(v[30]), "+r"(v[31])
                  :: "memory");
 }
-// f(c0, v) on 32 columns after 32 of a lane's 128, the next ones on their way meanwhile
+// f(c0, v) on 32 columns after 32 of a lane's 128.  Rolled up, and without the next columns on their way: unrolled four times, with the
+// loads ahead, the softmax did not stay in the instruction caches (no_instruction 2 of 6.5 stalled warps an issue): 111 us a layer of
+// 32 heads of 64 with a cap, 99 unrolled twice, 92 like this, and no better with the loads ahead in a rolled loop (95).
 template <typename F>
 __device__ __forceinline__ void each_32(uint32_t addr, F f) {
-    uint32_t v[2][32];
-    ptx::tmem_ld32(addr, v[0]);
-    ld_wait32(v[0]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (i < 3) ptx::tmem_ld32(addr + 32 * (i + 1), v[(i + 1) & 1]);
-        f(32 * i, v[i & 1]);
-        if (i < 3) ld_wait32(v[(i + 1) & 1]);
+#pragma unroll 1
+    for (int c0 = 0; c0 < kFlashKeys; c0 += 32) {
+        uint32_t v[32];
+        ptx::tmem_ld32(addr + c0, v);
+        ld_wait32(v);
+        f(c0, v);
     }
 }
 
