@@ -260,28 +260,29 @@ cudaError_t scan_launch_n(const SsmArgs& a, cudaStream_t s, bool pdl) {
 // in shared memory and then its tile of outputs; the state is cut over the warps by rows of 16 elements and columns.
 constexpr int kChunk = 64, kChunkThreads = 512, kMaxSegments = 8;
 enum class ChunkMode { kAll, kStates, kOutputs };
-template <int NP>
+template <int NP, bool ONE>
 struct ChunkCfg {
     static constexpr int WN = NP / 16 < 8 ? NP / 16 : 8, WP = 16 / WN < 4 ? 16 / WN : 4;  // warps over state rows / columns
     static constexpr int TN = NP / 16 / WN, TP = 8 / WP;                                  // 16-row tiles, 8-column tiles per warp
     static constexpr int NS = NP * 2 + 16, PS = 64 * 2 + 16;                              // bytes per shared-memory row
-    static constexpr int kC = kChunk * NS, kBx = kChunk * (NS + PS);                      // C of a chunk; B and x
-    static constexpr int kOver = 2 * NP * PS > 4 * kChunk * PS ? 2 * NP * PS : 4 * kChunk * PS;  // state, then scaled x and pair weights
+    static constexpr int kC = (ONE ? 2 : 1) * kChunk * NS, kBx = kChunk * (NS + PS);       // C of a chunk (ONE: and of the next); B and x
+    static constexpr int kOver = ONE ? 2 * NP * PS + 4 * kChunk * PS                         // state, then scaled x and pair weights
+                                     : (2 * NP * PS > 4 * kChunk * PS ? 2 * NP * PS : 4 * kChunk * PS);
     static constexpr size_t kSmem = (size_t)kC + 2 * kBx + kOver + 3 * kChunk * 4;
     static constexpr int kSlot = NP * 64;                                                 // floats of a CTA's state
     static constexpr int kLive = 32 * WN * WP;                                            // threads that hold it
 };
 
-// segs: segments (1: kAll), seg_chunks: chunks of each
-template <int NP, ChunkMode MODE>
-__global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_kernel(const SsmArgs a, int channels, int segs, int seg_chunks) {
-    using Cfg = ChunkCfg<NP>;
+// segs: segments (1: kAll), seg_chunks: chunks of each.  ONE: a CTA has its SM to itself, and nothing lies over anything else.
+template <int NP, ChunkMode MODE, bool ONE>
+__global__ void __launch_bounds__(kChunkThreads, NP <= 128 && !ONE ? 2 : 1) ssm_chunk_kernel(const SsmArgs a, int channels, int segs, int seg_chunks) {
+    using Cfg = ChunkCfg<NP, ONE>;
     constexpr int NS = Cfg::NS, PS = Cfg::PS, TN = Cfg::TN, TP = Cfg::TP;
     constexpr bool kOut = MODE != ChunkMode::kStates;
     extern __shared__ __align__(16) uint8_t csm[];   // C | B, x of a chunk and of the next | state, scaled x, pair weights
     uint8_t* s_hi = csm + Cfg::kC + 2 * Cfg::kBx;    // state [NP][64] hi, lo
     uint8_t* s_lo = s_hi + NP * PS;
-    uint8_t* w_hi = s_hi;                            // over the state, once C S is done: scaled x [64][64] hi, lo
+    uint8_t* w_hi = ONE ? s_lo + NP * PS : s_hi;     // (over the state, once C S is done): scaled x [64][64] hi, lo
     uint8_t* w_lo = w_hi + kChunk * PS;
     uint8_t* m_hi = w_lo + kChunk * PS;              // pair weights [64][64] hi, lo
     uint8_t* m_lo = m_hi + kChunk * PS;
@@ -360,8 +361,8 @@ __global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_ke
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto load_c = [&](int t0) {
-        const uint32_t dst = ptx::smem_u32(csm);
+    auto load_c = [&](int t0, int buf) {
+        const uint32_t dst = ptx::smem_u32(csm) + (ONE ? buf * kChunk * NS : 0);
         constexpr int NQ = NP / 8;
         for (int e = threadIdx.x; e < kChunk * NQ; e += kChunkThreads) {
             const int t = e / NQ, q = e - t * NQ;
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_ke
         const int t = t0 + (int)threadIdx.x;
         return threadIdx.x < kChunk && t < t_end ? a.proj[((int64_t)b * a.q_rows + t) * a.ld + inner + channels + head] : 0.0f;
     };
-    if (kOut) load_c(t_first);
+    if (kOut) load_c(t_first, 0);
     load_bx(t_first, 0);
     float dt_raw = raw_dt(t_first);
 
@@ -407,10 +408,11 @@ __global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_ke
                     }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
+        if (ONE && kOut && t0 + kChunk < t_end) load_c(t0 + kChunk, buf ^ 1);
         if (t0 + kChunk < t_end) load_bx(t0 + kChunk, buf ^ 1);
         uint8_t* bt = csm + Cfg::kC + buf * Cfg::kBx;
         uint8_t* xt = bt + kChunk * NS;
-        const uint32_t c_sm = ptx::smem_u32(csm), b_sm = ptx::smem_u32(bt), x_sm = b_sm + kChunk * NS;
+        const uint32_t c_sm = ptx::smem_u32(csm) + (ONE ? buf * kChunk * NS : 0), b_sm = ptx::smem_u32(bt), x_sm = b_sm + kChunk * NS;
         // ---- running sums of the decays' logarithms, while the other warps multiply ----
         if (warp == 0) {
             const float c0 = a_neg * dt_s[2 * lane], c1 = a_neg * dt_s[2 * lane + 1];
@@ -453,7 +455,7 @@ __global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_ke
             }
         }
         __syncthreads();  // running sums; C and the state's hi | lo have been read
-        if (kOut && t0 + kChunk < t_end) load_c(t0 + kChunk);
+        if (!ONE && kOut && t0 + kChunk < t_end) load_c(t0 + kChunk, 0);
         // ---- x scaled for the state update; pair weights ----
         for (int e = threadIdx.x; e < kChunk * 32; e += kChunkThreads) {
             const int t = e >> 5, o = t * PS + (e & 31) * 4;
@@ -558,21 +560,22 @@ __global__ void __launch_bounds__(kChunkThreads, NP <= 128 ? 2 : 1) ssm_chunk_ke
 }
 
 // Segments of a prompt: as many as there are CTA slots for every head (two CTAs an SM up to 128 state elements), of two chunks
-// at least.  Making the states apart costs a third of a segment's time (34 against 103 us above), so that two segments already
-// take 0.7 of the whole prompt's time; where a CTA per head fills the slots there is nothing to gain.
+// at least, where half of the SMs or more would be idle.  Two CTAs of an SM get through no more tokens than one, and making the
+// states apart costs a third of a segment's time (34 against 103 us above): 64 heads in two segments or in four take 0.67 of the
+// whole prompt's time, while 128 heads in two took 290 us a layer (with the convolution) where one CTA a head took 258.
 int ssm_segments(const SsmArgs& a) {
     const int64_t ctas = (int64_t)a.heads * ((a.vdim + 63) / 64) * a.batch, slots = (int64_t)a.sm_count * (a.state_pad <= 128 ? 2 : 1);
     const int chunks = (a.q_rows + kChunk - 1) / kChunk;
     const int64_t segs = std::min<int64_t>(std::min<int64_t>(slots / ctas, chunks / 2), kMaxSegments);
-    return a.seg_s && segs > 1 ? (int)segs : 1;
+    return a.seg_s && segs > 1 && 2 * ctas <= a.sm_count ? (int)segs : 1;
 }
 
-template <int NP, ChunkMode MODE>
+template <int NP, ChunkMode MODE, bool ONE = false>
 cudaError_t chunk_launch_mode(const SsmArgs& a, int segs, int seg_chunks, int grid_segs, cudaStream_t s) {
     static PerDeviceOnce once;
-    cudaError_t e = once.run([] { return cudaFuncSetAttribute(ssm_chunk_kernel<NP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChunkCfg<NP>::kSmem); });
+    cudaError_t e = once.run([] { return cudaFuncSetAttribute(ssm_chunk_kernel<NP, MODE, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChunkCfg<NP, ONE>::kSmem); });
     if (e != cudaSuccess) return e;
-    ssm_chunk_kernel<NP, MODE><<<dim3((unsigned)a.heads, (unsigned)((a.vdim + 63) / 64 * grid_segs), (unsigned)a.batch), kChunkThreads, ChunkCfg<NP>::kSmem, s>>>(
+    ssm_chunk_kernel<NP, MODE, ONE><<<dim3((unsigned)a.heads, (unsigned)((a.vdim + 63) / 64 * grid_segs), (unsigned)a.batch), kChunkThreads, ChunkCfg<NP, ONE>::kSmem, s>>>(
         a, a.heads * a.vdim + 2 * a.groups * a.state, segs, seg_chunks);
     return cudaGetLastError();
 }
@@ -582,7 +585,13 @@ cudaError_t chunk_launch(const SsmArgs& a, cudaStream_t s) {
     int segs = ssm_segments(a);
     const int seg_chunks = (chunks + segs - 1) / segs;
     segs = (chunks + seg_chunks - 1) / seg_chunks;
-    if (segs == 1) return chunk_launch_mode<NP, ChunkMode::kAll>(a, 1, chunks, 1, s);
+    if (segs == 1) {
+        // A CTA an SM at most: the form that has the SM to itself (1999 tokens, 64 x 128: 128 heads 192 us, in the form for two CTAs 280;
+        // 208 before there were two).  More CTAs than SMs: two an SM at a time (64 heads, 8 prompts: 1 809 us for 16 launches, 1 850 before).
+        if constexpr (NP <= 128)
+            if ((int64_t)a.heads * ((a.vdim + 63) / 64) * a.batch <= a.sm_count) return chunk_launch_mode<NP, ChunkMode::kAll, true>(a, 1, chunks, 1, s);
+        return chunk_launch_mode<NP, ChunkMode::kAll>(a, 1, chunks, 1, s);
+    }
     cudaError_t e = chunk_launch_mode<NP, ChunkMode::kStates>(a, segs, seg_chunks, segs - 1, s);
     return e == cudaSuccess ? chunk_launch_mode<NP, ChunkMode::kOutputs>(a, segs, seg_chunks, segs, s) : e;
 }
