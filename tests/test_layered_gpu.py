@@ -176,6 +176,18 @@ def test_recurrence_in_segments(bt, state, n):
     assert_close(feed(m, tokens, [15, n]), logits, "bfloat16")  # a state to start from
 
 
+@pytest.mark.parametrize("heads", [76, 150])  # a CTA for more than half of the SMs, and for more than all of them
+def test_recurrence_of_many_heads(bt, heads):
+    cfg = lay.LayersConfig(40, 48, 400, 1e-5, True, [ssm(heads, 8, 128, taps=2)])
+    t = make_tensors(cfg, seed=heads)
+    tokens = np.random.default_rng(heads).integers(0, 40, 340).astype(np.int32)
+    logits, _ = oracle(cfg, t, tokens)
+    m = lay.build_layered(cfg, t, dtype="bfloat16")
+    for sizes in ([320, 20], [15, 325]):
+        m.reset_kv_cache()
+        assert_close(feed(m, tokens, sizes), logits, "bfloat16", sizes)
+
+
 def needle_model(n_positions, dtype_seed=0):
     """One attention layer whose query of token 1 points at the key of token 0 (score far above all others)."""
     cfg = lay.LayersConfig(60, 96, n_positions, 1e-5, True, [attn(4, 2, 32, 24, scale=0.6, cap=18.0, coef=0.3, every=50)])
