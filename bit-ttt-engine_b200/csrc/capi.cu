@@ -314,6 +314,8 @@ bt_status run_product(bt_linear* lin, const WsPlan& p, int64_t m, void* out, bt_
 // meanwhile; every CTA repeats the rows' quantisation, though, which from the fourth token on costs what the launch did.  One call
 // with the quantiser -> fused, us: 2048 x 2048, 1 token 5.6 -> 3.4, 2: 6.4 -> 5.0, 3: 6.7 -> 6.5, 4: 7.0 -> 7.9; 4096 x 4096, 3: 7.7
 // -> 7.8; 14336 x 4096, 3: 16.3 -> 13.1, 4: 16.8 -> 15.7; 16384 x 16384, 4: 27.0 -> 27.2.
+// Rows and outputs have to be apart: a CTA reads the rows at its own time, when another may have stored its outputs already.  A call in
+// place keeps the quantiser's launch, which has read every row before the product stores anything.
 constexpr int64_t kRowTokens = 3;
 
 extern "C" bt_status bt_linear_forward(bt_linear* lin, bt_workspace* ws, const void* x_dev, int64_t m,
@@ -363,7 +365,10 @@ extern "C" bt_status bt_linear_forward(bt_linear* lin, bt_workspace* ws, const v
             return BT_OK;
         }
     }
-    if (m <= kRowTokens && lin->w.n_bases == 1 && gemv_takes_rows(x_dev, lin->w.k_in) && m <= gemv_max_tokens(lin->w.k_tiles)) {
+    const uint8_t *x0 = static_cast<const uint8_t*>(x_dev), *x1 = x0 + (size_t)m * lin->w.k_in * (x_dtype == BT_BF16 ? 2 : 4);
+    const uint8_t *y0 = static_cast<const uint8_t*>(y_dev), *y1 = y0 + (size_t)m * lin->w.n_out * (y_dtype == BT_BF16 ? 2 : 4);
+    const bool apart = x1 <= y0 || y1 <= x0;
+    if (m <= kRowTokens && apart && lin->w.n_bases == 1 && gemv_takes_rows(x_dev, lin->w.k_in) && m <= gemv_max_tokens(lin->w.k_tiles)) {
         FusedIn in{PRO_ROW, static_cast<const float*>(x_dev), lin->w.k_in, nullptr, 0.0f, nullptr, x_dtype == BT_BF16};
         BT_CUDA_TRY(linear_product_fused(lin->dev(), in, (int)m, y_dev, lin->w.n_out, y_dtype == BT_BF16 ? EPI_BF16 : EPI_F32, nullptr,
                                          device_error_word(lin->device), device_sm_count(lin->device), s));

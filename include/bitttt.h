@@ -97,7 +97,8 @@ bt_status bt_workspace_destroy(bt_workspace* ws);
  * x_dtype: BT_F32 or BT_BF16; y_dtype: BT_F32 or BT_BF16.  x_k must equal the handle's
  * k_in, else BT_ERR_SHAPE with the reference's message.  ws may be NULL: a workspace
  * owned by the handle is then used (allocated on first use; calls on one handle with
- * ws == NULL must not overlap). */
+ * ws == NULL must not overlap).  y_dev may be x_dev where n_out == k_in and the types are the
+ * same. */
 bt_status bt_linear_forward(bt_linear* lin, bt_workspace* ws, const void* x_dev, int64_t m,
                             int64_t x_k, bt_dtype x_dtype, void* y_dev, bt_dtype y_dtype,
                             void* stream);

@@ -275,6 +275,27 @@ def test_rows_quantised_in_the_product(bt, oracle, m, k, dtype):
     assert bt.lib().bt_device_check(0) == 0
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 9, 130])  # on both sides of where the product quantises its rows itself, and of the tensor-core product
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_in_place(bt, m, dtype):
+    # outputs over the inputs, and over a part of them, through the C entry: what the call with outputs of their own gives
+    n = 8192  # more row tiles than CTAs that run at once: the last outputs are stored long after the first
+    rng = np.random.default_rng(m)
+    lin = bt.BitLinear.from_packed(ternary_packed(rng, n, n), [0.5], n, n)
+    x = torch.from_numpy(rng.normal(0, 1, (m, n)).astype(np.float32)).to(getattr(torch, dtype)).cuda()
+    want, code = lin.forward(x), 0 if dtype == "float32" else 1
+    for shift in (0, 16, n // 2):  # y begins so many values into x
+        if shift and m > 8:
+            continue  # (every row has been read only up to a pass of the tensor-core product)
+        for _ in range(4):
+            buf = torch.empty(m * n + shift, dtype=x.dtype, device="cuda")
+            buf[:m * n] = x.view(-1)
+            y = buf[shift:]
+            assert bt.lib().bt_linear_forward(lin._h, None, buf.data_ptr(), m, n, code, y.data_ptr(), code, torch.cuda.current_stream().cuda_stream) == 0
+            assert torch.equal(y.view(m, n), want), (m, shift)
+    assert bt.lib().bt_device_check(0) == 0
+
+
 def test_row_quantisers_of_tiny_rows(bt, oracle):
     # rows whose 127 / max|x| overflows, among ordinary ones, through the kernel of many rows
     n, k, m = 48, 1024, 300
