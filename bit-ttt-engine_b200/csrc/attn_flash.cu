@@ -286,6 +286,9 @@ __global__ void __launch_bounds__(kFlashThreads, 1) attn_flash_kernel(const Dens
             if (mask) weights(std::true_type{});
             else weights(std::false_type{});
             ptx::tmem_st_wait();
+            // Not a tile ahead of the MMA thread: with three places the scores of tile t exist before the product of tile t - 2, and a
+            // second arrival on p_full while that product still waits for its values would complete a phase that nobody has seen.
+            if (t >= 2) ok &= ptx::mbar_wait_bounded(&sm.o_done[w], (uint32_t)(((t - 2) >> 1) & 1));
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&sm.p_full[w]);

@@ -246,6 +246,25 @@ def test_attention_by_tiles(bt, heads, kv, dim, vdim, cap, n):
     assert_close(feed(m, tokens, [100, n, 64]), logits, "bfloat16")  # positions before the prompt, in whole tiles and not
 
 
+@pytest.mark.parametrize("vdim", [64, 128])  # three places for scores, and two
+def test_attention_by_tiles_under_traffic(bt, vdim):
+    """Copies that come late, because another stream takes the memory: the same bits as on an idle GPU."""
+    cfg = lay.LayersConfig(50, 256, 2100, 1e-5, True, [attn(16, 4, 64, vdim, scale=0.125)])
+    t = make_tensors(cfg, seed=vdim)
+    tokens = np.random.default_rng(vdim).integers(0, 50, 2000).astype(np.int32)
+    m = lay.build_layered(cfg, t, dtype="bfloat16")
+    want = m.prefill_logits(tokens, np.arange(0, 2000, 40))
+    side, a, b = torch.cuda.Stream(), *torch.empty(2, 1 << 28, dtype=torch.uint8, device="cuda")
+    for _ in range(5):
+        m.reset_kv_cache()
+        with torch.cuda.stream(side):
+            for _ in range(20):  # 2 ms
+                b.copy_(a)
+        assert np.array_equal(m.prefill_logits(tokens, np.arange(0, 2000, 40)), want)
+        torch.cuda.synchronize()
+    assert bt.lib().bt_device_check(0) == 0
+
+
 def test_attention_references_that_move(bt):
     """A row's largest score far above that of the tiles before it: the sums so far are rescaled."""
     cfg, t = needle_model(700, 1)
