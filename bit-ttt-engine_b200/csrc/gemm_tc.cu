@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
     constexpr uint32_t kTmemCols = (kAccCols + kABufs * RS * kAChunkCols) <= 256 ? 256 : 512;
     static_assert(kAccCols + kABufs * RS * kAChunkCols <= 512, "tensor memory");
     static_assert(kStages >= 3, "ring");
+    static_assert(RS == 2 || kStages % 2 == 0 || kStages > kABufs, "a set of unpack warps must not ask for a stage whose chunk before has not landed");
     extern __shared__ __align__(1024) uint8_t smem[];  // (the swizzle of the activation blocks goes by address bits 7 and 8)
     uint8_t* stage_base = smem;                                           // kStages x (raw | B)
     int32_t* pbuf = reinterpret_cast<int32_t*>(stage_base + (size_t)kStages * kStageBytes);  // [RS][NT / 4][128 rows][4]
@@ -310,7 +311,16 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 if (RS == 1 && (g & 1) != set) continue;
                 const int slot = g % kStages, u = g % kABufs, a_use = g / kABufs;
-                const uint32_t full_parity = (uint32_t)((g / kStages) & 1);
+                const uint32_t full_parity = (uint32_t)((g / kStages) & 1), buffer_parity = (uint32_t)((a_use - 1) & 1);
+                // RS = 1: the buffer before the weights.  The chunk that lay in this stage before belongs to the other set (kStages is odd),
+                // and while its copies were still on their way the parity asked for below would be granted for the phase before
+                // them.  The buffer's last product, kABufs chunks back, came after that chunk's.  (A ring of four stages, in which a set
+                // meets the same stages again and again, takes the same time with single CTAs, but 2048 x 14336 -> 4096 142 us with
+                // pairs, and 133 like this.)
+                if (RS == 1 && a_use > 0 && !__all_sync(0xffffffffu, ptx::mbar_test_wait(&a_empty[u], buffer_parity))) {
+                    publish();
+                    ok &= ptx::mbar_wait_bounded(&a_empty[u], buffer_parity);
+                }
                 if (!__all_sync(0xffffffffu, ptx::mbar_test_wait(&full[slot], full_parity))) {  // (one answer for the whole warp)
                     publish();  // the next weights are not here yet: do not hold the finished buffer back
                     ok &= ptx::mbar_wait_bounded(&full[slot], full_parity);
@@ -323,7 +333,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                     if (r8 < rts) w[t] = *reinterpret_cast<const uint4*>(raw + t * 16);
                 }
                 publish();
-                if (a_use > 0) ok &= ptx::mbar_wait_bounded(&a_empty[u], (uint32_t)((a_use - 1) & 1));
+                if (RS == 2 && a_use > 0) ok &= ptx::mbar_wait_bounded(&a_empty[u], buffer_parity);
                 ptx::tc_fence_after();
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {

@@ -227,6 +227,27 @@ def test_tensor_core_path_cta_pairs(bt, oracle, m, n, k, dtype, bases):
 
 
 @pytest.mark.parametrize("m,n,k,bases", [
+    (9, 4000, 14336, 1), (64, 512, 8192, 1), (64, 20000, 2048, 1), (40, 1024, 8192, 3),  # inputs cut over clusters, 256-row tiles, several bases
+    (130, 1000, 14336, 1), (300, 9217, 4096, 1), (2049, 1160, 8192, 1)])                # 128-row tiles, CTA pairs
+def test_products_under_traffic(bt, m, n, k, bases):
+    # copies that come late and out of order, because another stream takes the memory: the bits of an idle GPU
+    rng = np.random.default_rng(m)
+    packed = np.stack([ternary_packed(rng, n, k) for _ in range(bases)], -1)
+    lin = bt.BitLinear.from_packed(packed, [0.5 / 3 ** b for b in range(bases)], n, k)
+    x = torch.from_numpy(rng.normal(0, 1, (m, k)).astype(np.float32)).cuda()
+    ws, want, side = bt.Workspace(nbytes=64 << 20), lin.forward(x), torch.cuda.Stream()
+    a, b = torch.empty(2, 1 << 27, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(40):  # 2 ms
+            b.copy_(a)
+    got = [lin.forward(x, workspace=ws) for _ in range(20)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want) for y in got)
+    assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("m,n,k,bases", [
     (9, 128, 256, 2), (40, 300, 516, 8),                     # one row tile; eight bases, rows that fill no tile
     (16, 4096, 4096, 3), (33, 1000, 8192, 3), (64, 600, 2048, 2),  # inputs cut over clusters
     (64, 19100, 260, 2)])                                    # more row tiles than SMs
