@@ -72,6 +72,22 @@ __device__ __forceinline__ bool mbar_spin_relaxed(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// The same with an acquire at cluster scope, for a barrier on which another CTA of the cluster arrives.
+__device__ __forceinline__ bool mbar_spin_cluster(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 24)) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 // Bounded wait for warps that are off the critical path (a producer waiting for a free slot,
 // an epilogue warp waiting for partial sums): a non-blocking test and a short sleep between
 // tests, so that the waiting warp leaves the shared-memory pipeline to the warps doing work.

@@ -240,14 +240,19 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             for (int tile = cid; tile < n_tiles; tile += n_clusters)
             for (int basis = 0; basis < bases; ++basis, ++tl) {
                 const int sel = tl % kAccSets, acc_use = tl / kAccSets;
-                if (acc_use > 0) ok &= ptx::mbar_wait_bounded(&acc_empty[sel], (uint32_t)((acc_use - 1) & 1));
+                if constexpr (PAIR) { if (acc_use > 0) ok &= ptx::mbar_spin_cluster(&acc_empty[sel], (uint32_t)((acc_use - 1) & 1)); }
+                else if (acc_use > 0) ok &= ptx::mbar_wait_bounded(&acc_empty[sel], (uint32_t)((acc_use - 1) & 1));
                 ptx::tc_fence_after();
                 for (int kt = kt0; kt < kt1; ++kt, ++g) {
                     const int slot = g % kStages, u = g % kABufs;
                     // One wait per chunk: the unpack warps arrive on a_full after they have seen full[slot] complete, which
                     // covers the stage's activation block as well as its weights.  Every instruction between two MMAs
                     // of this thread costs tensor-pipe time (the queue behind it is short), hence the relaxed wait.
-                    ok &= ptx::mbar_spin_relaxed(&a_full[u], (uint32_t)((g / kABufs) & 1));     // weights unpacked into tensor memory
+                    // (A pair's wait acquires at cluster scope: the peer's warps arrive too, for weights in its tensor memory and activations
+                    // in its shared memory.  The acquire costs nothing here, relaxed -> acquired us: 4096 x 14336 -> 4096 259.2 -> 255.9,
+                    // 2048 x 4096 -> 6144 60.8 -> 60.2; a relaxed wait with a cluster fence behind it 365.7 and 82.4.)
+                    if constexpr (PAIR) ok &= ptx::mbar_spin_cluster(&a_full[u], (uint32_t)((g / kABufs) & 1));
+                    else ok &= ptx::mbar_spin_relaxed(&a_full[u], (uint32_t)((g / kABufs) & 1));  // weights unpacked into tensor memory
                     ptx::tc_fence_after();
                     const uint32_t b_addr = ptx::smem_u32(stage_base + (size_t)slot * kStageBytes + kRawBytes);
 #pragma unroll
