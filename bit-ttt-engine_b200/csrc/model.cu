@@ -4,6 +4,7 @@
 // all arithmetic is in the kernels.
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "bt_model_impl.cuh"
@@ -626,7 +627,8 @@ extern "C" bt_status bt_model_finalize(bt_model* m) {
     BT_CUDA_TRY(dev_alloc(&m->q, (size_t)B * m->q_stride));
     BT_CUDA_TRY(dev_alloc(&m->sx, (size_t)B));
     BT_CUDA_TRY(dev_alloc(&m->qsum, (size_t)B));
-    BT_CUDA_TRY(dev_alloc(&m->gu, (size_t)B * 2 * I));
+    // (gate and up rows; the products on their own of bt_model_enqueue_products, all four kinds of them)
+    BT_CUDA_TRY(dev_alloc(&m->gu, (size_t)B * std::max<int64_t>({2ll * I, (int64_t)H, (int64_t)m->qkv_dim})));
     BT_CUDA_TRY(dev_alloc(&m->xn, (size_t)B * H));
     BT_CUDA_TRY(dev_alloc(&m->act, (size_t)B * I));
     if (B > 8) {
@@ -851,7 +853,7 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     BT_CUDA_TRY(dev_alloc(&m->pf_h, (size_t)rows * H));
     BT_CUDA_TRY(dev_alloc(&m->pf_qkv, (size_t)rows * qw));
     BT_CUDA_TRY(dev_alloc(&m->pf_att, (size_t)rows * H));
-    BT_CUDA_TRY(dev_alloc(&m->pf_gu, (size_t)rows * 2 * I));
+    BT_CUDA_TRY(dev_alloc(&m->pf_gu, (size_t)rows * std::max(2 * I, m->multi_basis ? H : (int64_t)0)));  // (with several bases a projection's sum as well)
     BT_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&m->pf_qtc), gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)));
     BT_CUDA_TRY(dev_alloc(&m->pf_sx, (size_t)rows));
     if (c.arch == 1) BT_CUDA_TRY(dev_alloc(&m->pf_qs, (size_t)rows * m->nh_l));

@@ -303,6 +303,18 @@ def test_prefill_silu_in_the_product(bt, oracle, syn, hidden, ff, batch, n):
     assert bt.lib().bt_device_check(0) == 0
 
 
+@pytest.mark.parametrize("arch,n", [("llama", 40), ("llama", 100), ("ttt", 100)])
+def test_prefill_of_several_bases_and_a_narrow_mlp(bt, oracle, syn, arch, n):
+    # the sum of a projection's bases is wider than the gate and up rows whose buffer it borrows
+    cfg = syn.BitLlamaConfig(arch, 64, 512, 2, 8, 4 if arch == "llama" else 8, 64, inner_lr=0.01, max_position_embeddings=256)
+    w = syn.make_weights(cfg, seed=n, n_bases=2)
+    gpu, ref = syn.build_model(w, max_batch=2), oracle.model_from_weights(w)
+    states = [ref.new_state() for _ in range(2)]
+    staged_prefill(oracle, ref, gpu, cfg, np.random.default_rng(n).integers(0, 64, size=(2, n)), states)
+    gpu.enqueue_products(2)  # (the other caller of such a buffer)
+    assert bt.lib().bt_device_check(0) == 0
+
+
 def test_prompts_of_more_rows_than_one_pass(bt, syn):
     # a call of more rows than the prefill works on at a time is cut by the host: the same as calls that fit one
     # pass each - bit for bit without attention, in the first layer's cache with it
