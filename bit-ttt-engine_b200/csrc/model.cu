@@ -841,23 +841,31 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     if (m->lay) return layered_prefill_buffers(m, rows);
     if (rows <= m->pf_rows) return BT_OK;
     const bt_model_config& c = m->cfg;
-    const int64_t H = c.hidden_dim, I = m->i_l;
+    const int64_t H = c.hidden_dim, I = m->i_l, kmax = H > I ? H : I;
     const int64_t qw = c.arch == 1 ? m->qkv_dim : m->d_small;  // q|k|v, or the TTT features and predictions (two slots)
-    BT_CUDA_TRY(cudaDeviceSynchronize());
-    auto drop = [](auto*& p) { cudaFree(p); p = nullptr; };
-    drop(m->pf_tokens); drop(m->pf_h); drop(m->pf_qkv); drop(m->pf_att); drop(m->pf_gu); drop(m->pf_qtc);
-    drop(m->pf_sx); drop(m->pf_qsum); drop(m->pf_qs);
-    m->pf_rows = 0;
-    const int64_t kmax = H > I ? H : I;
-    BT_CUDA_TRY(dev_alloc(&m->pf_tokens, (size_t)rows));
-    BT_CUDA_TRY(dev_alloc(&m->pf_h, (size_t)rows * H));
-    BT_CUDA_TRY(dev_alloc(&m->pf_qkv, (size_t)rows * qw));
-    BT_CUDA_TRY(dev_alloc(&m->pf_att, (size_t)rows * H));
-    BT_CUDA_TRY(dev_alloc(&m->pf_gu, (size_t)rows * std::max(2 * I, m->multi_basis ? H : (int64_t)0)));  // (with several bases a projection's sum as well)
-    BT_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&m->pf_qtc), gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)));
-    BT_CUDA_TRY(dev_alloc(&m->pf_sx, (size_t)rows));
-    if (c.arch == 1) BT_CUDA_TRY(dev_alloc(&m->pf_qs, (size_t)rows * m->nh_l));
-    BT_CUDA_TRY(dev_alloc(&m->pf_qsum, (size_t)rows));
+    const int64_t gu = std::max(2 * I, m->multi_basis ? H : (int64_t)0);  // (with several bases a projection's sum as well)
+    const size_t n = (size_t)rows;
+    struct { void** p; size_t bytes; void* fresh; } bufs[] = {
+        {(void**)&m->pf_tokens, n * sizeof(int32_t)}, {(void**)&m->pf_h, n * H * sizeof(float)}, {(void**)&m->pf_qkv, n * qw * sizeof(float)},
+        {(void**)&m->pf_att, n * H * sizeof(float)}, {(void**)&m->pf_gu, n * gu * sizeof(float)},
+        {(void**)&m->pf_qtc, gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)}, {(void**)&m->pf_sx, n * sizeof(float)},
+        {(void**)&m->pf_qs, c.arch == 1 ? n * m->nh_l * sizeof(float) : 0}, {(void**)&m->pf_qsum, n * sizeof(int32_t)}};
+    auto drop = [&]() -> cudaError_t {
+        const cudaError_t e = cudaDeviceSynchronize();
+        for (auto& b : bufs) { cudaFree(*b.p); *b.p = nullptr; }
+        m->pf_rows = 0;
+        return e;
+    };
+    // A large pass comes beside the buffers that there are, so that a model without the memory for it keeps what it works with.
+    const bool beside = rows > kPrefillRowsLeast;
+    cudaError_t e = beside ? cudaSuccess : drop();
+    for (auto& b : bufs)
+        if (e == cudaSuccess && b.bytes) e = cudaMalloc(&b.fresh, b.bytes);
+    if (e == cudaSuccess && beside) e = drop();
+    if (e != cudaSuccess)
+        for (auto& b : bufs) cudaFree(b.fresh);
+    BT_CUDA_TRY(e);
+    for (auto& b : bufs) *b.p = b.fresh;
     m->pf_rows = rows;
     return BT_OK;
 }
@@ -991,11 +999,12 @@ bt_status prefill_impl(bt_model* m, const int32_t* tokens_host, int batch, int n
         if (c.arch == 0 && per < n_tokens && per > ttt_chunk) per -= per % ttt_chunk;
         if (m->trace && (int64_t)batch * per > m->trace_rows) per = m->trace_rows / batch;
     };
-    cut(m->lay ? kPrefillRowsLeast : kPrefillRows);
+    cut(m->lay || m->pf_least ? kPrefillRowsLeast : kPrefillRows);
     if (per < 1) return set_error(BT_ERR_NOMEM, "bt_model_prefill: the trace buffer holds fewer rows than sequences");
     bt_status st = prefill_buffers(m, batch * per);
     if (st != BT_OK && batch * per > kPrefillRowsLeast) {
         cudaGetLastError();  // (an allocation that failed leaves the context as it was)
+        m->pf_least = true;  // (not tried again: every call would wait for the device and allocate)
         cut(kPrefillRowsLeast);
         st = prefill_buffers(m, batch * per);
     }

@@ -340,3 +340,32 @@ def test_prompts_of_more_rows_than_one_pass(bt, syn):
     # its row's largest: a few such steps over two layers)
     assert rel_err(la, lb) <= 5e-2
     assert bt.lib().bt_device_check(0) == 0
+
+
+def test_prompt_without_memory_for_the_large_pass(bt, syn):
+    # a model that cannot have the buffers of a large pass works in small ones, keeps those it has, and does not ask again
+    cfg = syn.BitLlamaConfig("llama", 500, 1024, 1, 8, 2, 4096, max_position_embeddings=1700)  # 350 MB for 6800 rows, 105 for 2048
+    w = syn.make_weights(cfg, seed=6602, from_latent=False)
+    import torch
+    free_bytes = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    tokens = np.random.default_rng(18).integers(0, 500, size=(4, 1700))
+    a, b, pieces = (syn.build_model(w, max_batch=4) for _ in range(3))
+    for i in range(0, 1700, 512):  # what passes of 2048 rows are
+        want, _ = pieces.prefill(tokens[:, i:i + 512])
+    b.prefill(tokens[:, :512])
+    b.reset_kv_cache()
+    torch.cuda.empty_cache()
+    filler = torch.empty(free_bytes() - (250 << 20), dtype=torch.uint8, device="cuda")  # (b has the buffers of a small pass already)
+    before = free_bytes()
+    for _ in range(2):
+        assert np.array_equal(b.prefill(tokens)[0], want)
+        assert free_bytes() == before
+        b.reset_kv_cache()
+    assert np.array_equal(a.prefill(tokens)[0], want)
+    a.reset_kv_cache()
+    del filler
+    torch.cuda.empty_cache()
+    before = free_bytes()
+    assert np.array_equal(a.prefill(tokens)[0], want) and np.array_equal(b.prefill(tokens)[0], want)
+    assert free_bytes() == before
+    assert bt.lib().bt_device_check(0) == 0
