@@ -833,7 +833,7 @@ namespace {
 
 // Rows (sequences x tokens) that one prefill pass works on.  Ternary models: with 2048 rows the products of a 2048-wide model have
 // 64 to 160 tiles for 74 CTA pairs, and every pass ends in a wait of the host (16 prompts of 511 tokens, 1B: 5 156 us in passes
-// of 2048, 3 874 in one).  Layer-list models keep more buffers a row, and a ternary model without the memory for 8192 (1.5 GB
+// of 2048, 3 874 in one).  Layer-list models keep more buffers a row, and a ternary model without the memory for 8192 (1.1 GB
 // at 4096 x 14336) works on 2048 as well.
 constexpr int kPrefillRows = 8192, kPrefillRowsLeast = 2048;
 
@@ -843,11 +843,15 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     const bt_model_config& c = m->cfg;
     const int64_t H = c.hidden_dim, I = m->i_l, kmax = H > I ? H : I;
     const int64_t qw = c.arch == 1 ? m->qkv_dim : m->d_small;  // q|k|v, or the TTT features and predictions (two slots)
-    const int64_t gu = std::max(2 * I, m->multi_basis ? H : (int64_t)0);  // (with several bases a projection's sum as well)
     const size_t n = (size_t)rows;
+    // Gate and up rows, or silu(gate) * up where the product leaves that (more than 64 rows: 470 MB instead of 940 for 8192 x 14336); with
+    // several bases a projection's sum as well.
+    bool act = true;
+    for (const Layer& L : m->layers) act = act && gemm_tc_swiglu(L.gate_up_il->dev(), rows);
+    const size_t gu = std::max({n * (act ? 1 : 2) * I, act ? (size_t)128 * I : 0, m->multi_basis ? n * H : 0});
     struct { void** p; size_t bytes; void* fresh; } bufs[] = {
         {(void**)&m->pf_tokens, n * sizeof(int32_t)}, {(void**)&m->pf_h, n * H * sizeof(float)}, {(void**)&m->pf_qkv, n * qw * sizeof(float)},
-        {(void**)&m->pf_att, n * H * sizeof(float)}, {(void**)&m->pf_gu, n * gu * sizeof(float)},
+        {(void**)&m->pf_att, n * H * sizeof(float)}, {(void**)&m->pf_gu, gu * sizeof(float)},
         {(void**)&m->pf_qtc, gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)}, {(void**)&m->pf_sx, n * sizeof(float)},
         {(void**)&m->pf_qs, c.arch == 1 ? n * m->nh_l * sizeof(float) : 0}, {(void**)&m->pf_qsum, n * sizeof(int32_t)}};
     auto drop = [&]() -> cudaError_t {

@@ -369,3 +369,27 @@ def test_prompt_without_memory_for_the_large_pass(bt, syn):
     assert np.array_equal(a.prefill(tokens)[0], want) and np.array_equal(b.prefill(tokens)[0], want)
     assert free_bytes() == before
     assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("n,nxt", [(65, 64), (128, 63), (200, 9), (10, 64)])
+def test_pieces_on_both_sides_of_64_rows(bt, oracle, syn, n, nxt):
+    # the buffer of a piece that stores silu(gate) * up holds gate and up rows of a shorter piece behind it
+    cfg = syn.BitLlamaConfig("llama", 64, 256, 2, 4, 2, 1040, max_position_embeddings=300)
+    w = syn.make_weights(cfg, seed=n, from_latent=False)
+    gpu, ref = syn.build_model(w), oracle.model_from_weights(w)
+    states, rng = [ref.new_state()], np.random.default_rng(n)
+    for piece in (n, nxt):
+        staged_prefill(oracle, ref, gpu, cfg, rng.integers(0, 64, size=(1, piece)), states)
+    assert bt.lib().bt_device_check(0) == 0
+
+
+def test_memory_of_a_long_prompt(bt, syn):
+    import torch
+    cfg = syn.BitLlamaConfig("llama", 64, 512, 1, 8, 2, 8192, max_position_embeddings=4096)
+    m = syn.build_model(syn.make_weights(cfg, seed=1, from_latent=False), max_batch=2)
+    m.prefill(np.zeros((2, 70), np.int64))  # (kernels are loaded)
+    m.reset_kv_cache()
+    before = torch.cuda.mem_get_info()[0]
+    m.prefill(np.zeros((2, 4096), np.int64))
+    rows = 8192 * (4 * (512 + 768 + 512 + 8192) + 8192 + 16 + 32)  # stream, q|k|v, attention, silu(gate) * up, int8, scales
+    assert before - torch.cuda.mem_get_info()[0] <= rows + (32 << 20)
