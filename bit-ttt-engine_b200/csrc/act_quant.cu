@@ -1,5 +1,6 @@
 // Per-token absmax int8 activation quantiser: s = max|x|/127, q = clamp(round(x*(127/max|x|))),
-// round half away from zero, s == 0 -> q = 0.  The reference has no such kernel; the
+// round half away from zero, s == 0 -> q = 0, and so for products that are no numbers: a
+// zero beside a 127/max|x| that overflows, or a value of x that is none.  The reference has no such kernel; the
 // definition follows its Q8 KV-cache quantiser (layers/kv_cache.rs:95-119) without the
 // zero point.  One CTA per token; x is read twice (the second pass hits L2).
 #include "bt_common.cuh"
@@ -42,8 +43,7 @@ __device__ __forceinline__ int block_sum_i32(int v, int* red) {
 __device__ __forceinline__ int quant_one(float x, float inv) {
     // one f32 multiply by 127/amax and round-half-away, so the CPU restatement reproduces every q
     float r = roundf(__fmul_rn(x, inv));
-    r = fminf(fmaxf(r, -127.0f), 127.0f);
-    return (int)r;
+    return r != r ? 0 : (int)fminf(fmaxf(r, -127.0f), 127.0f);
 }
 
 template <typename T>

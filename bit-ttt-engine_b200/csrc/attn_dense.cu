@@ -907,8 +907,8 @@ int pad8(int n) { return (n + 7) / 8 * 8; }
 // 16.4 and 17.4, 512 20.3 and 18.8; of 192 + 128, 128 rows 17.4 and 18.4, 256 26.1 and 18.3.
 // (With the softmax unrolled; rolled up these tiles take 9 to 28 % less, 640 rows of 32 heads of 64 21.9, and both kernels are close
 // together somewhat below the lines, which are on the safe side.)
-bool attn_flash_pays(const DenseAttn& a) {
-    return attn_flash_fits(a) && a.q_rows >= (a.kv.k_stride <= 64 ? 640 : (a.kv.k_stride <= 128 ? 448 : 192));
+bool attn_flash_pays(const DenseAttn& a, bool latent) {
+    return a.q_rows >= (a.kv.k_stride <= 64 ? 640 : (a.kv.k_stride <= 128 ? 448 : 192)) && attn_flash_fits(a, latent);
 }
 
 }  // namespace
@@ -935,7 +935,7 @@ bool attn_tile_fits(const DenseAttn& a) { return !a.kv.f32 && a.kv.k_stride <= 2
 
 cudaError_t launch_attn_tile(const DenseAttn& a, const ActOut& out, cudaStream_t s) {
     if (!attn_tile_fits(a) || !a.q_bf16 || !out.tiles) return cudaErrorInvalidValue;
-    if (attn_flash_pays(a)) return launch_attn_flash(a, nullptr, out, s);
+    if (attn_flash_pays(a, false)) return launch_attn_flash(a, nullptr, out, s);
     return tile_launch_k<false>(a, LatentTile(), out, s);
 }
 
@@ -953,7 +953,7 @@ cudaError_t launch_latent_tile(const LatentAttn& l, const __nv_bfloat16* kv16, i
     t.latent = l.kv; t.b0 = b0;
     t.gate = l.gate ? l.proj + l.heads * (l.dim + l.rot) + l.rank + l.rot : nullptr;
     t.gate_ld = l.ld;
-    if (attn_flash_pays(a)) return launch_attn_flash(a, &t, out, s);
+    if (attn_flash_pays(a, true)) return launch_attn_flash(a, &t, out, s);
     return tile_launch_k<true>(a, t, out, s);
 }
 

@@ -43,7 +43,7 @@ struct LatentTile {
 };
 
 // The tcgen05 form (attn_flash.cu); latent: lt describes keys and values, else the cache in a.kv does.
-bool attn_flash_fits(const DenseAttn& a);
+bool attn_flash_fits(const DenseAttn& a, bool latent);
 cudaError_t launch_attn_flash(const DenseAttn& a, const LatentTile* lt, const ActOut& out, cudaStream_t s);
 
 }  // namespace bt

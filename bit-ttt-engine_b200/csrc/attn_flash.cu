@@ -67,9 +67,11 @@ struct FlashSmem {  // behind the operands
     uint32_t tmem;
 };
 // Operands: [16-byte piece of a row][row] 16 bytes, a core matrix (8 rows) is 128 contiguous bytes
-__host__ __device__ inline size_t flash_bytes(int k_steps, int v_steps) {
+__host__ __device__ constexpr size_t flash_bytes(int k_steps, int v_steps) {
     return (size_t)(3 * k_steps + 2 * v_steps) * 2 * kFlashKeys * 16;
 }
+constexpr int kFlashSmemMost = 227 * 1024;
+static_assert(flash_bytes(kFlashMaxK / 16, kFlashMaxV / 16) + sizeof(FlashSmem) <= kFlashSmemMost, "the largest heads fit shared memory");
 
 template <bool LATENT, bool CAP>
 __global__ void __launch_bounds__(kFlashThreads, 1) attn_flash_kernel(const DenseAttn a, const LatentTile lt, const ActOut out) {
@@ -353,20 +355,24 @@ __global__ void __launch_bounds__(kFlashThreads, 1) attn_flash_kernel(const Dens
     if (warp == kMmaWarp) ptx::tmem_dealloc(tmem, 512);
 }
 
+// What a launch needs of the kernel, once per device.
 template <bool LATENT, bool CAP>
-cudaError_t flash_launch(const DenseAttn& a, const LatentTile& lt, const ActOut& out, cudaStream_t s) {
+cudaError_t flash_ready() {
     static PerDeviceOnce once;
-    constexpr size_t most = 227 * 1024;
-    cudaError_t e = once.run([] {
-        cudaError_t r = cudaFuncSetAttribute(attn_flash_kernel<LATENT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    return once.run([] {
+        cudaError_t e = cudaFuncSetAttribute(attn_flash_kernel<LATENT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlashSmemMost);
         // (a share beyond what the launch gives the CTA would be waited for without end)
         cudaFuncAttributes fa;
-        if (r == cudaSuccess) r = cudaFuncGetAttributes(&fa, attn_flash_kernel<LATENT, CAP>);
-        return r == cudaSuccess && fa.numRegs * kFlashThreads < kRegsShares ? cudaErrorLaunchOutOfResources : r;
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, attn_flash_kernel<LATENT, CAP>);
+        if (e != cudaSuccess) (void)cudaGetLastError();  // (answered by the caller, not by the next launch)
+        return e == cudaSuccess && fa.numRegs * kFlashThreads < kRegsShares ? cudaErrorLaunchOutOfResources : e;
     });
+}
+template <bool LATENT, bool CAP>
+cudaError_t flash_launch(const DenseAttn& a, const LatentTile& lt, const ActOut& out, cudaStream_t s) {
+    const cudaError_t e = flash_ready<LATENT, CAP>();
     if (e != cudaSuccess) return e;
     const size_t smem = flash_bytes((a.kv.k_stride + 15) / 16, (a.kv.v_stride + 15) / 16) + sizeof(FlashSmem);
-    if (smem > most) return cudaErrorInvalidConfiguration;
     attn_flash_kernel<LATENT, CAP><<<dim3((unsigned)a.heads, (unsigned)((a.q_rows + kFlashQ - 1) / kFlashQ), (unsigned)a.batch), kFlashThreads, smem, s>>>(a, lt, out);
     return cudaGetLastError();
 }
@@ -374,13 +380,16 @@ cudaError_t flash_launch(const DenseAttn& a, const LatentTile& lt, const ActOut&
 }  // namespace
 
 // Heads whose operands fit shared memory (three tiles of keys' width, two of values') and whose two accumulators fit tensor
-// memory; positive scales (the softmax takes the largest raw score for the largest score).
-bool attn_flash_fits(const DenseAttn& a) {
-    return !a.kv.f32 && a.kv.k_stride <= kFlashMaxK && a.kv.v_stride <= kFlashMaxV && a.scale > 0.0f;
+// memory; positive scales (the softmax takes the largest raw score for the largest score); a build whose kernel has the
+// registers that its warpgroups share out.
+bool attn_flash_fits(const DenseAttn& a, bool latent) {
+    if (a.kv.f32 || a.kv.k_stride > kFlashMaxK || a.kv.v_stride > kFlashMaxV || !(a.scale > 0.0f)) return false;
+    const bool cap = a.softcap > 0.0f;
+    return (latent ? (cap ? flash_ready<true, true>() : flash_ready<true, false>()) : (cap ? flash_ready<false, true>() : flash_ready<false, false>())) == cudaSuccess;
 }
 
 cudaError_t launch_attn_flash(const DenseAttn& a, const LatentTile* lt, const ActOut& out, cudaStream_t s) {
-    if (!attn_flash_fits(a) || !a.q_bf16 || !out.tiles) return cudaErrorInvalidValue;
+    if (!attn_flash_fits(a, lt != nullptr) || !a.q_bf16 || !out.tiles) return cudaErrorInvalidValue;
     const bool cap = a.softcap > 0.0f;
     if (lt) return cap ? flash_launch<true, true>(a, *lt, out, s) : flash_launch<true, false>(a, *lt, out, s);
     return cap ? flash_launch<false, true>(a, LatentTile(), out, s) : flash_launch<false, false>(a, LatentTile(), out, s);

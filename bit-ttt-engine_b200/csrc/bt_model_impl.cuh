@@ -99,6 +99,7 @@ struct bt_model {
     int trace_rows = 0;              // rows per tensor the trace buffer was sized for
     // prefill scratch (allocated at the first bt_model_prefill, for pf_rows = sequences x tokens of a chunk)
     int pf_rows = 0;
+    bool pf_least = false;           // there was no memory for a large pass
     int32_t* pf_tokens = nullptr;
     float* pf_h = nullptr;
     float* pf_qkv = nullptr;

@@ -83,7 +83,8 @@ __device__ __forceinline__ int quant_store_group(const float (&v)[16], float inv
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         // |x| <= max|x| makes |x * inv| <= 127 up to two roundings, so the rounded values lie in
-        // [-127, 127] and the saturating pack to signed bytes never changes one
+        // [-127, 127] and the saturating pack to signed bytes never changes one (but where 127/max|x| overflows:
+        // values below 4e-37, of which it leaves -128, 0 or 127)
         int qv[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) qv[r] = ptx::round_half_away(__fmul_rn(v[4 * b + r], inv));
@@ -115,9 +116,9 @@ __device__ __forceinline__ int quant_store_half(const float (&v)[8], float inv, 
     return sum;
 }
 
-// The definition of the quantiser to the letter (act_quant.cu), values that are no numbers included: they become -127, and so
-// do products with an infinite 127 / max|x| that are none.
-__device__ __forceinline__ float clamp127(float v) { return fminf(fmaxf(v, -127.0f), 127.0f); }
+// What a product with 127 / max|x| must not exceed before quant_store_group: that overflows for rows of tiny values, and the pack
+// would leave -128 then.  (A product that is no number passes, and becomes 0.)
+__device__ __forceinline__ float clamp127(float v) { return v < -127.0f ? -127.0f : v; }
 
 __device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&v)[16]) {
 #pragma unroll

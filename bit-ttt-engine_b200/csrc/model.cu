@@ -4,6 +4,7 @@
 // all arithmetic is in the kernels.
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "bt_model_impl.cuh"
@@ -626,7 +627,8 @@ extern "C" bt_status bt_model_finalize(bt_model* m) {
     BT_CUDA_TRY(dev_alloc(&m->q, (size_t)B * m->q_stride));
     BT_CUDA_TRY(dev_alloc(&m->sx, (size_t)B));
     BT_CUDA_TRY(dev_alloc(&m->qsum, (size_t)B));
-    BT_CUDA_TRY(dev_alloc(&m->gu, (size_t)B * 2 * I));
+    // (gate and up rows; the products on their own of bt_model_enqueue_products, all four kinds of them)
+    BT_CUDA_TRY(dev_alloc(&m->gu, (size_t)B * std::max<int64_t>({2ll * I, (int64_t)H, (int64_t)m->qkv_dim})));
     BT_CUDA_TRY(dev_alloc(&m->xn, (size_t)B * H));
     BT_CUDA_TRY(dev_alloc(&m->act, (size_t)B * I));
     if (B > 8) {
@@ -831,7 +833,7 @@ namespace {
 
 // Rows (sequences x tokens) that one prefill pass works on.  Ternary models: with 2048 rows the products of a 2048-wide model have
 // 64 to 160 tiles for 74 CTA pairs, and every pass ends in a wait of the host (16 prompts of 511 tokens, 1B: 5 156 us in passes
-// of 2048, 3 874 in one).  Layer-list models keep more buffers a row, and a ternary model without the memory for 8192 (1.5 GB
+// of 2048, 3 874 in one).  Layer-list models keep more buffers a row, and a ternary model without the memory for 8192 (1.1 GB
 // at 4096 x 14336) works on 2048 as well.
 constexpr int kPrefillRows = 8192, kPrefillRowsLeast = 2048;
 
@@ -839,23 +841,35 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     if (m->lay) return layered_prefill_buffers(m, rows);
     if (rows <= m->pf_rows) return BT_OK;
     const bt_model_config& c = m->cfg;
-    const int64_t H = c.hidden_dim, I = m->i_l;
+    const int64_t H = c.hidden_dim, I = m->i_l, kmax = H > I ? H : I;
     const int64_t qw = c.arch == 1 ? m->qkv_dim : m->d_small;  // q|k|v, or the TTT features and predictions (two slots)
-    BT_CUDA_TRY(cudaDeviceSynchronize());
-    auto drop = [](auto*& p) { cudaFree(p); p = nullptr; };
-    drop(m->pf_tokens); drop(m->pf_h); drop(m->pf_qkv); drop(m->pf_att); drop(m->pf_gu); drop(m->pf_qtc);
-    drop(m->pf_sx); drop(m->pf_qsum); drop(m->pf_qs);
-    m->pf_rows = 0;
-    const int64_t kmax = H > I ? H : I;
-    BT_CUDA_TRY(dev_alloc(&m->pf_tokens, (size_t)rows));
-    BT_CUDA_TRY(dev_alloc(&m->pf_h, (size_t)rows * H));
-    BT_CUDA_TRY(dev_alloc(&m->pf_qkv, (size_t)rows * qw));
-    BT_CUDA_TRY(dev_alloc(&m->pf_att, (size_t)rows * H));
-    BT_CUDA_TRY(dev_alloc(&m->pf_gu, (size_t)rows * 2 * I));
-    BT_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&m->pf_qtc), gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)));
-    BT_CUDA_TRY(dev_alloc(&m->pf_sx, (size_t)rows));
-    if (c.arch == 1) BT_CUDA_TRY(dev_alloc(&m->pf_qs, (size_t)rows * m->nh_l));
-    BT_CUDA_TRY(dev_alloc(&m->pf_qsum, (size_t)rows));
+    const size_t n = (size_t)rows;
+    // Gate and up rows, or silu(gate) * up where the product leaves that (more than 64 rows: 470 MB instead of 940 for 8192 x 14336); with
+    // several bases a projection's sum as well.
+    bool act = true;
+    for (const Layer& L : m->layers) act = act && gemm_tc_swiglu(L.gate_up_il->dev(), rows);
+    const size_t gu = std::max({n * (act ? 1 : 2) * I, act ? (size_t)128 * I : 0, m->multi_basis ? n * H : 0});
+    struct { void** p; size_t bytes; void* fresh; } bufs[] = {
+        {(void**)&m->pf_tokens, n * sizeof(int32_t)}, {(void**)&m->pf_h, n * H * sizeof(float)}, {(void**)&m->pf_qkv, n * qw * sizeof(float)},
+        {(void**)&m->pf_att, n * H * sizeof(float)}, {(void**)&m->pf_gu, gu * sizeof(float)},
+        {(void**)&m->pf_qtc, gemm_tc_act_bytes(rows, (kmax + kTileK - 1) / kTileK)}, {(void**)&m->pf_sx, n * sizeof(float)},
+        {(void**)&m->pf_qs, c.arch == 1 ? n * m->nh_l * sizeof(float) : 0}, {(void**)&m->pf_qsum, n * sizeof(int32_t)}};
+    auto drop = [&]() -> cudaError_t {
+        const cudaError_t e = cudaDeviceSynchronize();
+        for (auto& b : bufs) { cudaFree(*b.p); *b.p = nullptr; }
+        m->pf_rows = 0;
+        return e;
+    };
+    // A large pass comes beside the buffers that there are, so that a model without the memory for it keeps what it works with.
+    const bool beside = rows > kPrefillRowsLeast;
+    cudaError_t e = beside ? cudaSuccess : drop();
+    for (auto& b : bufs)
+        if (e == cudaSuccess && b.bytes) e = cudaMalloc(&b.fresh, b.bytes);
+    if (e == cudaSuccess && beside) e = drop();
+    if (e != cudaSuccess)
+        for (auto& b : bufs) cudaFree(b.fresh);
+    BT_CUDA_TRY(e);
+    for (auto& b : bufs) *b.p = b.fresh;
     m->pf_rows = rows;
     return BT_OK;
 }
@@ -989,11 +1003,12 @@ bt_status prefill_impl(bt_model* m, const int32_t* tokens_host, int batch, int n
         if (c.arch == 0 && per < n_tokens && per > ttt_chunk) per -= per % ttt_chunk;
         if (m->trace && (int64_t)batch * per > m->trace_rows) per = m->trace_rows / batch;
     };
-    cut(m->lay ? kPrefillRowsLeast : kPrefillRows);
+    cut(m->lay || m->pf_least ? kPrefillRowsLeast : kPrefillRows);
     if (per < 1) return set_error(BT_ERR_NOMEM, "bt_model_prefill: the trace buffer holds fewer rows than sequences");
     bt_status st = prefill_buffers(m, batch * per);
     if (st != BT_OK && batch * per > kPrefillRowsLeast) {
         cudaGetLastError();  // (an allocation that failed leaves the context as it was)
+        m->pf_least = true;  // (not tried again: every call would wait for the device and allocate)
         cut(kPrefillRowsLeast);
         st = prefill_buffers(m, batch * per);
     }

@@ -265,6 +265,7 @@ EXPORT void oracle_act_quant(const float* x, int64_t m, int64_t k, int8_t* q, fl
                 r = roundf(xr[l] * inv);
                 if (r > 127.0f) r = 127.0f;
                 if (r < -127.0f) r = -127.0f;
+                if (r != r) r = 0.0f;  /* a zero times an infinite 127/max|x| */
             }
             q[i * k + l] = (int8_t)r;
             sum += (int32_t)r;

@@ -327,3 +327,21 @@ def test_row_quantisers_of_tiny_rows(bt, oracle):
     x[250] = np.where(np.arange(k) % 3, 1e-40, -2e-40)
     lin = bt.BitLinear.from_packed(packed, [0.5], n, k)
     assert np.array_equal(lin.forward(torch.from_numpy(x).cuda()).cpu().numpy(), oracle.bitlinear_q(x, packed, [0.5], n))
+
+
+@pytest.mark.parametrize("m", [1, 3, 4, 8, 9, 65, 300])  # every quantiser
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_zeros_of_tiny_rows_stay_zeros(bt, oracle, m, dtype):
+    # 127 / max|x| overflows, and a zero times infinity is no number
+    n, k = 48, 1024
+    rng = np.random.default_rng(6)
+    packed = ternary_packed(rng, n, k)
+    x = np.where(rng.random((m, k)) < 0.5, 0, rng.choice([-1, 1], (m, k)) * 2.0 ** -130).astype(np.float32)
+    x = torch.from_numpy(x).to(getattr(torch, dtype))
+    lin = bt.BitLinear.from_packed(packed, [0.5], n, k)
+    ref = torch.from_numpy(oracle.bitlinear_q(x.float().numpy(), packed, [0.5], n)).to(x.dtype)
+    assert torch.equal(lin.forward(x.cuda()).cpu(), ref)
+    q, _, qsum = bt.act_quant(x.cuda())
+    assert torch.equal(q.cpu() == 0, x == 0) and torch.equal(qsum.cpu(), q.cpu().sum(1, dtype=torch.int32))
+    if dtype == "float32":
+        assert np.array_equal(q.cpu().numpy(), oracle.act_quant(x.numpy())[0])

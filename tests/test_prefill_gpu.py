@@ -303,6 +303,18 @@ def test_prefill_silu_in_the_product(bt, oracle, syn, hidden, ff, batch, n):
     assert bt.lib().bt_device_check(0) == 0
 
 
+@pytest.mark.parametrize("arch,n", [("llama", 40), ("llama", 100), ("ttt", 100)])
+def test_prefill_of_several_bases_and_a_narrow_mlp(bt, oracle, syn, arch, n):
+    # the sum of a projection's bases is wider than the gate and up rows whose buffer it borrows
+    cfg = syn.BitLlamaConfig(arch, 64, 512, 2, 8, 4 if arch == "llama" else 8, 64, inner_lr=0.01, max_position_embeddings=256)
+    w = syn.make_weights(cfg, seed=n, n_bases=2)
+    gpu, ref = syn.build_model(w, max_batch=2), oracle.model_from_weights(w)
+    states = [ref.new_state() for _ in range(2)]
+    staged_prefill(oracle, ref, gpu, cfg, np.random.default_rng(n).integers(0, 64, size=(2, n)), states)
+    gpu.enqueue_products(2)  # (the other caller of such a buffer)
+    assert bt.lib().bt_device_check(0) == 0
+
+
 def test_prompts_of_more_rows_than_one_pass(bt, syn):
     # a call of more rows than the prefill works on at a time is cut by the host: the same as calls that fit one
     # pass each - bit for bit without attention, in the first layer's cache with it
@@ -328,3 +340,56 @@ def test_prompts_of_more_rows_than_one_pass(bt, syn):
     # its row's largest: a few such steps over two layers)
     assert rel_err(la, lb) <= 5e-2
     assert bt.lib().bt_device_check(0) == 0
+
+
+def test_prompt_without_memory_for_the_large_pass(bt, syn):
+    # a model that cannot have the buffers of a large pass works in small ones, keeps those it has, and does not ask again
+    cfg = syn.BitLlamaConfig("llama", 500, 1024, 1, 8, 2, 4096, max_position_embeddings=1700)  # 350 MB for 6800 rows, 105 for 2048
+    w = syn.make_weights(cfg, seed=6602, from_latent=False)
+    import torch
+    free_bytes = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    tokens = np.random.default_rng(18).integers(0, 500, size=(4, 1700))
+    a, b, pieces = (syn.build_model(w, max_batch=4) for _ in range(3))
+    for i in range(0, 1700, 512):  # what passes of 2048 rows are
+        want, _ = pieces.prefill(tokens[:, i:i + 512])
+    b.prefill(tokens[:, :512])
+    b.reset_kv_cache()
+    torch.cuda.empty_cache()
+    filler = torch.empty(free_bytes() - (250 << 20), dtype=torch.uint8, device="cuda")  # (b has the buffers of a small pass already)
+    before = free_bytes()
+    for _ in range(2):
+        assert np.array_equal(b.prefill(tokens)[0], want)
+        assert free_bytes() == before
+        b.reset_kv_cache()
+    assert np.array_equal(a.prefill(tokens)[0], want)
+    a.reset_kv_cache()
+    del filler
+    torch.cuda.empty_cache()
+    before = free_bytes()
+    assert np.array_equal(a.prefill(tokens)[0], want) and np.array_equal(b.prefill(tokens)[0], want)
+    assert free_bytes() == before
+    assert bt.lib().bt_device_check(0) == 0
+
+
+@pytest.mark.parametrize("n,nxt", [(65, 64), (128, 63), (200, 9), (10, 64)])
+def test_pieces_on_both_sides_of_64_rows(bt, oracle, syn, n, nxt):
+    # the buffer of a piece that stores silu(gate) * up holds gate and up rows of a shorter piece behind it
+    cfg = syn.BitLlamaConfig("llama", 64, 256, 2, 4, 2, 1040, max_position_embeddings=300)
+    w = syn.make_weights(cfg, seed=n, from_latent=False)
+    gpu, ref = syn.build_model(w), oracle.model_from_weights(w)
+    states, rng = [ref.new_state()], np.random.default_rng(n)
+    for piece in (n, nxt):
+        staged_prefill(oracle, ref, gpu, cfg, rng.integers(0, 64, size=(1, piece)), states)
+    assert bt.lib().bt_device_check(0) == 0
+
+
+def test_memory_of_a_long_prompt(bt, syn):
+    import torch
+    cfg = syn.BitLlamaConfig("llama", 64, 512, 1, 8, 2, 8192, max_position_embeddings=4096)
+    m = syn.build_model(syn.make_weights(cfg, seed=1, from_latent=False), max_batch=2)
+    m.prefill(np.zeros((2, 70), np.int64))  # (kernels are loaded)
+    m.reset_kv_cache()
+    before = torch.cuda.mem_get_info()[0]
+    m.prefill(np.zeros((2, 4096), np.int64))
+    rows = 8192 * (4 * (512 + 768 + 512 + 8192) + 8192 + 16 + 32)  # stream, q|k|v, attention, silu(gate) * up, int8, scales
+    assert before - torch.cuda.mem_get_info()[0] <= rows + (32 << 20)
