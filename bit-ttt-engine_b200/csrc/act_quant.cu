@@ -42,8 +42,9 @@ __device__ __forceinline__ int block_sum_i32(int v, int* red) {
 
 __device__ __forceinline__ int quant_one(float x, float inv) {
     // one f32 multiply by 127/amax and round-half-away, so the CPU restatement reproduces every q
-    float r = roundf(__fmul_rn(x, inv));
-    return r != r ? 0 : (int)fminf(fmaxf(r, -127.0f), 127.0f);
+    // (the conversion saturates, and makes 0 of what is no number; a comparison of r with itself in front of a float clamp took
+    // 6 x 13220 -> 421 from 15.6 to 17.7 us)
+    return max(-127, min(127, __float2int_rz(roundf(__fmul_rn(x, inv)))));
 }
 
 template <typename T>
