@@ -105,10 +105,14 @@ struct TcArgs {
 // NT: tokens per tile (64 / 128).  RS: 128-row sets per tile (1 / 2).  S: CTAs of a cluster that share a tile
 // along k (1: no cluster work at all).
 // PAIR: the cluster is a CTA pair that works on one tile of 256 rows x 256 tokens (see kPairTokens).
-template <int NT, int RS, int S, bool PAIR>
+// SEVERAL: a.bases bases in this launch, one behind the other.  An instantiation of its own: with both epilogues in one kernel a
+// product of a single basis had 88 to 128 registers a thread instead of 83 to 108, and the quantiser in front of it no longer
+// fitted beside its CTA, which starts under it (64 tokens of the 8B shapes with their quantisers: 2 241 us a step, now 2 181).
+template <int NT, int RS, int S, bool PAIR, bool SEVERAL>
 __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(TcArgs a) {
     static_assert(S == 1 || (NT == 64 && (S == 2 || S == 4 || S == 8)), "k split: 64 tokens, 2 / 4 / 8 CTAs");
     static_assert(!PAIR || (NT == 128 && RS == 1 && S == 1), "a CTA of a pair: 128 rows and the activations of 128 tokens");
+    static_assert(!SEVERAL || NT == 64, "larger products fill the GPU basis by basis");
     // Eight unpack warps.  RS = 2: one per (row set, TMEM lane quarter).  RS = 1: two per lane quarter, which take
     // the chunks in turn (two independent chains of load - unpack - store, four A buffers).
     constexpr int kUnpackWarps = 8, kEpiWarps = PAIR ? 8 : 4 * RS, kUnpackWarp0 = tc_lead_warps(PAIR ? 2 : RS), kEpiWarp0 = kUnpackWarp0 + kUnpackWarps;
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
     const int cid = blockIdx.x / kCtas, n_clusters = gridDim.x / kCtas;
     const int cps = (k_tiles + S - 1) / S;                 // chunks per split (the host makes every split non-empty)
     const int kt0 = PAIR ? 0 : rank * cps, kt1 = min(k_tiles, kt0 + cps);
-    const int bases = NT == 64 ? a.bases : 1;              // a tile's bases are worked through like tiles of their own
+    const int bases = SEVERAL ? a.bases : 1;               // a tile's bases are worked through like tiles of their own
     const int n_tiles = row_sets * tok_blocks;             // this CTA works on the tiles cid, cid + n_clusters, ...
     // this CTA's row tiles of a tile begin at row_tile0(rs): rts(rs) of them exist (none, where the matrix ends in the first half)
     auto row_tile0 = [&](int rs) -> int64_t { return (int64_t)rs * (8 * kTileSets) + (PAIR ? 8 * rank : 0); };
@@ -374,18 +378,20 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         // The epilogue kind is a compile-time constant of everything below (one copy of the role per kind, chosen once):
         // the unrolled store sequences are long, and a kind switch inside every element made them four times as long -
         // code that is fetched once per tile and does not stay in the instruction cache.
-        // MULTI: several bases, added up in basis order in f32 rows (the output, or aside before a bf16 output); the thread that
+        // Several bases are added up in basis order in f32 rows (the output, or aside before a bf16 output); the thread that
         // adds a basis is the one that stored the one before.
-        auto epilogue_role = [&](auto kind, auto multi) {
+        auto epilogue_role = [&](auto kind) {
         constexpr int EPI = decltype(kind)::value;
-        constexpr bool MULTI = decltype(multi)::value;
-        constexpr bool accum = MULTI || EPI == EPI_F32_ACCUM || EPI == kEpiBf16Accum;
+        constexpr bool accum = SEVERAL || EPI == EPI_F32_ACCUM || EPI == kEpiBf16Accum;
         int basis = 0;
         auto load_old = [&](int token, int64_t row) -> float {
-            const int64_t o = (int64_t)token * a.out_stride + row;
-            if (!accum || token >= a.m || row >= a.n_out) return 0.0f;
-            if constexpr (MULTI) return basis == 0 ? 0.0f : (EPI == EPI_BF16 ? a.sum[o] : reinterpret_cast<const float*>(a.out)[o]);
-            else return a.acc_in[o];
+            if constexpr (SEVERAL) {
+                const int64_t o = (int64_t)token * a.out_stride + row;
+                if (basis == 0 || token >= a.m || row >= a.n_out) return 0.0f;
+                return EPI == EPI_BF16 ? a.sum[o] : reinterpret_cast<const float*>(a.out)[o];
+            } else {
+                return (accum && token < a.m && row < a.n_out) ? a.acc_in[(int64_t)token * a.out_stride + row] : 0.0f;
+            }
         };
         // i = token inside the tile; tq / ts = the tile's staged per-token terms
         // tqi / tsi: the token's sum of q and scale (read from shared memory by the caller, ahead of its stores)
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                     reinterpret_cast<int32_t*>(a.out)[o] = accv;
                 } else {
                     const float y = __fmul_rn(__fmul_rn((float)accv, sw), tsi);
-                    if constexpr (MULTI) {
+                    if constexpr (SEVERAL) {
                         const float v = basis == 0 ? y : __fadd_rn(old, y);
                         if (EPI == EPI_F32) reinterpret_cast<float*>(a.out)[o] = v;
                         else if (basis + 1 < a.bases) a.sum[o] = v;
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
         };
         int tl = 0;
         for (int tile = cid; tile < n_tiles; tile += n_clusters)
-        for (basis = 0; basis < (MULTI ? a.bases : 1); ++basis, ++tl) {
+        for (basis = 0; basis < bases; ++basis, ++tl) {
             const int rs = tile % row_sets, tb = tile / row_sets;
             const int sel = tl % kAccSets;
             // the tile's per-token terms, once per row set's four warps into shared memory (named barrier 1 + h)
@@ -630,22 +636,17 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
             }
         }
         };
-        constexpr std::false_type one{};
-        if constexpr (NT == 64) {
-            constexpr std::true_type several{};
-            if (a.bases > 1) {
-                if (a.epilogue == EPI_F32) epilogue_role(std::integral_constant<int, EPI_F32>{}, several);
-                else epilogue_role(std::integral_constant<int, EPI_BF16>{}, several);
-            }
-        }
-        if (bases == 1) {
+        if constexpr (SEVERAL) {
+            if (a.epilogue == EPI_F32) epilogue_role(std::integral_constant<int, EPI_F32>{});
+            else epilogue_role(std::integral_constant<int, EPI_BF16>{});
+        } else {
             switch (a.epilogue) {
-                case EPI_I32: epilogue_role(std::integral_constant<int, EPI_I32>{}, one); break;
-                case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}, one); break;
-                case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}, one); break;
-                case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}, one); break;
-                case EPI_SWIGLU: if constexpr (NT == 128) epilogue_role(std::integral_constant<int, EPI_SWIGLU>{}, one); break;
-                default: epilogue_role(std::integral_constant<int, EPI_BF16>{}, one); break;
+                case EPI_I32: epilogue_role(std::integral_constant<int, EPI_I32>{}); break;
+                case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}); break;
+                case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}); break;
+                case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}); break;
+                case EPI_SWIGLU: if constexpr (NT == 128) epilogue_role(std::integral_constant<int, EPI_SWIGLU>{}); break;
+                default: epilogue_role(std::integral_constant<int, EPI_BF16>{}); break;
             }
         }
     }
@@ -678,13 +679,13 @@ struct TcVariant {
     cudaError_t status = cudaErrorNotReady;
 };
 
-template <int NT, int RS, int S, bool PAIR = false>
+template <int NT, int RS, int S, bool PAIR = false, bool SEVERAL = false>
 const TcVariant& tc_variant(int sm_count) {
     static TcVariant v;              // cluster limit: once per process (every device of a process is the same GPU model)
     static PerDeviceOnce attributes;  // the kernel's shared-memory limit: once per device
     constexpr int kCtas = PAIR ? 2 : S, kThreads = tc_threads(PAIR ? 2 : RS);
     v.smem = (size_t)tc_stages(NT, RS, S) * (RS * kSetBytes + 4 * NT * 64) + (S > 1 ? RS * kRows * NT * 4 : 0) + 512 + (PAIR ? 32 : 16) * NT;
-    auto* kernel = gemm_tc_kernel<NT, RS, S, PAIR>;
+    auto* kernel = gemm_tc_kernel<NT, RS, S, PAIR, SEVERAL>;
     const size_t smem = v.smem;
     v.status = attributes.run([kernel, smem] {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -721,9 +722,9 @@ const TcVariant& tc_variant(int sm_count) {
     return v;
 }
 
-template <int NT, int RS, int S, bool PAIR = false>
+template <int NT, int RS, int S, bool PAIR = false, bool SEVERAL = false>
 cudaError_t launch_variant(TcArgs a, int sm_count, cudaStream_t stream) {
-    const TcVariant& v = tc_variant<NT, RS, S, PAIR>(sm_count);
+    const TcVariant& v = tc_variant<NT, RS, S, PAIR, SEVERAL>(sm_count);
     if (v.status != cudaSuccess) return v.status;
     constexpr int kCtas = PAIR ? 2 : S, kSets = PAIR ? 2 : RS, kTokens = PAIR ? kPairTokens : NT;
     const int n_tiles = (int)((a.row_tiles + 8 * kSets - 1) / (8 * kSets)) * ((a.m + kTokens - 1) / kTokens);
@@ -740,7 +741,7 @@ cudaError_t launch_variant(TcArgs a, int sm_count, cudaStream_t stream) {
     attr[1].val.clusterDim.x = (unsigned)kCtas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = kCtas > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NT, RS, S, PAIR>, a);
+    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<NT, RS, S, PAIR, SEVERAL>, a);
 }
 
 // Chunk steps on the busiest CTA when a tile's k range is cut over `s` CTAs (one step charged for the exchange of
@@ -753,43 +754,45 @@ int64_t tc_split_cost(int s, int max_clusters, int n_tiles, int64_t k_tiles) {
     return (int64_t)((n_tiles + nc - 1) / nc) * (cps + (s > 1 ? 1 : 0));
 }
 
-cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) {
-    const int tok_blocks = (a.m + nt - 1) / nt;
-    const int n_tiles = (int)((a.row_tiles + 7) / 8) * tok_blocks;          // tiles of 128 rows
-    const int n_tiles2 = (int)((a.row_tiles + 15) / 16) * tok_blocks;       // tiles of 256 rows
-    if (nt == 128) {
-        // Pairs where there are tiles for most SMs and no more rounds of them than of single CTAs' tiles, which are half as large
-        // (257 x 4096 -> 28672 has one more: 59.7 -> 68.7 us).  More than 16384 rows of plain output stay with single CTAs: their
-        // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240);
-        // with SiLU * up, which stores half of that, pairs are ahead again (prefill of 2048 tokens, 8B: 3 242 us and 3 290).
-        const TcVariant& pair = tc_variant<128, 1, 1, true>(sm_count);
-        const int n_pairs = (int)((a.row_tiles + 15) / 16) * ((a.m + kPairTokens - 1) / kPairTokens);
-        // 256-row tiles halve the activation traffic per weight; 128-row tiles when there is too little work for them
-        const int waves2 = (n_tiles2 + sm_count - 1) / sm_count;
-        if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && (a.row_tiles <= 1024 || a.epilogue == EPI_SWIGLU) &&
-            (n_pairs + pair.max_clusters - 1) / pair.max_clusters <= waves2)
-            return launch_variant<128, 1, 1, true>(a, sm_count, stream);
-        return 2 * n_tiles2 >= sm_count ? launch_variant<128, 2, 1>(a, sm_count, stream) : launch_variant<128, 1, 1>(a, sm_count, stream);
-    }
-    // 64 tokens at most.  More 128-row tiles than SMs: 256-row tiles.  Fewer than half: cut k over a cluster so that
-    // one wave of CTAs covers the product.
-    if (n_tiles > sm_count) return launch_variant<64, 2, 1>(a, sm_count, stream);
+// 64 tokens at most.  More 128-row tiles than SMs: 256-row tiles.  Fewer than half: cut k over a cluster so that
+// one wave of CTAs covers the product.
+template <bool SEVERAL>
+cudaError_t launch_product_64(TcArgs a, int sm_count, cudaStream_t stream) {
+    const int n_tiles = (int)((a.row_tiles + 7) / 8);  // tiles of 128 rows
+    if (n_tiles > sm_count) return launch_variant<64, 2, 1, false, SEVERAL>(a, sm_count, stream);
     int best = 1;
     int64_t best_cost = tc_split_cost(1, sm_count, n_tiles, a.k_tiles);
     if (n_tiles * 2 <= sm_count) {
-        const int64_t c2 = tc_split_cost(2, tc_variant<64, 1, 2>(sm_count).max_clusters, n_tiles, a.k_tiles);
-        const int64_t c4 = tc_split_cost(4, tc_variant<64, 1, 4>(sm_count).max_clusters, n_tiles, a.k_tiles);
-        const int64_t c8 = tc_split_cost(8, tc_variant<64, 1, 8>(sm_count).max_clusters, n_tiles, a.k_tiles);
+        const int64_t c2 = tc_split_cost(2, tc_variant<64, 1, 2, false, SEVERAL>(sm_count).max_clusters, n_tiles, a.k_tiles);
+        const int64_t c4 = tc_split_cost(4, tc_variant<64, 1, 4, false, SEVERAL>(sm_count).max_clusters, n_tiles, a.k_tiles);
+        const int64_t c8 = tc_split_cost(8, tc_variant<64, 1, 8, false, SEVERAL>(sm_count).max_clusters, n_tiles, a.k_tiles);
         if (c2 < best_cost) { best = 2; best_cost = c2; }
         if (c4 < best_cost) { best = 4; best_cost = c4; }
         if (c8 < best_cost) { best = 8; best_cost = c8; }
     }
     switch (best) {
-        case 2: return launch_variant<64, 1, 2>(a, sm_count, stream);
-        case 4: return launch_variant<64, 1, 4>(a, sm_count, stream);
-        case 8: return launch_variant<64, 1, 8>(a, sm_count, stream);
-        default: return launch_variant<64, 1, 1>(a, sm_count, stream);
+        case 2: return launch_variant<64, 1, 2, false, SEVERAL>(a, sm_count, stream);
+        case 4: return launch_variant<64, 1, 4, false, SEVERAL>(a, sm_count, stream);
+        case 8: return launch_variant<64, 1, 8, false, SEVERAL>(a, sm_count, stream);
+        default: return launch_variant<64, 1, 1, false, SEVERAL>(a, sm_count, stream);
     }
+}
+
+cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) {
+    if (nt == 64) return a.bases > 1 ? launch_product_64<true>(a, sm_count, stream) : launch_product_64<false>(a, sm_count, stream);
+    const int n_tiles2 = (int)((a.row_tiles + 15) / 16) * ((a.m + nt - 1) / nt);  // tiles of 256 rows
+    // Pairs where there are tiles for most SMs and no more rounds of them than of single CTAs' tiles, which are half as large
+    // (257 x 4096 -> 28672 has one more: 59.7 -> 68.7 us).  More than 16384 rows of plain output stay with single CTAs: their
+    // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240);
+    // with SiLU * up, which stores half of that, pairs are ahead again (prefill of 2048 tokens, 8B: 3 242 us and 3 290).
+    const TcVariant& pair = tc_variant<128, 1, 1, true>(sm_count);
+    const int n_pairs = (int)((a.row_tiles + 15) / 16) * ((a.m + kPairTokens - 1) / kPairTokens);
+    // 256-row tiles halve the activation traffic per weight; 128-row tiles when there is too little work for them
+    const int waves2 = (n_tiles2 + sm_count - 1) / sm_count;
+    if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && (a.row_tiles <= 1024 || a.epilogue == EPI_SWIGLU) &&
+        (n_pairs + pair.max_clusters - 1) / pair.max_clusters <= waves2)
+        return launch_variant<128, 1, 1, true>(a, sm_count, stream);
+    return 2 * n_tiles2 >= sm_count ? launch_variant<128, 2, 1>(a, sm_count, stream) : launch_variant<128, 1, 1>(a, sm_count, stream);
 }
 
 }  // namespace
