@@ -72,6 +72,7 @@ __host__ __device__ constexpr int tc_stages(int nt, int rs, int s) {
 // Per launch, single CTAs -> pairs (us, f32 outputs): 2048 x 14336 -> 4096 129.2 -> 108.3, 4096 tokens 248 -> 202; 2048 x 4096 ->
 // 4096 43.2 -> 40.0, -> 6144 60.6 -> 56.0; 2048 x 5632 -> 2048 31.8 -> 29.6; 2048 x 2048 -> 11264 57.6 -> 57.2.
 constexpr int kPairTokens = 256;
+constexpr int kPairChunks = 8;  // chunks of 256 inputs from which on pairs pay (see launch_product)
 
 // Instruction descriptor for kind::i8: D = s32, A = u8, B = s8, both K-major, M x N tile.
 __device__ __forceinline__ uint32_t instr_desc_i8(int m, int n) {
@@ -107,7 +108,8 @@ struct TcArgs {
 // PAIR: the cluster is a CTA pair that works on one tile of 256 rows x 256 tokens (see kPairTokens).
 // SEVERAL: a.bases bases in this launch, one behind the other.  An instantiation of its own: with both epilogues in one kernel a
 // product of a single basis had 88 to 128 registers a thread instead of 83 to 108, and the quantiser in front of it no longer
-// fitted beside its CTA, which starts under it (64 tokens of the 8B shapes with their quantisers: 2 241 us a step, now 2 181).
+// fitted beside its CTA, which starts under it (64 tokens of the 8B shapes with their quantisers, us a step in runs of two kinds,
+// by where the process' memory lies: 2 167 and 2 264, now 2 118 and 2 198).
 template <int NT, int RS, int S, bool PAIR, bool SEVERAL>
 __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(TcArgs a) {
     static_assert(S == 1 || (NT == 64 && (S == 2 || S == 4 || S == 8)), "k split: 64 tokens, 2 / 4 / 8 CTAs");
@@ -784,12 +786,15 @@ cudaError_t launch_product(TcArgs a, int nt, int sm_count, cudaStream_t stream) 
     // Pairs where there are tiles for most SMs and no more rounds of them than of single CTAs' tiles, which are half as large
     // (257 x 4096 -> 28672 has one more: 59.7 -> 68.7 us).  More than 16384 rows of plain output stay with single CTAs: their
     // stores, 1 KB of a token at a time instead of 512 bytes, disturb the loads less (2048 x 4096 -> 28672 233 us and 240);
-    // with SiLU * up, which stores half of that, pairs are ahead again (prefill of 2048 tokens, 8B: 3 242 us and 3 290).
+    // with SiLU * up, which stores half of that, pairs are ahead again (prefill of 2048 tokens, 8B: 3 242 us and 3 290).  Fewer than 2048
+    // inputs stay with single CTAs too, because a pair's tile ends in 3 000 clocks without MMAs and is twice as large: over 200 to
+    // 4096 tokens and 2048 to 16384 rows pairs take 1.08 to 1.24 of their time for 256 inputs, 1.02 to 1.16 for 768, 0.96 to 1.05 for
+    // 1280 and for 1536, 0.95 to 1.02 for 2048 (but 1354 x 2048 -> 10722: 1.08).
     const TcVariant& pair = tc_variant<128, 1, 1, true>(sm_count);
     const int n_pairs = (int)((a.row_tiles + 15) / 16) * ((a.m + kPairTokens - 1) / kPairTokens);
     // 256-row tiles halve the activation traffic per weight; 128-row tiles when there is too little work for them
     const int waves2 = (n_tiles2 + sm_count - 1) / sm_count;
-    if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && (a.row_tiles <= 1024 || a.epilogue == EPI_SWIGLU) &&
+    if (pair.status == cudaSuccess && pair.max_clusters > 0 && 2 * n_tiles2 >= sm_count && a.k_tiles >= kPairChunks && (a.row_tiles <= 1024 || a.epilogue == EPI_SWIGLU) &&
         (n_pairs + pair.max_clusters - 1) / pair.max_clusters <= waves2)
         return launch_variant<128, 1, 1, true>(a, sm_count, stream);
     return 2 * n_tiles2 >= sm_count ? launch_variant<128, 2, 1>(a, sm_count, stream) : launch_variant<128, 1, 1>(a, sm_count, stream);

@@ -207,11 +207,12 @@ def test_row_quantisers(bt, oracle, m, k, dtype):
     (129, 9217, 260),    # the last tile's second half: no rows; one token in the second token block
     (300, 6300, 516),    # token blocks in odd number: a half without tokens
     (2049, 1160, 1028),  # more token blocks than row tiles
-    (1030, 9000, 256),   # several tiles of a single 256-input chunk to a CTA pair
+    (1030, 9000, 256),   # several tiles of a single 256-input chunk
+    (129, 9217, 1796), (300, 6300, 2052), (2049, 1160, 2048), (600, 8300, 1792),  # with pairs, the last one on their near side
 ])
 @pytest.mark.parametrize("dtype,bases", [("float32", 1), ("bfloat16", 1), ("float32", 2), ("bfloat16", 3)])
 def test_tensor_core_path_cta_pairs(bt, oracle, m, n, k, dtype, bases):
-    # products large enough for tiles of 256 rows x 256 tokens over two CTAs: the oracle's bits
+    # products of tiles of 256 rows x 256 tokens over two CTAs (from 2048 inputs on, rounded up to 256): the oracle's bits
     rng = np.random.default_rng(m + n + bases)
     packed = np.stack([ternary_packed(rng, n, k, p_code3=0.01) for _ in range(bases)], -1)
     scales = np.array([0.5 / 3 ** b for b in range(bases)], np.float32)

@@ -291,7 +291,7 @@ def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, pa
     assert bt.lib().bt_device_check(0) == 0
 
 
-@pytest.mark.parametrize("hidden,ff,batch,n", [(256, 176, 1, 65), (256, 1040, 1, 129), (1024, 4112, 3, 90), (512, 5008, 5, 199)])
+@pytest.mark.parametrize("hidden,ff,batch,n", [(256, 176, 1, 65), (256, 1040, 1, 129), (1024, 4112, 3, 90), (512, 5008, 5, 199), (2048, 5008, 5, 199)])
 def test_prefill_silu_in_the_product(bt, oracle, syn, hidden, ff, batch, n):
     # more than 64 rows: silu(gate) * up leaves the gate|up product itself; few row tiles, row tiles that end inside a set of
     # 128, tiles without some of their tokens, CTA pairs (the last)
