@@ -193,8 +193,8 @@ cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride
                            bool prequantised = false,     // qtc / sx / qsum are already filled (x unused)
                            bt_dtype x_dtype = BT_F32,     // element type of x: BT_F32 or BT_BF16
                            float* sum = nullptr);         // [m, out_stride] f32: where several bases meet before a bf16 output
-// Whether the product can leave silu(gate) * up of interleaved rows (EPI_SWIGLU: out[m, j], out_stride elements a token).
-bool gemm_tc_swiglu(const LinearDev& lin, int64_t m);
+// From how many tokens on the product leaves silu(gate) * up of interleaved rows (EPI_SWIGLU: out[m, j], out_stride elements a token).
+int64_t gemm_tc_swiglu_from(const LinearDev& lin, int sm_count);
 // Whether the row kernel that lays the activations out can hold a row of this many inputs.
 bool row_quant_fits(int64_t k, int64_t k_tiles);
 

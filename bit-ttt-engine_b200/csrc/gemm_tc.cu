@@ -26,6 +26,7 @@
 // activations are stored residue-split: B_r[m, k'] = q[m, 4k' + r]; the four residue products of a
 // chunk accumulate into the same accumulator.
 #include <cstdint>
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR ? 2 : RS), 1) gemm_tc_kernel(T
                 case EPI_F32: epilogue_role(std::integral_constant<int, EPI_F32>{}); break;
                 case EPI_F32_ACCUM: epilogue_role(std::integral_constant<int, EPI_F32_ACCUM>{}); break;
                 case kEpiBf16Accum: epilogue_role(std::integral_constant<int, kEpiBf16Accum>{}); break;
-                case EPI_SWIGLU: if constexpr (NT == 128) epilogue_role(std::integral_constant<int, EPI_SWIGLU>{}); break;
+                case EPI_SWIGLU: if constexpr (NT == 128 && (RS == 2 || PAIR)) epilogue_role(std::integral_constant<int, EPI_SWIGLU>{}); break;
                 default: epilogue_role(std::integral_constant<int, EPI_BF16>{}); break;
             }
         }
@@ -812,10 +813,17 @@ size_t gemm_tc_act_bytes(int64_t m, int64_t k_tiles) {
     return (size_t)((m + nt - 1) / nt * k_tiles * 4 * nt * 64);
 }
 
-// More than 64 tokens, where tiles follow one another and the exponentials of one are worked out under the MMAs of the next (2048 x
-// 4096 -> 28672 with the quantiser behind it, 32 layers: 3 428 -> 3 274 us a prefill).  With fewer a CTA has one tile, and its eight
-// epilogue warps are the last thing the launch waits for: the decode step of 64 sequences became slower, and keeps the quantiser's.
-bool gemm_tc_swiglu(const LinearDev& lin, int64_t m) { return m > 64 && lin.w.n_bases == 1 && lin.w.n_out % kTileRows == 0; }
+// The epilogue pays where tiles follow one another and the exponentials of one are worked out under the MMAs of the next: more rounds of
+// 256 x 128 tiles over the SMs the fewer MMAs a tile has.  A prefill with the quantiser's exponentials -> the epilogue's, us (two layers):
+// 4096 inputs, 28672 rows, 256 tokens (1.5 rounds) 548 -> 565, 512 (3.0) 695 -> 689, 2048 (12) 1 576 -> 1 506; 3072 -> 16384, 1536 tokens
+// (5.2) 835 -> 840, 2048 (6.9) 1 038 -> 1 024; 2048 -> 11264, 3072 tokens (7.1) 976 -> 980, 4096 (9.5) 1 184 -> 1 180, 8192 (19) 2 385 ->
+// 2 337; 1024 -> 16384, 8192 tokens (28) 1 561 -> 1 694.
+int64_t gemm_tc_swiglu_from(const LinearDev& lin, int sm_count) {
+    if (lin.w.n_bases != 1 || lin.w.n_out % kTileRows != 0 || lin.w.k_tiles < 8) return INT64_MAX;
+    const int64_t rounds = lin.w.k_tiles >= 16 ? 2 : (lin.w.k_tiles >= 12 ? 6 : 9), row_sets = (lin.w.row_tiles + 15) / 16;
+    const int64_t blocks = (rounds * sm_count + row_sets - 1) / row_sets;  // of 128 tokens
+    return std::max<int64_t>((blocks - 1) * 128 + 1, 65);
+}
 
 cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride, int64_t m, int8_t* qtc, float* sx,
                            int32_t* qsum, void* out, int64_t out_stride, int epilogue, unsigned int* err, int sm_count,
@@ -823,7 +831,7 @@ cudaError_t launch_gemm_tc(const LinearDev& lin, const void* x, int64_t x_stride
     if (lin.w.n_bases != 1 && epilogue == EPI_BF16 && !sum) return cudaErrorInvalidValue;
     const int nt = m <= 64 ? 64 : 128;
     if (epilogue != EPI_I32 && epilogue != EPI_F32 && epilogue != EPI_F32_ACCUM && epilogue != EPI_BF16 &&
-        !(epilogue == EPI_SWIGLU && gemm_tc_swiglu(lin, m)))
+        !(epilogue == EPI_SWIGLU && m >= gemm_tc_swiglu_from(lin, sm_count)))
         return cudaErrorInvalidValue;
     const int k = (int)lin.w.k_in, kts = (int)lin.w.k_tiles;
     cudaError_t e = cudaSuccess;

@@ -844,11 +844,11 @@ bt_status prefill_buffers(bt_model* m, int rows) {
     const int64_t H = c.hidden_dim, I = m->i_l, kmax = H > I ? H : I;
     const int64_t qw = c.arch == 1 ? m->qkv_dim : m->d_small;  // q|k|v, or the TTT features and predictions (two slots)
     const size_t n = (size_t)rows;
-    // Gate and up rows, or silu(gate) * up where the product leaves that (more than 64 rows: 470 MB instead of 940 for 8192 x 14336); with
-    // several bases a projection's sum as well.
-    bool act = true;
-    for (const Layer& L : m->layers) act = act && gemm_tc_swiglu(L.gate_up_il->dev(), rows);
-    const size_t gu = std::max({n * (act ? 1 : 2) * I, act ? (size_t)128 * I : 0, m->multi_basis ? n * H : 0});
+    // Gate and up rows, or silu(gate) * up where the product leaves that (470 MB instead of 940 for 8192 x 14336; a shorter piece has gate
+    // and up rows); with several bases a projection's sum as well.
+    int64_t from = 0;
+    for (const Layer& L : m->layers) from = std::max(from, gemm_tc_swiglu_from(L.gate_up_il->dev(), m->sm_count));
+    const size_t gu = std::max({n * I, (size_t)std::min<int64_t>(rows, from - 1) * 2 * I, m->multi_basis ? n * H : 0});
     struct { void** p; size_t bytes; void* fresh; } bufs[] = {
         {(void**)&m->pf_tokens, n * sizeof(int32_t)}, {(void**)&m->pf_h, n * H * sizeof(float)}, {(void**)&m->pf_qkv, n * qw * sizeof(float)},
         {(void**)&m->pf_att, n * H * sizeof(float)}, {(void**)&m->pf_gu, gu * sizeof(float)},
@@ -950,7 +950,7 @@ bt_status enqueue_prefill_chunk(bt_model* m, int batch, int n, int past, int ttt
         }
         BT_CUDA_TRY(trace_copy(m, li, TR_H_MID, m->pf_h, M, s));
         BT_CUDA_TRY(launch_row_quant(PRE_RMSNORM, m->pf_h, H, L.norm2, kRmsEps, M, H, nullptr, 0, m->pf_sx, m->pf_qsum, nullptr, s, m->pf_qtc, kt_h));
-        if (gemm_tc_swiglu(L.gate_up_il->dev(), M)) {
+        if (M >= gemm_tc_swiglu_from(L.gate_up_il->dev(), sm)) {
             // silu(gate) * up in the product's epilogue, under the next tile's MMAs: half the output bytes, and a quantiser without the
             // exponential
             BT_CUDA_TRY(launch_gemm_tc(L.gate_up_il->dev(), nullptr, H, M, m->pf_qtc, m->pf_sx, m->pf_qsum, m->pf_gu, I, EPI_SWIGLU, err, sm, s, true));

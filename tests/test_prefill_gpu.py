@@ -291,11 +291,12 @@ def test_prefill_attention_against_decode(bt, syn, heads, kv_heads, hd, kind, pa
     assert bt.lib().bt_device_check(0) == 0
 
 
-@pytest.mark.parametrize("hidden,ff,batch,n", [(256, 176, 1, 65), (256, 1040, 1, 129), (1024, 4112, 3, 90), (512, 5008, 5, 199), (2048, 5008, 5, 199)])
+@pytest.mark.parametrize("hidden,ff,batch,n", [(256, 176, 1, 65), (256, 1040, 1, 129), (1024, 4112, 3, 90), (512, 5008, 5, 199),
+                                                  (4096, 14336, 1, 300), (4096, 4112, 5, 210), (2048, 5632, 8, 490)])
 def test_prefill_silu_in_the_product(bt, oracle, syn, hidden, ff, batch, n):
-    # more than 64 rows: silu(gate) * up leaves the gate|up product itself; few row tiles, row tiles that end inside a set of
-    # 128, tiles without some of their tokens, CTA pairs (the last)
-    cfg = syn.BitLlamaConfig("llama", 64, hidden, 1, hidden // 64, hidden // 128, ff, max_position_embeddings=256)
+    # silu(gate) * up in the quantiser (the first four: few row tiles, row tiles that end inside a set of 128), and leaving the
+    # gate|up product itself: tiles without some of their tokens, CTA pairs and row tiles that end inside a set (the last two)
+    cfg = syn.BitLlamaConfig("llama", 64, hidden, 1, hidden // 64, hidden // 128, ff, max_position_embeddings=512)
     w = syn.make_weights(cfg, seed=ff, from_latent=False)
     gpu, ref = syn.build_model(w, max_batch=batch), oracle.model_from_weights(w)
     states = [ref.new_state() for _ in range(batch)]
@@ -371,10 +372,10 @@ def test_prompt_without_memory_for_the_large_pass(bt, syn):
     assert bt.lib().bt_device_check(0) == 0
 
 
-@pytest.mark.parametrize("n,nxt", [(65, 64), (128, 63), (200, 9), (10, 64)])
-def test_pieces_on_both_sides_of_64_rows(bt, oracle, syn, n, nxt):
+@pytest.mark.parametrize("n,nxt", [(257, 256), (290, 64), (40, 257)])
+def test_pieces_with_and_without_silu_in_the_product(bt, oracle, syn, n, nxt):
     # the buffer of a piece that stores silu(gate) * up holds gate and up rows of a shorter piece behind it
-    cfg = syn.BitLlamaConfig("llama", 64, 256, 2, 4, 2, 1040, max_position_embeddings=300)
+    cfg = syn.BitLlamaConfig("llama", 64, 4096, 1, 32, 8, 14336, max_position_embeddings=600)
     w = syn.make_weights(cfg, seed=n, from_latent=False)
     gpu, ref = syn.build_model(w), oracle.model_from_weights(w)
     states, rng = [ref.new_state()], np.random.default_rng(n)
@@ -385,11 +386,11 @@ def test_pieces_on_both_sides_of_64_rows(bt, oracle, syn, n, nxt):
 
 def test_memory_of_a_long_prompt(bt, syn):
     import torch
-    cfg = syn.BitLlamaConfig("llama", 64, 512, 1, 8, 2, 8192, max_position_embeddings=4096)
+    cfg = syn.BitLlamaConfig("llama", 64, 4096, 1, 32, 8, 4096, max_position_embeddings=4096)
     m = syn.build_model(syn.make_weights(cfg, seed=1, from_latent=False), max_batch=2)
     m.prefill(np.zeros((2, 70), np.int64))  # (kernels are loaded)
     m.reset_kv_cache()
     before = torch.cuda.mem_get_info()[0]
     m.prefill(np.zeros((2, 4096), np.int64))
-    rows = 8192 * (4 * (512 + 768 + 512 + 8192) + 8192 + 16 + 32)  # stream, q|k|v, attention, silu(gate) * up, int8, scales
+    rows = 8192 * (4 * (4096 + 6144 + 4096 + 4096) + 4096 + 4 * 35)  # stream, q|k|v, attention, silu(gate) * up, int8, scales and tokens
     assert before - torch.cuda.mem_get_info()[0] <= rows + (32 << 20)
