@@ -827,53 +827,83 @@ __global__ void __launch_bounds__(512) embed_pos_kernel(const int32_t* __restric
     }
 }
 
-// Norm in equal parts of a multiple of eight columns: LG lanes per part and turn, the part in registers.  (A whole warp for parts
-// of 64 columns left three of four lanes idle, a part in flight a warp: 1999 rows of 32 parts 32.1 us, now 11.3.)
-template <int NI, int LG>
+// Norm in equal parts of a multiple of eight columns: a warp per part and turn, the part in registers.
+template <int NI>
 __global__ void __launch_bounds__(256) group_norm_kernel(const RowArgs a, int part) {
-    constexpr int kPer = 256 / LG;  // parts at a time
     const int64_t row = blockIdx.x;
-    const int k = a.k, lane = threadIdx.x % LG;
+    const int k = a.k, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    const float* y = a.y + row * a.ld;
+    const float* gate = a.gate ? a.gate + row * a.gate_ld : nullptr;
+    const bool vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0, gvec = (reinterpret_cast<uintptr_t>(gate) & 15) == 0;
+    for (int g = warp; g < a.groups; g += 8) {
+        float v[NI][8];
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) get8(y + g * part, (i * 32 + lane) * 8, part, vec, v[i]);
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(v[i][j], v[i][j], ss);
+        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)part + a.eps);
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int c0 = (i * 32 + lane) * 8;
+            if (c0 >= part) break;
+            float w[8];
+            get8(a.w + g * part, c0, part, true, w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[i][j] = v[i][j] * inv * w[j];
+            if (gate) {
+                get8(gate + g * part, c0, part, gvec, w);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[i][j] *= silu_f(w[j]);
+            }
+            put8(a.act, row, g * part + c0, k, v[i]);
+        }
+    }
+    const float zero[8] = {};
+    for (int c0 = k + (int)threadIdx.x * 8; c0 < dense_kpad(k); c0 += 256 * 8) put8(a.act, row, c0, k, zero);
+}
+// The same for parts of up to 64 columns: eight lanes a part, four parts a warp, the gates requested with the values.  (A whole warp
+// left three of four lanes idle, a part in flight a warp: 1999 rows of 32 parts 32.1 us, now 11.3.  With parts of 2048 columns this
+// form holds twice the registers of the one above: 46 us and 24.)
+__global__ void __launch_bounds__(256) group_norm_small_kernel(const RowArgs a, int part) {
+    constexpr int kLanes = 8, kPer = 256 / kLanes;  // lanes of a part, parts at a time
+    const int64_t row = blockIdx.x;
+    const int k = a.k, c0 = (int)threadIdx.x % kLanes * 8;
     ptx::pdl_wait();
     ptx::pdl_launch_dependents();
     const float* y = a.y + row * a.ld;
     const float* gate = a.gate ? a.gate + row * a.gate_ld : nullptr;
     const bool vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0, gvec = (reinterpret_cast<uintptr_t>(gate) & 15) == 0;
     for (int g0 = 0; g0 < a.groups; g0 += kPer) {  // (every lane of a warp takes every turn)
-        const int g = g0 + (int)threadIdx.x / LG;
+        const int g = g0 + (int)threadIdx.x / kLanes;
         const bool live = g < a.groups;
-        float v[NI][8], q[NI][8];
+        float v[8], q[8];
         float ss = 0.0f;
+        get8(y + g * part, c0, live ? part : 0, vec, v);
+        if (gate) get8(gate + g * part, c0, live ? part : 0, gvec, q);
 #pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int c0 = (i * LG + lane) * 8;
-            get8(y + g * part, c0, live ? part : 0, vec, v[i]);
-            if (gate) get8(gate + g * part, c0, live ? part : 0, gvec, q[i]);
-        }
+        for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
 #pragma unroll
-        for (int i = 0; i < NI; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ss = fmaf(v[i][j], v[i][j], ss);
-#pragma unroll
-        for (int o = LG / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         const float inv = 1.0f / sqrtf(ss / (float)part + a.eps);
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int c0 = (i * LG + lane) * 8;
-            if (!live || c0 >= part) break;
+        if (live && c0 < part) {
             float w[8];
             get8(a.w + g * part, c0, part, true, w);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[i][j] = v[i][j] * inv * w[j];
+            for (int j = 0; j < 8; ++j) v[j] = v[j] * inv * w[j];
             if (gate)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[i][j] *= silu_f(q[i][j]);
-            put8(a.act, row, g * part + c0, k, v[i]);
+                for (int j = 0; j < 8; ++j) v[j] *= silu_f(q[j]);
+            put8(a.act, row, g * part + c0, k, v);
         }
         __syncwarp();
     }
     const float zero[8] = {};
-    for (int c0 = k + (int)threadIdx.x * 8; c0 < dense_kpad(k); c0 += 256 * 8) put8(a.act, row, c0, k, zero);
+    for (int c = k + (int)threadIdx.x * 8; c < dense_kpad(k); c += 256 * 8) put8(a.act, row, c, k, zero);
 }
 
 // NC: groups of eight columns per thread; the whole row is requested before anything is computed.
@@ -1132,10 +1162,10 @@ cudaError_t launch_row_op(const RowArgs& a, cudaStream_t s, bool pdl) {
         const int part = a.k / a.groups;
         if (part % 8 == 0 && part <= 2048) {
             const dim3 grid((unsigned)a.rows);
-            if (part <= 64) return launch_pdl(group_norm_kernel<1, 8>, grid, dim3(256), 0, s, pdl, a, part);
-            if (part <= 256) return launch_pdl(group_norm_kernel<1, 32>, grid, dim3(256), 0, s, pdl, a, part);
-            if (part <= 1024) return launch_pdl(group_norm_kernel<4, 32>, grid, dim3(256), 0, s, pdl, a, part);
-            return launch_pdl(group_norm_kernel<8, 32>, grid, dim3(256), 0, s, pdl, a, part);
+            if (part <= 64) return launch_pdl(group_norm_small_kernel, grid, dim3(256), 0, s, pdl, a, part);
+            if (part <= 256) return launch_pdl(group_norm_kernel<1>, grid, dim3(256), 0, s, pdl, a, part);
+            if (part <= 1024) return launch_pdl(group_norm_kernel<4>, grid, dim3(256), 0, s, pdl, a, part);
+            return launch_pdl(group_norm_kernel<8>, grid, dim3(256), 0, s, pdl, a, part);
         }
     }
     // many rows: fewer threads with more of the row each, so that more rows share an SM

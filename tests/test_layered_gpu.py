@@ -188,6 +188,17 @@ def test_recurrence_of_many_heads(bt, heads):
         assert_close(feed(m, tokens, sizes), logits, "bfloat16", sizes)
 
 
+@pytest.mark.parametrize("heads,vdim,groups", [(12, 16, 6), (8, 24, 3), (8, 24, 2), (24, 64, 2), (48, 64, 3), (34, 64, 2), (50, 64, 2)])
+def test_norm_in_parts(bt, heads, vdim, groups):  # parts of 32, 64, 96, 768, 1024, 1088 and 1600 columns
+    cfg = lay.LayersConfig(40, 48, 120, 1e-5, True, [ssm(heads, vdim, 16, taps=2, norm_groups=groups)])
+    t = make_tensors(cfg, seed=heads)
+    tokens = np.random.default_rng(heads).integers(0, 40, 90).astype(np.int32)
+    logits, _ = oracle(cfg, t, tokens)
+    for dtype in ("bfloat16", "float32"):
+        m = lay.build_layered(cfg, t, dtype=dtype)
+        assert_close(feed(m, tokens, [70, 20]), logits, dtype)
+
+
 def needle_model(n_positions, dtype_seed=0):
     """One attention layer whose query of token 1 points at the key of token 0 (score far above all others)."""
     cfg = lay.LayersConfig(60, 96, n_positions, 1e-5, True, [attn(4, 2, 32, 24, scale=0.6, cap=18.0, coef=0.3, every=50)])
