@@ -597,13 +597,8 @@ __global__ void __launch_bounds__(256) lm_head_fused_kernel(const __nv_bfloat16*
 // whatever the warps do; the first ones are requested before the wait for the kernel in front.  Through registers (above) 64 KB
 // an SM were.  Bound by the reads of the weights: 32000 x 4096 64 -> 57 us, 4.6 TB/s (the same with slots of 2 KB, six a warp; 64 with
 // eight warps and slots of 8 KB).  Sums in the same order.  Rows of other lengths, or more than 8192 values, stay with the kernel
-// above; so do several tokens, whose values for one row the rings leave no room for, and large vocabularies (head_stream_rows).
+// above; so do several tokens, whose values for one row the rings leave no room for.
 constexpr int kHeadWarps = 16, kHeadSlot = 4096, kHeadSlots = 3, kHeadMaxLd = 8192;
-// Up to how many rows: its early start is worth 5 to 10 us a step, and behind that its 16 warps an SM get through short rows more slowly
-// than the 32 of the kernel above.  A step of a one-layer model, above -> here, us: width 1024, 16 000 rows 40.2 -> 40.1, 24 000 42.8 ->
-// 44.3; 4096, 16 000 73.4 -> 68.0, 32 000 91.1 -> 91.0, 50 304 112.6 -> 116.3, 128 256 203 -> 222; 6144, 64 000 179 -> 177, 128 256 292 ->
-// 300; 8192, 32 000 168 -> 145, 128 256 432 -> 376.
-int64_t head_stream_rows(int ld) { return ld < 2048 ? 16384 : (ld <= 4096 ? 32768 : (ld <= 7168 ? 65536 : INT64_MAX)); }
 constexpr unsigned kErrHeadTimeout = 0x48454144u;  // 'HEAD'
 template <bool F16>
 __global__ void __launch_bounds__(kHeadWarps * 32, 1) lm_head_stream_kernel(const __nv_bfloat16* __restrict__ w, const float* __restrict__ h, const float* __restrict__ norm_w,
@@ -870,7 +865,7 @@ cudaError_t launch_lm_head_fused(const __nv_bfloat16* w, const float* h, const f
     if (ld == 0) ld = hidden;
     if (ld % 8 != 0 || ld < hidden || batch < 1) return cudaErrorInvalidValue;
     // (a row must be whole pieces of a warp: 32 lanes x 8 values)
-    if (batch == 1 && ld % 256 == 0 && ld <= kHeadMaxLd && vocab <= head_stream_rows(ld) && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && !(f16 && (ld != hidden || cap > 0.0f))) {
+    if (batch == 1 && ld % 256 == 0 && ld <= kHeadMaxLd && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && !(f16 && (ld != hidden || cap > 0.0f))) {
         constexpr size_t rings = (size_t)kHeadWarps * kHeadSlots * kHeadSlot;
         static PerDeviceOnce once;
         cudaError_t ce = once.run([] {
