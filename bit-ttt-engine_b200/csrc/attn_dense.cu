@@ -900,13 +900,11 @@ cudaError_t tile_launch_k(const DenseAttn& a, const LatentTile& lt, const ActOut
 }
 int pad8(int n) { return (n + 7) / 8 * 8; }
 
-// Tiles of 128 positions pay from this many rows on.  Their first tile takes 14 us (set-up, 128 queries, the sum of the groups at
-// the end), each further one of 128 keys 2.2 to 3.2; a tile of 64 keys of the kernel above takes 2.4 us for heads of 64 and 6 for
-// keys of 192.  64-position tiles and these, us: 32 heads of 64 with a cap, 512 rows 23.6 and 24.2, 1024 58.6 and 50.5; of 32, 512
-// rows 20.4 and 22.7, 768 36.3 and 31.0; 16 heads of 128 with a cap, 320 rows 24.5 and 25.2, 512 35.5 and 27.5; of 80 + 64, 384 rows
-// 16.4 and 17.4, 512 20.3 and 18.8; of 192 + 128, 128 rows 17.4 and 18.4, 256 26.1 and 18.3.
-// (With the softmax unrolled; rolled up these tiles take 9 to 28 % less, 640 rows of 32 heads of 64 21.9, and both kernels are close
-// together somewhat below the lines, which are on the safe side.)
+// Tiles of 128 positions are taken from this many rows on.  64-position tiles and these, us under the profiler, nothing before the prompt: 32
+// heads of 64 with a cap, 320 rows 15.8 and 15.9, 640 35.9 and 22.1; of 32, 192 rows 9.1 and 10.2, 640 26.2 and 17.1; 16 heads of 128 with
+// a cap, 96 rows 15.7 and 13.7, 448 32.9 and 20.6; keys of 80 + 64, 192 rows 12.5 and 13.5, 448 22.6 and 17.8; 192 + 128, 96 rows 18.2 and
+// 14.6, 192 21.6 and 15.9.  The lines are on the safe side: below them the two are within a fifth of each other, and behind 1000
+// positions these tiles are ahead of the others at 96 rows already (37.6 and 29.1, 31.0 and 21.1, 74.5 and 34.6, 48.9 and 30.0, 94.0 and 39.5).
 bool attn_flash_pays(const DenseAttn& a, bool latent) {
     return a.q_rows >= (a.kv.k_stride <= 64 ? 640 : (a.kv.k_stride <= 128 ? 448 : 192)) && attn_flash_fits(a, latent);
 }
